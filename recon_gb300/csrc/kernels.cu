@@ -1132,12 +1132,8 @@ static_assert(alignof(IterShared) >= 16 && offsetof(IterShared, J) % 16 == 0 && 
 
 struct SolveShared {
     float T[16];
-    double A_ph[27], A_icp[27];
+    double A_icp[27];
     SolveScratch S;
-    // scalars loaded with the sums
-    double fuse_c2;
-    unsigned long long work0, work1;
-    int nsel, median, st_iters, st_solves, st_nonspd, trace_slot;
 };
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
@@ -1616,119 +1612,122 @@ __device__ __forceinline__ int packed_index(int r, int c) {
     return a * 6 - (a * (a - 1)) / 2 + (b - a);
 }
 
-// The end of an iteration of an instance: the accumulated terms in FP64 (reset
-// for the next iteration), the system of the mode (fused in FP64 for
-// BIOBJECTIVE with weights precomputed off this path, linearFuseKernel
-// warp.cu:918-924), the solve and SE(3) update (warp 0), the statistics and
-// the optional trace.  Every global value it reads is loaded in one round trip
-// at the start (threads 54..63 fetch the scalars), since the FP64 solve that
-// follows is a long serial chain.
+// The end of an iteration of an instance: the accumulated terms in FP64, the
+// system of the mode (fused in FP64 for BIOBJECTIVE with weights precomputed
+// off this path, linearFuseKernel warp.cu:918-924), the solve and SE(3) update.
+// Warp 0 takes the photometric terms (lane q: term q), warp 1 the ICP terms,
+// handed over through shared memory; every global value is loaded in one round
+// trip at the start, since the FP64 solve that follows is one serial chain on
+// warp 0.  Warp 1 meanwhile resets the sums, keeps the work counters and writes
+// the optional trace.  With the small-twist path, the column-at-once Cholesky and
+// the lane-parallel conjugate gradients of solve.cuh (measured on one instance, graph replay):
+// an iteration of 320x240 photometric tracking 21.7 us against 25.1 us, a
+// bi-objective 640x480 frame of 19 iterations 559 against 630 us, a 482x362
+// geometric keyframe and frame with the CG solver 458 against 668 us.
 __device__ __forceinline__ void finalize_iter(const InstDesc &d, SolveShared &sh, int level, int it, bool use_ph,
                                               bool use_icp) {
-    int t = threadIdx.x;
+    int lane = threadIdx.x & 31, set = threadIdx.x >> 5;
     SolveScratch &S = sh.S;
-    long long L[kFxLimbs];
-    int bad = 0;
-    unsigned long long *src = nullptr;
-    if (t < 54) {
-        int set = t / 27, q = t % 27;
-        src = d.fx + set * kFxTerms + q * kFxLimbs;
-#pragma unroll
-        for (int k = 0; k < kFxLimbs; k++) L[k] = (long long)__ldcg(src + k);
-        bad = __ldcg(d.fx_bad + set);
-    } else if (t == 54) {
-        sh.nsel = use_icp ? __ldcg(d.icp_nsel + level) : 0;
-    } else if (t == 55) {
-        sh.fuse_c2 = __ldcg(d.fuse_c2 + level);
-    } else if (t == 56) {
-        sh.median = use_ph ? __ldcg(d.ph_hist + 512) : -1;
-    } else if (t == 57) {
-        sh.st_iters = __ldcg(d.stats + ST_ITERS);
-        sh.st_solves = __ldcg(d.stats + ST_SOLVES);
-        sh.st_nonspd = __ldcg(d.stats + ST_NONSPD);
-    } else if (t == 58) {
-        sh.work0 = __ldcg(d.work + 0);
-        sh.work1 = __ldcg(d.work + 1);
-    } else if (t == 59) {
-        sh.trace_slot = d.trace ? __ldcg(d.trace_count) : 0;
+    int q = lane < 27 ? lane : 26;
+    unsigned long long *src = d.fx + set * kFxTerms + q * kFxLimbs;
+    longlong2 l0 = __ldcg(reinterpret_cast<const longlong2 *>(src));
+    longlong2 l1 = __ldcg(reinterpret_cast<const longlong2 *>(src) + 1);
+    int bad = __ldcg(d.fx_bad + set);
+    int nsel = use_icp ? __ldcg(d.icp_nsel + level) : 0;
+    double c2 = __ldcg(d.fuse_c2 + level);
+    int median = use_ph ? __ldcg(d.ph_hist + 512) : -1;
+    float T_before = lane < 16 ? __ldcg(d.T + lane) : 0.0f;
+    int st_iters = 0, st_solves = 0, st_nonspd = 0, slot = 0;
+    unsigned long long work0 = 0, work1 = 0;
+    if (set == 0) {
+        st_iters = __ldcg(d.stats + ST_ITERS);
+        st_solves = __ldcg(d.stats + ST_SOLVES);
+        st_nonspd = __ldcg(d.stats + ST_NONSPD);
+    } else {
+        work0 = __ldcg(d.work + 0);
+        work1 = __ldcg(d.work + 1);
     }
-    if (t < 16) sh.T[t] = __ldcg(d.T + t);
-    if (t < 54) {
-        double v = bad ? __longlong_as_double(0x7ff8000000000000LL) : fx_to_double(L);
-        (t >= 27 ? sh.A_icp : sh.A_ph)[t % 27] = v;
-#pragma unroll
-        for (int k = 0; k < kFxLimbs; k++) src[k] = 0ull;
+    if (d.trace) slot = __ldcg(d.trace_count);
+    static_assert(kFxLimbs == 4, "two 16-byte loads per term");
+    long long L[kFxLimbs] = {l0.x, l0.y, l1.x, l1.y};
+    double term = bad ? __longlong_as_double(0x7ff8000000000000LL) : fx_to_double(L);
+    if (set == 1) {
+        if (lane < 27) sh.A_icp[lane] = term;
+        if (lane < 16) S.T[lane] = (double)T_before;
+    } else if (lane < 16) {
+        sh.T[lane] = T_before;
     }
-    __syncthreads();
-    if (t < 2) d.fx_bad[t] = 0;
-    int nsel = sh.nsel;
     bool ok = !(use_icp && nsel <= 0);  // ShapeTracker "not enough points": no solve
-    int slot = sh.trace_slot;
-    bool tr_on = d.trace && slot < d.trace_max;
-    recon_iter_trace *tr = tr_on ? d.trace + slot : nullptr;
-    if (t < 42) {
-        int q = (t < 36) ? packed_index(t / 6, t % 6) : 21 + (t - 36);
-        double aph = sh.A_ph[q], aic = sh.A_icp[q];
-        double v;
-        if (d.mode == RECON_PHOTOMETRIC) v = aph;
-        else if (d.mode == RECON_GEOMETRIC) v = aic;
-        else v = ok ? __fma_rn(d.fuse_c1, aph, sh.fuse_c2 * aic) : aph;  // (1-lambda)/P * photo + lambda/N * icp
-        if (t < 36) S.A[t] = v;
-        else S.b[t - 36] = v;
+    recon_iter_trace *tr = d.trace && slot < d.trace_max ? d.trace + slot : nullptr;
+    __syncthreads();
+    // the packed term q of the mode's system
+    auto fused = [&](double aph, double aic) {
+        if (d.mode == RECON_PHOTOMETRIC) return aph;
+        if (d.mode == RECON_GEOMETRIC) return aic;
+        return ok ? __fma_rn(d.fuse_c1, aph, c2 * aic) : aph;  // (1-lambda)/P * photo + lambda/N * icp
+    };
+    if (set == 1) {
+        ulonglong2 zero = make_ulonglong2(0ull, 0ull);
+        for (int k = lane; k < 2 * kFxTerms / 2; k += 32) reinterpret_cast<ulonglong2 *>(d.fx)[k] = zero;
+        if (lane < 2) d.fx_bad[lane] = 0;
+        if (lane == 0) {
+            if (use_ph) d.work[0] = work0 + (unsigned long long)d.P;
+            if (use_icp) d.work[1] = work1 + (unsigned long long)nsel;
+            if (use_icp) d.stats[ST_ICPSEL0 + level] = nsel;
+            if (use_ph) d.stats[ST_MEDIAN] = median;
+            if (d.trace) *d.trace_count = slot + 1;
+        }
         if (tr) {
-            if (t < 36) {
-                tr->A[t] = v;
-                tr->A_ph[t] = aph;
-                tr->A_icp[t] = aic;
+            for (int k = lane; k < 256; k += 32)
+                tr->hist[k] = (use_ph && k < d.hist_bins) ? __ldcg(d.ph_hist + 256 + k) : 0;
+            if (lane == 0) {
+                tr->level = level;
+                tr->iter = it;
+                tr->mode = d.mode;
+                tr->solved = ok ? 1 : 0;
+                tr->icp_selected = use_icp ? nsel : 0;
+                tr->median_bin = median;
+            }
+        }
+        return;
+    }
+    double icp = sh.A_icp[q];
+    double v = fused(term, icp);
+    if (tr) {
+        // the packed term's one or two entries of the full matrices
+        for (int k = 0; k < 42; k++) {
+            int qk = (k < 36) ? packed_index(k / 6, k % 6) : 21 + (k - 36);
+            if (lane != qk) continue;
+            if (k < 36) {
+                tr->A[k] = v;
+                tr->A_ph[k] = term;
+                tr->A_icp[k] = icp;
             } else {
-                tr->b[t - 36] = v;
-                tr->b_ph[t - 36] = aph;
-                tr->b_icp[t - 36] = aic;
+                tr->b[k - 36] = v;
+                tr->b_ph[k - 36] = term;
+                tr->b_icp[k - 36] = icp;
             }
         }
     }
-    int median = sh.median;
-    if (tr) {
-        for (int k = t; k < 256; k += blockDim.x)
-            tr->hist[k] = (use_ph && k < d.hist_bins) ? __ldcg(d.ph_hist + 256 + k) : 0;
-    }
-    __syncthreads();
-    if (t >= 32) return;
-    int lane = t;
     int st = 0;
-    float T_before = lane < 16 ? sh.T[lane] : 0.0f;
-    if (ok) st = wsolve_update(S, d.solver, sh.T, (double)d.opt_out, lane);
-    __syncwarp();
+    if (ok) st = wsolve_packed(S, d.solver, v, sh.T, (double)d.opt_out, lane);
+    float T_after = lane < 16 ? sh.T[lane] : 0.0f;
+    if (lane < 16) d.T[lane] = T_after;
     if (d.settle_mm > 0.0f) {
         // settle rule (orc_pose_settled): every translation entry moved by at
         // most settle_mm and every rotation entry by at most settle_rot; the
         // instance's remaining iterations of this level are skipped
         bool small = true;
-        if (lane < 12) small = fabsf(sh.T[lane] - T_before) <= ((lane & 3) == 3 ? d.settle_mm : d.settle_rot);
+        if (lane < 12) small = fabsf(T_after - T_before) <= ((lane & 3) == 3 ? d.settle_mm : d.settle_rot);
         if (__all_sync(0xffffffffu, small) && lane == 0) d.stats[ST_SETTLED] = level + 1;
     }
-    if (lane < 16) d.T[lane] = sh.T[lane];
-    if (tr && lane < 16) tr->T[lane] = sh.T[lane];
+    if (tr && lane < 16) tr->T[lane] = T_after;
     if (lane == 0) {
         int *stt = d.stats;
-        unsigned long long *wk = d.work;
-        stt[ST_ITERS] = sh.st_iters + 1;
-        if (ok) stt[ST_SOLVES] = sh.st_solves + 1;
-        if (st != 0) stt[ST_NONSPD] = sh.st_nonspd + 1;
-        if (use_ph) stt[ST_MEDIAN] = median;
-        if (use_ph) wk[0] = sh.work0 + (unsigned long long)d.P;
-        if (use_icp) wk[1] = sh.work1 + (unsigned long long)nsel;
-        if (use_icp) stt[ST_ICPSEL0 + level] = nsel;
-        if (tr) {
-            tr->level = level;
-            tr->iter = it;
-            tr->mode = d.mode;
-            tr->solved = ok ? 1 : 0;
-            tr->status = st;
-            tr->icp_selected = use_icp ? nsel : 0;
-            tr->median_bin = median;
-        }
-        if (d.trace) *d.trace_count = slot + 1;
+        stt[ST_ITERS] = st_iters + 1;
+        if (ok) stt[ST_SOLVES] = st_solves + 1;
+        if (st != 0) stt[ST_NONSPD] = st_nonspd + 1;
+        if (tr) tr->status = st;
     }
 }
 
@@ -2063,7 +2062,10 @@ __global__ void __launch_bounds__(32) k_gate_twist(const InstDesc *D, const floa
     __shared__ float Dm[16];
     __shared__ SolveScratch S;
     int t = threadIdx.x;
-    if (t < 16) Dm[t] = (t % 5 == 0) ? 1.0f : 0.0f;
+    if (t < 16) {
+        Dm[t] = (t % 5 == 0) ? 1.0f : 0.0f;
+        S.T[t] = (t % 5 == 0) ? 1.0 : 0.0;
+    }
     __syncwarp();
     double x[6];
     for (int k = 0; k < 6; k++) x[k] = (double)(net_out[blockIdx.x * 6 + k] * scale[k]);
