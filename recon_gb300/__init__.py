@@ -161,6 +161,7 @@ def lib() -> ctypes.CDLL:
             L.recon_render_depth.argtypes = [vp, vp, f32, ctypes.c_uint32, ctypes.c_uint32, vp, vp]
             L.recon_render_gray.argtypes = [vp, vp, vp, vp]
             L.recon_selftest_exact_arith.argtypes = [vp]
+            L.recon_selftest_division.argtypes = [vp]
             L.recon_kinect_disparity_to_depth.argtypes = [vp, i32, i32, f32, f32, f32, f32, f32, f32, i32, vp, vp]
             L.recon_kinect_rgb_to_gray.argtypes = [vp, i32, i32, vp, vp]
             L.recon_kinect_undistort_gray.argtypes = [vp, i32, i32, vp, vp, vp, vp, vp]
@@ -600,6 +601,13 @@ def selftest_exact_arith() -> int:
     over every float in [0, 2^23), run on the current GPU."""
     out = np.zeros(1, np.int64)
     check(lib().recon_selftest_exact_arith(out.ctypes.data))
+    return int(out[0])
+
+
+def selftest_division() -> int:
+    """Mismatches of the kernels' reciprocal and division against IEEE division, run on the current GPU."""
+    out = np.zeros(1, np.int64)
+    check(lib().recon_selftest_division(out.ctypes.data))
     return int(out[0])
 
 

@@ -21,7 +21,7 @@ BUILD = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "librecon_track.so")
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 UNITS = ["kernels.cu", "host.cu", "refshim.cu", "initnet.cu", "selftest.cu", "tsdf.cu", "trajio.cu", "kinect.cu"]
-HEADERS = ["scene.h", "fx.cuh", "solve.cuh", "track_kernels.cuh", "track_math.cuh", "exact_arith.cuh"]
+HEADERS = ["scene.h", "fx.cuh", "solve.cuh", "track_kernels.cuh", "track_math.cuh", "exact_arith.cuh", "pair_math.cuh"]
 
 
 def nvcc() -> str:

@@ -41,6 +41,32 @@ __device__ __forceinline__ void fx_split(float v, int &k0, long long &lo, long l
     if (bits >> 31) { lo = -lo; hi = -hi; }
 }
 
+// Adds v to a 128-bit sum of the same units held as four 32-bit words (two's
+// complement), in registers; sets bad when v is out of range.
+__device__ __forceinline__ void fx_accumulate(uint32_t *a, float v, int &bad) {
+    uint32_t bits = __float_as_uint(v), E = (bits >> 23) & 0xffu;
+    if (E >= 175u) {  // |v| >= 2^48, Inf or NaN
+        bad = 1;
+        return;
+    }
+    // below 2^-64 the value is cut to units of 2^-64 (E == 0 shifts everything out)
+    uint32_t m = (bits & 0x7fffffu) | 0x800000u;
+    int s = (int)E - 86;
+    if (s < 0) {
+        m = s <= -24 ? 0u : m >> -s;
+        s = 0;
+    }
+    uint64_t t = (uint64_t)m << (s & 31);
+    uint32_t lo = (uint32_t)t, hi = (uint32_t)(t >> 32), neg = bits >> 31, sign = 0u - neg;
+    int k = s >> 5;  // 0..2
+    uint32_t w0 = (k == 0 ? lo : 0u) ^ sign, w1 = (k == 0 ? hi : (k == 1 ? lo : 0u)) ^ sign;
+    uint32_t w2 = (k == 1 ? hi : (k == 2 ? lo : 0u)) ^ sign, w3 = (k == 2 ? hi : 0u) ^ sign;
+    asm("{\n.reg .u32 c;\nadd.cc.u32 c, %8, %9;\naddc.cc.u32 %0, %0, %4;\naddc.cc.u32 %1, %1, %5;\n"
+        "addc.cc.u32 %2, %2, %6;\naddc.u32 %3, %3, %7;\n}\n"
+        : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3])
+        : "r"(w0), "r"(w1), "r"(w2), "r"(w3), "r"(sign), "r"(neg));
+}
+
 __device__ __forceinline__ double fx_to_double(const long long *L) {
     unsigned __int128 Q = 0;
 #pragma unroll

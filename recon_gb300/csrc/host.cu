@@ -254,7 +254,8 @@ size_t layout(InstDesc &d, char *base) {
         d.cur_gray[l] = nl ? a.take<float>(nl) : nullptr;
         d.ref_pts[l] = nl ? a.take<float4>(nl) : nullptr;
         d.ref_nrm[l] = nl ? a.take<float4>(nl) : nullptr;
-        d.cur_pts[l] = nl ? a.take<float4>(nl) : nullptr;
+        d.ref_pl[l] = nl ? a.take<float>(6 * (size_t)((nl + kChunk - 1) / kChunk) * kChunk) : nullptr;
+        d.cur_pts[l] = nl && l > 0 ? a.take<float4>(nl) : nullptr;
         d.sel_I[l] = (l < d.L) ? a.take<float>(P) : nullptr;
         d.sel_J[l] = (l < d.L) ? a.take<float>(6 * (size_t)P) : nullptr;
         bool mixed = d.precision == RECON_PRECISION_MIXED && l < d.L;
@@ -275,8 +276,8 @@ size_t layout(InstDesc &d, char *base) {
     d.ph_hist = a.take<int>(1024);
     d.icp_mask = a.take<uint8_t>(n);
     d.icp_r2 = a.take<float>(n);
-    d.icp_w = a.take<float>(n);
     int nblk = (n + kChunk - 1) / kChunk;
+    d.icp_w = a.take<float>((size_t)nblk * kChunk);
     d.icp_blkcnt = a.take<int>(nblk);
     d.icp_blkvar = a.take<long long>(nblk);
     d.icp_part = a.take<long long>(nblk);
@@ -1288,6 +1289,21 @@ int64_t recon_batch_get_array(recon_batch *b, int32_t inst, const char *name, in
     else return fail(RECON_ERR_INVALID_ARG, "unknown array");
     if (sz > nbytes) return fail(RECON_ERR_INVALID_ARG, "destination too small");
     CK(cudaStreamSynchronize(b->stream));
+    if (nm == "cur_pts" && level == 0) {
+        // not stored: the points of the depth image, as the kernels form them
+        std::vector<float> z(n0);
+        CK(cudaMemcpy(z.data(), d.cur_z, (size_t)n0 * 4, cudaMemcpyDeviceToHost));
+        const float *K = d.calib + 43;  // the IR camera matrix (calib.h:22-37)
+        float *o = (float *)host_dst;
+        for (int i = 0; i < n0; i++, o += 4) {
+            bool ok = z[i] < 0;
+            o[0] = ok ? ((float)(i % d.W) - K[2]) * z[i] / K[0] : 0.0f;
+            o[1] = ok ? ((float)(i / d.W) - K[5]) * z[i] / K[4] : 0.0f;
+            o[2] = ok ? z[i] : 0.0f;
+            o[3] = ok ? 1.0f : 0.0f;
+        }
+        return sz;
+    }
     CK(cudaMemcpy(host_dst, src, sz, cudaMemcpyDeviceToHost));
     return sz;
 }

@@ -14,6 +14,7 @@
 #include "scene.h"
 #include "exact_arith.cuh"
 #include "fx.cuh"
+#include "pair_math.cuh"
 #include "solve.cuh"
 #include "track_kernels.cuh"
 #include "track_math.cuh"
@@ -179,7 +180,6 @@ __global__ void __launch_bounds__(256) k_prep_current_pyramid(const InstDesc *D,
             d.cur_gray[0][i] = g[k];
             if (d.cur_grayh[0]) d.cur_grayh[0][i] = __float2half_rn(g[k]);  // mixed precision
             d.cur_z[i] = z;
-            d.cur_pts[0][i] = pt[k];
         }
     }
     if (d.L < 2) return;
@@ -220,6 +220,18 @@ __global__ void __launch_bounds__(256) k_prep_current_pyramid(const InstDesc *D,
             }
         }
     }
+}
+
+// the ICP kernels' copy of reference pixel i: z NaN where the mask is 0
+__device__ __forceinline__ void store_ref_planes(float *pl, int i, float x, float y, float z, float mask, float nx,
+                                                 float ny, float nz) {
+    float *o = pl + ref_plane(i, 0);
+    o[0] = x;
+    o[kChunk] = y;
+    o[2 * kChunk] = mask != 0.0f ? z : __int_as_float(0x7fffffff);
+    o[3 * kChunk] = nx;
+    o[4 * kChunk] = ny;
+    o[5 * kChunk] = nz;
 }
 
 // fastDownSampleHdrKernel (downSample2Cuda.cu:35-42) for the reference gray
@@ -265,10 +277,12 @@ __global__ void k_downsample(const InstDesc *D, int level, const int *active) {
         normalize3(n0, n1, n2);
         d.ref_nrm[level][i] = make_float4(n0, n1, n2, 0.0f);
         d.ref_pts[level][i] = make_float4(p0, p1, p2, 1.0f);
+        store_ref_planes(d.ref_pl[level], i, p0, p1, p2, 1.0f, n0, n1, n2);
     } else {
         float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
         d.ref_pts[level][i] = o;
         d.ref_nrm[level][i] = o;
+        store_ref_planes(d.ref_pl[level], i, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f);
     }
 }
 
@@ -422,9 +436,11 @@ __global__ void k_oriented_points(const InstDesc *D, const float *const *in_pts,
     if (v.z < 0 && len > 1e-7f) {
         d.ref_pts[0][i] = make_float4(v.x, v.y, v.z, 1.0f);
         d.ref_nrm[0][i] = make_float4(n.x, n.y, n.z, 0.0f);
+        store_ref_planes(d.ref_pl[0], i, v.x, v.y, v.z, 1.0f, n.x, n.y, n.z);
     } else {
         d.ref_pts[0][i] = make_float4(0.f, 0.f, 0.f, 0.f);
         d.ref_nrm[0][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        store_ref_planes(d.ref_pl[0], i, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f);
     }
 }
 
@@ -459,6 +475,7 @@ __global__ void k_normals(const InstDesc *D, const int *active) {
     d.ref_nrm[0][i] = nrm;
     // only .w changes; neighbours read x/y/z of this element, which stay the same
     d.ref_pts[0][i].w = mask;
+    store_ref_planes(d.ref_pl[0], i, me.x, me.y, me.z, mask, nrm.x, nrm.y, nrm.z);
 }
 
 // ------------------------------------------------------------------
@@ -827,33 +844,144 @@ __device__ __forceinline__ long long trunc_prod(float r2, float w) {
 // rgb2gray.cu:827-850)
 __device__ __forceinline__ float student_w(float r2, float sigma2) { return 6 / (5 + r2 / sigma2); }
 
-// The residual and mask of pixel i of the level (icpResidualKernel2) from its
-// loaded reference point p and normal rn; returns the mask, sets r2.
-__device__ __forceinline__ uint8_t icp_mask_pixel(const InstDesc &d, const float *T, int level, float4 p, float4 rn,
-                                                  float &r2) {
+// What the ICP kernels need of a level for every pixel: the current frame's
+// points there and the projection into it.
+struct IcpLevel {
+    const float *z;     // level 0: the depth image (its points are formed from it)
+    const float4 *cur;  // the other levels' points
+    int w;
+    float wm1, hm1, fx, cx, fy, cy, a, b, rfx, rfy;
+    bool plain;  // the focal lengths are in the range of div_rn
+    __device__ __forceinline__ IcpLevel(const InstDesc &d, int level) {
+        w = d.W >> level;
+        z = d.cur_z;
+        cur = d.cur_pts[level];
+        wm1 = (float)(w - 1);
+        hm1 = (float)((d.H >> level) - 1);
+        const float *K = d.calib + RC_KL;
+        fx = K[0];
+        cx = K[2];
+        fy = K[4];
+        cy = K[5];
+        a = 1.0f / (float)(1 << level);
+        b = 0.5f * (a - 1.0f);
+        plain = div_in_range(fx, fy, fx);
+        rfx = rcp_rn(fx);
+        rfy = rcp_rn(fy);
+    }
+};
+
+// The projection of the transformed point q into the level (icpResidualKernel2
+// and icpResidualIndexKernel2, the reference's expressions without contraction:
+// they decide which pixels count), with the exact division of pair_math.cuh.
+// Returns whether it lies inside.
+__device__ __forceinline__ bool icp_project(const IcpLevel &L, float qx, float qy, float qz, float &px, float &py) {
+    float y = rcp_rn(qz), ux = div_rn(qx, -qz, y), uy = div_rn(qy, -qz, y);
+    if (!div_in_range(qx, qy, qz)) {
+        ux = ieee_div(qx, qz);
+        uy = ieee_div(qy, qz);
+    }
+    px = L.a * (L.fx * ux + L.cx) + L.b;
+    py = L.a * (L.fy * uy + L.cy) + L.b;
+    return px >= 0.0f && px < L.wm1 && py >= 0.0f && py < L.hm1;
+}
+
+// The four taps of a projected pixel.  At level 0 they are depths, and the
+// points are formed from them as genPointsCloud6Kernel does (d2z.cu:436-469; zero
+// where there is no depth): a quarter of the bytes and of the cache lines that
+// gathering points costs, for 36 operations, half of them packed.  At the other
+// levels (averages of points) they are float4 points.
+template <bool kDepth> struct IcpTaps;
+template <> struct IcpTaps<true> {
+    float z[4];
+    __device__ __forceinline__ void load(const IcpLevel &L, int o) {
+        const float *p = L.z + o, *q = p + L.w;
+        z[0] = __ldg(p);
+        z[1] = __ldg(p + 1);
+        z[2] = __ldg(q);
+        z[3] = __ldg(q + 1);
+    }
+    // which taps have a point
+    __device__ __forceinline__ bool first() const { return z[0] < 0.0f; }
+    __device__ __forceinline__ bool all() const { return z[0] < 0.0f && z[1] < 0.0f && z[2] < 0.0f && z[3] < 0.0f; }
+    __device__ __forceinline__ void points(const IcpLevel &L, float xf, float yf, float *x, float *y, float *zc) const {
+#pragma unroll
+        for (int k = 0; k < 4; k++) zc[k] = fminf(z[k], 0.0f);  // a positive depth or NaN has no point
+        float2 X = make_float2(xf - L.cx, (xf + 1.0f) - L.cx);
+        float Y0 = yf - L.cy, Y1 = (yf + 1.0f) - L.cy;
+        float2 z0 = make_float2(zc[0], zc[1]), z1 = make_float2(zc[2], zc[3]);
+        float2 ax = mul2(X, z0), bx = mul2(X, z1), ay = mul2(dup2(Y0), z0), by = mul2(dup2(Y1), z1);
+        float2 nfx = dup2(-L.fx), rx = dup2(L.rfx), nfy = dup2(-L.fy), ry = dup2(L.rfy);
+        float2 qx = div_rn2(ax, nfx, rx), sx = div_rn2(bx, nfx, rx), qy = div_rn2(ay, nfy, ry), sy = div_rn2(by, nfy, ry);
+        if (!L.plain || !(fminf(fminf(zc[0], zc[1]), fminf(zc[2], zc[3])) >= -1e12f)) {
+            qx = make_float2(ieee_div(ax.x, L.fx), ieee_div(ax.y, L.fx));
+            sx = make_float2(ieee_div(bx.x, L.fx), ieee_div(bx.y, L.fx));
+            qy = make_float2(ieee_div(ay.x, L.fy), ieee_div(ay.y, L.fy));
+            sy = make_float2(ieee_div(by.x, L.fy), ieee_div(by.y, L.fy));
+        }
+        x[0] = qx.x; x[1] = qx.y; x[2] = sx.x; x[3] = sx.y;
+        y[0] = qy.x; y[1] = qy.y; y[2] = sy.x; y[3] = sy.y;
+    }
+};
+template <> struct IcpTaps<false> {
+    float4 t[4];
+    __device__ __forceinline__ void load(const IcpLevel &L, int o) {
+        const float4 *p = L.cur + o, *q = p + L.w;
+        t[0] = __ldg(p);
+        t[1] = __ldg(p + 1);
+        t[2] = __ldg(q);
+        t[3] = __ldg(q + 1);
+    }
+    __device__ __forceinline__ bool first() const { return t[0].w != 0.0f; }
+    __device__ __forceinline__ bool all() const {
+        return t[0].w != 0.0f && t[1].w != 0.0f && t[2].w != 0.0f && t[3].w != 0.0f;
+    }
+    __device__ __forceinline__ void points(const IcpLevel &, float, float, float *x, float *y, float *z) const {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            x[k] = t[k].x;
+            y[k] = t[k].y;
+            z[k] = t[k].z;
+        }
+    }
+};
+
+// bilinearInterpolation6 of the taps at the projection (px, py), kernelUtils.h:305-316
+template <bool kDepth>
+__device__ __forceinline__ void icp_blend(const IcpLevel &L, const IcpTaps<kDepth> &t, float px, float py, float &cx,
+                                          float &cy, float &cz) {
+    // trunc by a sum rounded toward zero (index_sum): no conversions
+    float xf = index_sum(px) - 8388608.0f, yf = index_sum(py) - 8388608.0f;
+    float u = px - xf, v = py - yf;
+    float x[4], y[4], z[4];
+    t.points(L, xf, yf, x, y, z);
+    float w0 = (1 - u) * (1 - v), w1 = u * (1 - v), w2 = (1 - u) * v, w3 = u * v;
+    cx = w0 * x[0] + w1 * x[1] + w2 * x[2] + w3 * x[3];
+    cy = w0 * y[0] + w1 * y[1] + w2 * y[2] + w3 * y[3];
+    cz = w0 * z[0] + w1 * z[1] + w2 * z[2] + w3 * z[3];
+}
+
+__device__ __forceinline__ int icp_tap_index(const IcpLevel &L, bool inside, float px, float py) {
+    return inside ? index_of(index_sum(px)) + index_of(index_sum(py)) * L.w : 0;
+}
+
+// The mask and squared residual of a pixel of the level (icpResidualKernel2) from
+// its reference point (x y z, z NaN where there is none) and normal.
+template <bool kDepth>
+__device__ __forceinline__ bool icp_mask_pixel(const IcpLevel &L, const float *T, const float *p, float &r2) {
     r2 = 0.0f;
-    if (p.w == 0.0f) return 0;
-    int w = d.W >> level, h = d.H >> level;
-    const float *K = d.calib + RC_KL;
-    float a = 1.0f / (float)(1 << level);
-    float b = 0.5f * (a - 1.0f);
-    float qx, qy, qz, cnx, cny, cnz;
-    mul4(T, p.x, p.y, p.z, qx, qy, qz);
-    rot4(T, rn.x, rn.y, rn.z, cnx, cny, cnz);
-    float q2x = qx / qz, q2y = qy / qz;
-    float p2x = a * (K[0] * q2x + K[2]) + b;
-    float p2y = a * (K[4] * q2y + K[5]) + b;
-    if (!(p2x >= 0 && p2x < (w - 1) && p2y >= 0 && p2y < (h - 1))) return 0;
-    int xdi = ftoi(p2x), ydi = ftoi(p2y);
-    int off2 = xdi + ydi * w;
-    float fx = p2x - xdi, fy = p2y - ydi;
-    float cx, cy, cz, m0, m1, m2, m3;
-    bilin_pts(d.cur_pts[level], off2, w, fx, fy, cx, cy, cz, m0, m1, m2, m3);
-    if (!(m0 != 0.0f && m1 != 0.0f && m2 != 0.0f && m3 != 0.0f)) return 0;
-    float dx = cx - qx, dy = cy - qy, dz = cz - qz;
-    float res = dx * cnx + dy * cny + dz * cnz;
+    if (p[2] != p[2]) return false;
+    float qx, qy, qz, px, py, nx, ny, nz, cx, cy, cz;
+    mul4(T, p[0], p[1], p[2], qx, qy, qz);
+    if (!icp_project(L, qx, qy, qz, px, py)) return false;
+    IcpTaps<kDepth> t;
+    t.load(L, icp_tap_index(L, true, px, py));
+    if (!t.all()) return false;
+    rot4(T, p[3], p[4], p[5], nx, ny, nz);
+    icp_blend<kDepth>(L, t, px, py, cx, cy, cz);
+    float res = (cx - qx) * nx + (cy - qy) * ny + (cz - qz) * nz;
     r2 = res * res;
-    return 1;
+    return true;
 }
 
 // Whether this CTA is the last of the instance's `nblk` CTAs of the launch to
@@ -908,34 +1036,23 @@ __global__ void __launch_bounds__(kLanes, RECON_MASK_MIN_BLOCKS) k_icp_mask(cons
     __syncthreads();
     int cnt = 0;
     long long vsum = 0;
+    const IcpLevel L(d, level);
+    const float *pl = d.ref_pl[level] + (size_t)blockIdx.x * 6 * kChunk + threadIdx.x;
 #pragma unroll
-    for (int g = 0; g < 2; g++) {
-        // two pixels at a time: point and normal loads in flight together
-        int i0 = blockIdx.x * kChunk + threadIdx.x + kLanes * (2 * g);
-        float4 p[2], rn[2];
+    for (int m = 0; m < 4; m++) {
+        // (past the last pixel the planes hold 0, and the test on i ends it)
+        float p[6], r2;
+        bool ok;
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            int i = i0 + kLanes * u;
-            p[u] = rn[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (i < n) {
-                p[u] = __ldg(d.ref_pts[level] + i);
-                rn[u] = __ldg(d.ref_nrm[level] + i);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            int i = i0 + kLanes * u;
-            if (i >= n) continue;
-            float r2;
-            uint8_t ok = icp_mask_pixel(d, sT, level, p[u], rn[u], r2);
-            if (ok) {
-                float w0 = student_w(r2, 100.0f);
-                vsum += trunc_prod(r2, w0);
-            }
-            d.icp_r2[i] = r2;
-            d.icp_mask[i] = ok;
-            cnt += ok;
-        }
+        for (int k = 0; k < 6; k++) p[k] = __ldg(pl + k * kChunk + m * kLanes);
+        if (level == 0) ok = icp_mask_pixel<true>(L, sT, p, r2);
+        else ok = icp_mask_pixel<false>(L, sT, p, r2);
+        int i = blockIdx.x * kChunk + threadIdx.x + kLanes * m;
+        if (i >= n) continue;
+        if (ok) vsum += trunc_prod(r2, student_w(r2, 100.0f));
+        d.icp_r2[i] = r2;
+        d.icp_mask[i] = ok;
+        cnt += ok;
     }
     cnt = __reduce_add_sync(0xffffffffu, cnt);
     for (int o = 16; o > 0; o >>= 1) vsum += __shfl_xor_sync(0xffffffffu, vsum, o);
@@ -1059,21 +1176,16 @@ __global__ void __launch_bounds__(kLanes) k_icp_student_pass(const InstDesc *D, 
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             int i = (b0 + u) * kChunk + 4 * threadIdx.x;
-            if (b0 + u >= b_last || i >= n) continue;
+            if (b0 + u >= b_last) continue;
             if (pass == 3) {
+                // pixels past the level's last one have mask 0: the weights
+                // are zero up to the end of the block
                 float4 w = make_float4(m[u].x ? fminf(student_w(r[u].x, sigma2), 1.0f) : 0.0f,
                                        m[u].y ? fminf(student_w(r[u].y, sigma2), 1.0f) : 0.0f,
                                        m[u].z ? fminf(student_w(r[u].z, sigma2), 1.0f) : 0.0f,
                                        m[u].w ? fminf(student_w(r[u].w, sigma2), 1.0f) : 0.0f);
-                if (i + 3 < n) {
-                    *reinterpret_cast<float4 *>(d.icp_w + i) = w;
-                } else {
-                    d.icp_w[i] = w.x;
-                    if (i + 1 < n) d.icp_w[i + 1] = w.y;
-                    if (i + 2 < n) d.icp_w[i + 2] = w.z;
-                }
+                *reinterpret_cast<float4 *>(d.icp_w + i) = w;
             } else {
-                // pixels past the end have mask 0
                 if (m[u].x) vsum += trunc_prod(r[u].x, student_w(r[u].x, sigma2));
                 if (m[u].y) vsum += trunc_prod(r[u].y, student_w(r[u].y, sigma2));
                 if (m[u].z) vsum += trunc_prod(r[u].z, student_w(r[u].z, sigma2));
@@ -1111,24 +1223,57 @@ constexpr int kIterThreads = kIterBlock;  // one canonical lane (4 points of a c
 constexpr int kCluster = kIterCluster;
 constexpr int kFxTerms = 27 * kFxLimbs;
 
-// 16-byte aligned: J is the destination of 16-byte cp.async copies
-struct __align__(16) IterShared {
-    float T[16];
-    long long fx[27][kFxLimbs];  // this CTA's fixed-point sums of its warp totals
-    int fx_bad;
-    double A_ph[27];    // the allocation-free entry point's photometric terms
-    // photometric CTAs: the Jacobian of the CTA's first chunk; ICP CTAs: the
-    // Jacobians of the chunk being reduced (with R, its residuals)
-    __align__(16) float J[6][kChunk];
-    float R[kChunk];
-    int hist[256];      // this CTA's photometric histogram (read by its cluster)
-    int hist_all[256];  // the instance's histogram
-    int median;
-    SolveScratch S;     // the allocation-free entry point's solve
+// Constants of photo_pair, alike in both halves: the pose, the rig's transforms
+// (their upper three rows), the RGB camera with its distortion, the level's
+// scale and offset, the IR camera's upper two rows.
+struct alignas(16) PhotoConsts {
+    float2 T[12], TLR[12], TRL[12], KR[4], kc[3], ab[2], KL[6];
+    __device__ __forceinline__ void set_level(const InstDesc &d, int level) {
+        int t = threadIdx.x;
+        float s = 1.0f / (float)(1 << level);
+        if (t < 12) {
+            TLR[t] = dup2(d.calib[RC_TLR + t]);
+            TRL[t] = dup2(d.calib[RC_TRL + t]);
+        }
+        if (t < 6) KL[t] = dup2(d.calib[RC_KL + t]);
+        if (t < 3) kc[t] = dup2(d.calib[RC_KCR + (t < 2 ? t : 4)]);
+        if (t < 4) KR[t] = dup2(d.calib[RC_KR + (t < 2 ? 2 * t : t + 2)]);  // entries 0, 2, 4, 5
+        if (t < 2) ab[t] = dup2(t == 0 ? s : 0.5f * (s - 1.0f));
+    }
+    __device__ __forceinline__ void set_pose(float v) {
+        if (threadIdx.x < 12) T[threadIdx.x] = dup2(v);
+    }
 };
 
-static_assert(alignof(IterShared) >= 16 && offsetof(IterShared, J) % 16 == 0 && (kChunk * sizeof(float)) % 16 == 0,
-              "cp.async destinations must be 16-byte aligned");
+// 16-byte aligned: stage is the destination of 16-byte cp.async copies
+struct alignas(16) IterShared {
+    // ICP: the terms of the chunk being reduced (term k of pixel i at
+    // 1024 k + i); photometric: the Jacobian of the CTA's first chunk.  Once a warp
+    // has read its points, the 28 runs of 32 floats they occupied are its own
+    // scratch for the reduction (warp_terms).
+    float stage[7 * kChunk];
+    union {
+        uint4 sums[kIterBlock / 32][27];  // the warps' fixed-point sums, when the CTA is done
+        int peers[kCluster][256];         // before: the histograms of the cluster's CTAs, written by them
+    };
+    PhotoConsts photo;
+    float T[16];
+    int bad;        // an accumulated value was out of range
+    int hist[256];  // this CTA's photometric histogram
+    int median;
+    int warp_tot[kIterBlock / 32];
+};
+
+// The allocation-free entry point's single CTA.
+struct PhotoShared {
+    float T[16];
+    long long fx[27][kFxLimbs];  // fixed-point sums of the warp totals
+    int fx_bad;
+    double A_ph[27];
+    int hist[256];
+    int median;
+    SolveScratch S;
+};
 
 struct SolveShared {
     float T[16];
@@ -1146,14 +1291,9 @@ template <class T> __device__ __forceinline__ T *cluster_peer(T *p, int rank) {
     return reinterpret_cast<T *>(out);
 }
 
-__device__ __forceinline__ void fx_clear(IterShared &sh) {
-    for (int k = threadIdx.x; k < kFxTerms; k += blockDim.x) (&sh.fx[0][0])[k] = 0;
-    if (threadIdx.x == 0) sh.fx_bad = 0;
-}
-
-// Adds warp total v of term q (lane q of warp_terms) to the CTA's fixed-point
-// sums; the 8 warps of a CTA add to the same limbs with shared-memory atomics.
-__device__ __forceinline__ void fx_add_term(IterShared &sh, int q, float v) {
+// Adds warp total v of term q to the sums of the allocation-free entry
+// point's CTA; its 8 warps add to the same limbs with shared-memory atomics.
+__device__ __forceinline__ void fx_add_term(PhotoShared &sh, int q, float v) {
     int k0, bad = 0;
     long long lo, hi;
     fx_split(v, k0, lo, hi, bad);
@@ -1162,13 +1302,26 @@ __device__ __forceinline__ void fx_add_term(IterShared &sh, int q, float v) {
     if (bad) sh.fx_bad = 1;
 }
 
-// Adds the CTA's fixed-point sums to the instance's (after a __syncthreads).
-__device__ __forceinline__ void fx_flush(const IterShared &sh, unsigned long long *dst, int *dst_bad) {
+// Adds the CTA's sums, a 128-bit value per warp and term (lane q of a warp:
+// term q), to the instance's limbs: the warps' words are added as limbs, the top
+// one signed, so no carries are needed.  sh.bad must be 0 before.
+__device__ __forceinline__ void fx_flush(IterShared &sh, const uint32_t *acc, int bad, unsigned long long *dst,
+                                         int *dst_bad) {
+    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (lane < 27) sh.sums[w][lane] = make_uint4(acc[0], acc[1], acc[2], acc[3]);
+    if (lane < 27 && bad) sh.bad = 1;
+    __syncthreads();
     if (threadIdx.x < kFxTerms) {
-        long long v = (&sh.fx[0][0])[threadIdx.x];
+        const uint32_t *words = reinterpret_cast<const uint32_t *>(&sh.sums[0][0]) + threadIdx.x;
+        long long v = 0;
+#pragma unroll
+        for (int k = 0; k < kIterBlock / 32; k++) {
+            uint32_t x = words[k * kFxTerms];
+            v += (threadIdx.x & 3) == 3 ? (long long)(int)x : (long long)x;
+        }
         if (v) atomicAdd(dst + threadIdx.x, (unsigned long long)v);
     }
-    if (threadIdx.x == 0 && sh.fx_bad) atomicOr(dst_bad, 1);
+    if (threadIdx.x == 0 && sh.bad) atomicOr(dst_bad, 1);
 }
 
 // canonical per-lane accumulation of the 27 normal-equation terms, one fused
@@ -1224,9 +1377,43 @@ __device__ __forceinline__ float warp_terms(const float *v) {
     return keep + __shfl_xor_sync(kFull, send, 1);
 }
 
+// The same totals through shared memory: `own` points to the warp's first run
+// of 32 floats, run r = 4 k + m lies 1024 k + 256 m floats on (all lanes past
+// their last use of them).  Run q takes the lanes' term q, rotated by 4q so that
+// neither the stores nor the 16-byte loads of 8 runs at once meet in a bank, and
+// lane q adds the butterfly's pairs of run q two at a time.  51 instructions
+// where the recursive halving takes 124 (31 shuffles of 4 issue cycles each
+// among them).  Returns term q on lane q < 27; the runs may be written again
+// after the call.
+__device__ __forceinline__ float warp_terms(const float *v, float *own) {
+    int lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 27; q++) own[(q >> 2) * kChunk + (q & 3) * kLanes + ((lane + 4 * q) & 31)] = v[q];
+    __syncwarp();
+    int q = lane < 27 ? lane : 26;
+    const float *run = own + (q >> 2) * kChunk + (q & 3) * kLanes;
+    float2 s[8];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float4 x = *reinterpret_cast<const float4 *>(run + ((4 * i + 4 * q) & 31));
+        float4 y = *reinterpret_cast<const float4 *>(run + ((16 + 4 * i + 4 * q) & 31));
+        s[2 * i] = plus2(make_float2(x.x, x.y), make_float2(y.x, y.y));  // lanes l and l ^ 16
+        s[2 * i + 1] = plus2(make_float2(x.z, x.w), make_float2(y.z, y.w));
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; i++) s[i] = plus2(s[i], s[i + 4]);  // l ^ 8
+    s[0] = plus2(s[0], s[2]);                                  // l ^ 4
+    s[1] = plus2(s[1], s[3]);
+    s[0] = plus2(s[0], s[1]);                                  // l ^ 2
+    return s[0].x + s[0].y;                                    // l ^ 1
+}
+
 // Median bin of an instance histogram (seekThreshold64Kernel,
 // histogram64.cu:48-61): first bin whose cumulative count exceeds P/2.  Warp 0.
-__device__ __forceinline__ void hist_median(IterShared &sh, const int *hist, int nb, int P) {
+template <class Shared>
+__device__ __forceinline__ void hist_median(Shared &sh, const int *hist, int nb, int P) {
     if (threadIdx.x >= 32) return;
     int lane = threadIdx.x;
     int per = (nb + 31) / 32;
@@ -1263,7 +1450,7 @@ __device__ __forceinline__ void hist_median(IterShared &sh, const int *hist, int
 // One photometric iteration by a single 256-thread CTA (the allocation-free
 // entry point): residuals, histogram, median, weights and the fixed-point sums
 // of all P points; the 27 terms end in sh.A_ph.
-__device__ void photo_iteration(const InstDesc &d, IterShared &sh, int level) {
+__device__ void photo_iteration(const InstDesc &d, PhotoShared &sh, int level) {
     int P = d.P;
     int w = d.W >> level, h = d.H >> level;
     float a = 1.0f / (float)(1 << level);
@@ -1272,7 +1459,8 @@ __device__ void photo_iteration(const InstDesc &d, IterShared &sh, int level) {
     const float *I = d.sel_I[level];
     int nb = d.hist_bins;
     for (int k = threadIdx.x; k < nb; k += blockDim.x) sh.hist[k] = 0;
-    fx_clear(sh);
+    for (int k = threadIdx.x; k < kFxTerms; k += blockDim.x) (&sh.fx[0][0])[k] = 0;
+    if (threadIdx.x == 0) sh.fx_bad = 0;
     __syncthreads();
     for (int i = threadIdx.x; i < P; i += blockDim.x) {
         float r, zw;
@@ -1313,89 +1501,49 @@ __device__ void photo_iteration(const InstDesc &d, IterShared &sh, int level) {
     }
 }
 
-// The inputs of ICP pixel `idx` of the level: its last Student-t weight and
-// its reference point and normal (weight 0 past the end of the grid).  (A
-// packed 24-byte point + normal layout was measured: no change, the kernel is
-// bound by latency and issue, not by these bytes.)
-__device__ __forceinline__ void icp_load(const InstDesc &d, int level, int idx, int npix, float &weight, float4 &p,
-                                         float4 &rn) {
-    weight = 0.0f;
-    p = rn = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (idx < npix) {
-        weight = __ldg(d.icp_w + idx);
-        p = __ldg(d.ref_pts[level] + idx);
-        rn = __ldg(d.ref_nrm[level] + idx);
-    }
-}
-
-// icpResidualIndexKernel2, rgb2gray.cu:323-390, for one pixel of the level.  A
-// pixel that is not a correspondence has weight 0, and the reference's test
-// `weight > 0` then gives zeros.  The projection, the bilinear taps and the
-// correspondence test are the reference's expressions without contraction
-// (they decide which pixels count); the rotated normal, the residual and the
-// Jacobian, continuous terms of the normal equations only, are evaluated with
-// fused multiply-adds (one rounding per multiply-add; the oracle's
-// orc_icp_residual_jacobian_grid states the same sequence with fmaf).
-__device__ __forceinline__ void icp_point(const InstDesc &d, const float *T, int level, float weight, float4 p,
-                                          float4 rn, float *j, float &res) {
+// icpResidualIndexKernel2, rgb2gray.cu:323-390, for one pixel of the level from
+// its reference point p, normal n and weight, its transformed point q, the
+// projection (px, py) of q and the taps there; inside: the pixel has a weight
+// and q projects into the level (else, as in the reference, zeros).  The rotated
+// normal, the residual and the Jacobian, continuous terms of the normal equations
+// only, are evaluated with fused multiply-adds (one rounding per multiply-add;
+// the oracle's orc_icp_residual_jacobian_grid states the same sequence with fmaf).
+template <bool kDepth>
+__device__ __forceinline__ void icp_point(const IcpLevel &L, const float *T, float opt_in, float weight, const float *p,
+                                          const float *n, const float *q, float px, float py, bool inside,
+                                          const IcpTaps<kDepth> &t, float *j, float &res) {
     res = 0.0f;
 #pragma unroll
     for (int c = 0; c < 6; c++) j[c] = 0.0f;
-    if (!(weight > 0.0f)) return;
-    int w = d.W >> level, h = d.H >> level;
-    const float *K = d.calib + RC_KL;
-    float a = 1.0f / (float)(1 << level);
-    float b = 0.5f * (a - 1.0f);
-    float qx, qy, qz;
-    mul4(T, p.x, p.y, p.z, qx, qy, qz);
-    float q2x = qx / qz, q2y = qy / qz;
-    float p2x = a * (K[0] * q2x + K[2]) + b;
-    float p2y = a * (K[4] * q2y + K[5]) + b;
-    if (!(p2x >= 0 && p2x < (w - 1) && p2y >= 0 && p2y < (h - 1))) return;
-    int xdi = ftoi(p2x), ydi = ftoi(p2y);
-    float fx = p2x - xdi, fy = p2y - ydi;
-    int off2 = xdi + ydi * w;
-    float cx, cy, cz, m0, m1, m2, m3;
-    bilin_pts(d.cur_pts[level], off2, w, fx, fy, cx, cy, cz, m0, m1, m2, m3);
-    if (!(m0 != 0.0f && fabsf(cz - qz) < 300.0f)) return;
-    float optScaleIn = d.opt_in;
-    float rvx = cx - qx, rvy = cy - qy, rvz = cz - qz;
-    float cnx = __fmaf_rn(T[2], rn.z, __fmaf_rn(T[1], rn.y, T[0] * rn.x));
-    float cny = __fmaf_rn(T[6], rn.z, __fmaf_rn(T[5], rn.y, T[4] * rn.x));
-    float cnz = __fmaf_rn(T[10], rn.z, __fmaf_rn(T[9], rn.y, T[8] * rn.x));
-    res = optScaleIn * weight * __fmaf_rn(rvz, cnz, __fmaf_rn(rvy, cny, rvx * cnx));
+    float cx, cy, cz;
+    if (!(inside && t.first())) return;
+    icp_blend<kDepth>(L, t, px, py, cx, cy, cz);
+    if (!(fabsf(cz - q[2]) < 300.0f)) return;
+    float mx = __fmaf_rn(T[2], n[2], __fmaf_rn(T[1], n[1], T[0] * n[0]));
+    float my = __fmaf_rn(T[6], n[2], __fmaf_rn(T[5], n[1], T[4] * n[0]));
+    float mz = __fmaf_rn(T[10], n[2], __fmaf_rn(T[9], n[1], T[8] * n[0]));
+    float rx = cx - q[0], ry = cy - q[1], rz = cz - q[2];
+    res = opt_in * weight * __fmaf_rn(rz, mz, __fmaf_rn(ry, my, rx * mx));
     // The reference rotates the columns of [p]x and [n]x and the unit vectors
     // with full 3x3 products.  The terms it multiplies by an exact 0 or 1 are
     // dropped here: for a finite pose that changes at most the sign of a zero
     // Jacobian entry, and signed zeros add nothing to the fixed-point sums.
-    float b0x = __fmaf_rn(T[1], -p.z, T[2] * p.y), b0y = __fmaf_rn(T[5], -p.z, T[6] * p.y),
-          b0z = __fmaf_rn(T[9], -p.z, T[10] * p.y);
-    float b1x = __fmaf_rn(T[0], p.z, T[2] * -p.x), b1y = __fmaf_rn(T[4], p.z, T[6] * -p.x),
-          b1z = __fmaf_rn(T[8], p.z, T[10] * -p.x);
-    float b2x = __fmaf_rn(T[0], -p.y, T[1] * p.x), b2y = __fmaf_rn(T[4], -p.y, T[5] * p.x),
-          b2z = __fmaf_rn(T[8], -p.y, T[9] * p.x);
-    float n0x = __fmaf_rn(T[1], -rn.z, T[2] * rn.y), n0y = __fmaf_rn(T[5], -rn.z, T[6] * rn.y),
-          n0z = __fmaf_rn(T[9], -rn.z, T[10] * rn.y);
-    float n1x = __fmaf_rn(T[0], rn.z, T[2] * -rn.x), n1y = __fmaf_rn(T[4], rn.z, T[6] * -rn.x),
-          n1z = __fmaf_rn(T[8], rn.z, T[10] * -rn.x);
-    float n2x = __fmaf_rn(T[0], -rn.y, T[1] * rn.x), n2y = __fmaf_rn(T[4], -rn.y, T[5] * rn.x),
-          n2z = __fmaf_rn(T[8], -rn.y, T[9] * rn.x);
-    float so = -optScaleIn * weight;
-    // -cn . b + rv . n, accumulated left to right
-    auto row = [&](float bx, float by, float bz, float nx, float ny, float nz) {
-        float t = -cnx * bx;
-        t = __fmaf_rn(-cny, by, t);
-        t = __fmaf_rn(-cnz, bz, t);
-        t = __fmaf_rn(rvx, nx, t);
-        t = __fmaf_rn(rvy, ny, t);
-        return __fmaf_rn(rvz, nz, t);
+    // A row: -m . b + r . c with b = T_a p_a + T_b p_b, c likewise of n
+    auto row = [&](int a, float pa, float na, int b, float pb, float nb) {
+        float s = -mx * __fmaf_rn(T[a], pa, T[b] * pb);
+        s = __fmaf_rn(-my, __fmaf_rn(T[4 + a], pa, T[4 + b] * pb), s);
+        s = __fmaf_rn(-mz, __fmaf_rn(T[8 + a], pa, T[8 + b] * pb), s);
+        s = __fmaf_rn(rx, __fmaf_rn(T[a], na, T[b] * nb), s);
+        s = __fmaf_rn(ry, __fmaf_rn(T[4 + a], na, T[4 + b] * nb), s);
+        return __fmaf_rn(rz, __fmaf_rn(T[8 + a], na, T[8 + b] * nb), s);
     };
-    j[0] = so * row(b0x, b0y, b0z, n0x, n0y, n0z);
-    j[1] = so * row(b1x, b1y, b1z, n1x, n1y, n1z);
-    j[2] = so * row(b2x, b2y, b2z, n2x, n2y, n2z);
+    float so = -opt_in * weight;
+    j[0] = so * row(1, -p[2], -n[2], 2, p[1], n[1]);
+    j[1] = so * row(0, p[2], n[2], 2, -p[0], -n[0]);
+    j[2] = so * row(0, -p[1], -n[1], 1, p[0], n[0]);
 #pragma unroll
     for (int c = 0; c < 3; c++)
-        j[3 + c] = -weight * __fmaf_rn(-cnz, T[8 + c], __fmaf_rn(-cny, T[4 + c], -cnx * T[c]));
+        j[3 + c] = -weight * __fmaf_rn(-mz, T[8 + c], __fmaf_rn(-my, T[4 + c], -mx * T[c]));
 }
 
 // The arrays the photometric term reads: FP32, or (mixed precision) the FP16
@@ -1418,122 +1566,252 @@ template <> struct PhotoArrays<true> {
     static __device__ const __nv_bfloat16 *J(const InstDesc &d, int l) { return d.sel_Jb[l]; }
 };
 
-// Photometric residuals of lane t's 4 points of chunk c
-// (interpolateResidualKernel2, warp.cu:269-332).
-template <bool kMixed>
-__device__ __forceinline__ void photo_lane_residuals(const InstDesc &d, const float *T, int level, int c, int t,
-                                                     float *r, float *zw) {
-    int P = d.P;
-    int w = d.W >> level, h = d.H >> level;
-    float a = 1.0f / (float)(1 << level);
-    float b = 0.5f * (a - 1.0f);
-    const auto *img = PhotoArrays<kMixed>::img(d, level);
-    const auto *I = PhotoArrays<kMixed>::I(d, level);
+// Photometric residuals and depth weights of two points (interpolateResidualKernel2,
+// warp.cu:269-332, the expressions of photo_residual) in the halves of register
+// pairs: position p, keyframe intensity I.  Nothing branches on a point, so that
+// the taps and the depth taps of all the points a thread evaluates are in flight
+// together: the photometric term of a small batch is one chain of latencies.
+// Points that fall outside read the image's first pixel and are set afterwards.
+template <typename TImg>
+__device__ __forceinline__ void photo_pair(const PhotoConsts &k, float2 one, const float2 *p, float2 I, const TImg *img,
+                                           int w, int h, const float *zcur, int zw, int zh, float2 &res, float2 &zwt) {
+    auto map = [&](const float2 *M, const float2 *v, float2 *o) {
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-        int i = c * kChunk + t + kLanes * m;
-        photo_residual(d.calib, T, a, b, __ldg(d.sel_xyz + i), __ldg(d.sel_xyz + P + i), __ldg(d.sel_xyz + 2 * P + i),
-                       ldf(I + i), img, w, h, d.cur_z, d.W, d.H, r[m], zw[m]);
-    }
+        for (int i = 0; i < 3; i++)
+            o[i] = plus2(add2(mul2(M[4 * i + 2], v[2]), add2(mul2(M[4 * i + 1], v[1]), mul2(M[4 * i], v[0]), one), one),
+                         M[4 * i + 3]);
+    };
+    auto divide = [&](const float2 *v, float2 &x, float2 &y) {
+        float2 nz = mul2(v[2], dup2(-1.0f)), r = rcp_rn2(v[2]);
+        x = div_rn2(v[0], nz, r);
+        y = div_rn2(v[1], nz, r);
+        if (!div_in_range(v[0].x, v[1].x, v[2].x)) {
+            x.x = ieee_div(v[0].x, v[2].x);
+            y.x = ieee_div(v[1].x, v[2].x);
+        }
+        if (!div_in_range(v[0].y, v[1].y, v[2].y)) {
+            x.y = ieee_div(v[0].y, v[2].y);
+            y.y = ieee_div(v[1].y, v[2].y);
+        }
+    };
+    // float -> int truncation of a coordinate, as an index >= 0 (the fraction
+    // of a coordinate in (-1, 0) is itself: it truncates to 0)
+    auto whole = [](float2 v) { return index_sum2(make_float2(fmaxf(v.x, 0.0f), fmaxf(v.y, 0.0f))); };
+    float2 q[3], r[3], l[3], ux, uy, lx, ly;
+    map(k.T, p, q);
+    map(k.TLR, q, r);
+    divide(r, ux, uy);
+    // distortPoint
+    float2 r2 = add2(mul2(uy, uy), mul2(ux, ux), one), r4 = mul2(r2, r2), r6 = mul2(r4, r2);
+    float2 rad = add2(mul2(k.kc[2], r6), add2(mul2(k.kc[1], r4), add2(mul2(k.kc[0], r2), dup2(1.0f), one), one), one);
+    float2 dx = add2(mul2(mul2(k.KR[0], ux), rad), k.KR[1], one), dy = add2(mul2(mul2(k.KR[2], uy), rad), k.KR[3], one);
+    float2 px = add2(mul2(k.ab[0], dx), k.ab[1], one), py = add2(mul2(k.ab[0], dy), k.ab[1], one);
+    float wm1 = (float)(w - 1), hm1 = (float)(h - 1);
+    bool in0 = px.x > -1.0f && px.x < wm1 && py.x > -1.0f && py.x < hm1;
+    bool in1 = px.y > -1.0f && px.y < wm1 && py.y > -1.0f && py.y < hm1;
+    float2 sx = whole(px), sy = whole(py);
+    const TImg *a = img + (in0 ? index_of(sx.x) + index_of(sy.x) * w : 0);
+    const TImg *b = img + (in1 ? index_of(sx.y) + index_of(sy.y) * w : 0);
+    float2 t0 = make_float2(ldf(a), ldf(b)), t1 = make_float2(ldf(a + 1), ldf(b + 1));
+    float2 t2 = make_float2(ldf(a + w), ldf(b + w)), t3 = make_float2(ldf(a + w + 1), ldf(b + w + 1));
+    // the depth at the nearest IR pixel
+    map(k.TRL, r, l);
+    divide(l, lx, ly);
+    float2 vx = plus2(plus2(add2(mul2(k.KL[1], ly), mul2(k.KL[0], lx), one), k.KL[2]), dup2(0.5f));
+    float2 vy = plus2(plus2(add2(mul2(k.KL[4], ly), mul2(k.KL[3], lx), one), k.KL[5]), dup2(0.5f));
+    float zwf = (float)zw, zhf = (float)zh;
+    bool zin0 = in0 && vx.x > -1.0f && vx.x < zwf && vy.x > -1.0f && vy.x < zhf;
+    bool zin1 = in1 && vx.y > -1.0f && vx.y < zwf && vy.y > -1.0f && vy.y < zhf;
+    float2 ix = whole(vx), iy = whole(vy);
+    float2 zc = make_float2(__ldg(zcur + (zin0 ? index_of(ix.x) + index_of(iy.x) * zw : 0)),
+                            __ldg(zcur + (zin1 ? index_of(ix.y) + index_of(iy.y) * zw : 0)));
+    // bilinear tap and residual
+    float2 u = sub2(px, whole_of2(sx)), v = sub2(py, whole_of2(sy));
+    float2 gu = sub2(dup2(1.0f), u), gv = sub2(dup2(1.0f), v);
+    float2 col = add2(mul2(mul2(u, v), t3),
+                      add2(mul2(mul2(gu, v), t2), add2(mul2(mul2(u, gv), t1), mul2(mul2(gu, gv), t0), one), one), one);
+    res = sub2(I, col);
+    if (!in0) res.x = 1.0f;
+    if (!in1) res.y = 1.0f;
+    // 1 - (dz / 100)^2: the squared error over 1e4 by the exact division (below
+    // its range the quotient leaves 1 as it is, however it is rounded)
+    float2 e = sub2(zc, r[2]);
+    e = mul2(e, e);
+    float2 f = sub2(dup2(1.0f), div_rn2(e, dup2(-10000.0f), dup2(1.0f / 10000.0f)));
+    zwt.x = zin0 && e.x < 10000.0f ? f.x : 0.0f;
+    zwt.y = zin1 && e.y < 10000.0f ? f.y : 0.0f;
 }
 
 // The photometric term of an instance by its cluster of 8 CTAs: CTA `rank`
-// evaluates chunks rank, rank + 8, ...; the cluster adds its histograms
-// (histogram64.cu:115-145) through distributed shared memory, every CTA finds
-// the median bin (seekThreshold64Kernel, histogram64.cu:48-61) and weighs its
-// own points (generateWeights64Kernel, 79-94) into the CTA's fixed-point sums.
-// Returns whether this CTA had a chunk.
+// evaluates chunks rank, rank + 8, ...; every CTA writes its histogram
+// (histogram64.cu:115-145) into the others' shared memory, each finds the median
+// bin (seekThreshold64Kernel, histogram64.cu:48-61) and weighs its own points
+// (generateWeights64Kernel, 79-94) into the CTA's fixed-point sums.  In two
+// parts: `photo_begin` before the kernels ahead have finished (constants, and
+// the first chunk's points and Jacobian, which belong to the keyframe), the rest
+// after.
+struct PhotoLane {
+    float2 p[2][3], I[2];  // the lane's points t + 256 m of the first chunk, m and m + 1 a pair
+};
+
 template <bool kMixed>
-__device__ bool photo_cluster(const InstDesc &d, IterShared &sh, int level, int rank) {
+__device__ __forceinline__ void photo_load(const InstDesc &d, int level, int c, PhotoLane &o) {
+    const auto *I = PhotoArrays<kMixed>::I(d, level);
+#pragma unroll
+    for (int g = 0; g < 2; g++) {
+        int i = c * kChunk + threadIdx.x + 2 * g * kLanes;
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            o.p[g][k] = make_float2(__ldg(d.sel_xyz + k * d.P + i), __ldg(d.sel_xyz + k * d.P + i + kLanes));
+        o.I[g] = make_float2(ldf(I + i), ldf(I + i + kLanes));
+    }
+}
+
+// the Jacobian tile in shared memory, in its stored type: column k of point i
+// of the chunk at 1024 k + i (in 4-byte steps of 32 points, so that a warp's
+// points are the runs of its reduction for either type)
+template <typename TJ> __device__ __forceinline__ TJ *photo_tile(IterShared &sh, int col, int i) {
+    return reinterpret_cast<TJ *>(&sh.stage[col * kChunk + (i & ~31)]) + (i & 31);
+}
+
+template <bool kMixed>
+__device__ __forceinline__ void photo_begin(const InstDesc &d, IterShared &sh, int level, int rank, PhotoLane &o) {
     using TJ = typename PhotoArrays<kMixed>::TJ;
-    int P = d.P, nph = P / kChunk, nb = d.hist_bins;
-    int t = threadIdx.x, lane = t & 31;
-    const TJ *J = PhotoArrays<kMixed>::J(d, level);
-    // the Jacobian tile in shared memory, in its stored type (a BF16 tile uses
-    // the first half of sh.J)
-    TJ(*sJ)[kChunk] = reinterpret_cast<TJ(*)[kChunk]>(&sh.J[0][0]);
-    constexpr int kPer16 = 16 / sizeof(TJ);  // values per 16-byte copy
-    // the first chunk's Jacobian does not depend on the pose: copy it to shared
-    // memory asynchronously while the residuals are evaluated
-    if (rank < nph) {
+    int P = d.P, t = threadIdx.x;
+    cluster_arrive();  // awaited before the first write to another CTA's shared memory
+    if (rank < P / kChunk) {
+        photo_load<kMixed>(d, level, rank, o);
+        const TJ *J = PhotoArrays<kMixed>::J(d, level);
+        constexpr int kPer16 = 16 / sizeof(TJ);  // values per 16-byte copy
         for (int k = t; k < 6 * (kChunk / kPer16); k += blockDim.x) {
-            int col = k / (kChunk / kPer16), q = k % (kChunk / kPer16);
-            const TJ *src = J + (size_t)col * P + rank * kChunk + kPer16 * q;
-            unsigned int dst = (unsigned int)__cvta_generic_to_shared(&sJ[col][kPer16 * q]);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+            int col = k / (kChunk / kPer16), q = kPer16 * (k % (kChunk / kPer16));
+            const TJ *src = J + (size_t)col * P + rank * kChunk + q;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(photo_tile<TJ>(sh, col, q))),
+                         "l"(src)
+                         : "memory");
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
-    for (int k = t; k < nb; k += blockDim.x) sh.hist[k] = 0;
-    __syncthreads();
-    float r0[4], zw0[4];
+    sh.photo.set_level(d, level);
+    for (int k = t; k < d.hist_bins; k += blockDim.x) sh.hist[k] = 0;
+}
+
+// Returns whether this CTA had a chunk.
+template <bool kMixed>
+__device__ bool photo_cluster(const InstDesc &d, IterShared &sh, int level, int rank, PhotoLane &lane0, uint32_t *sums,
+                              int &bad) {
+    using TJ = typename PhotoArrays<kMixed>::TJ;
+    int P = d.P, nph = P / kChunk, nb = d.hist_bins;
+    int t = threadIdx.x, lane = t & 31;
+    int w = d.W >> level, h = d.H >> level;
+    const auto *img = PhotoArrays<kMixed>::img(d, level);
+    const float2 one = unseen_one();
+    float2 r0[2], zw0[2];
     for (int c = rank; c < nph; c += kCluster) {
-        float r[4], zw[4];
-        photo_lane_residuals<kMixed>(d, sh.T, level, c, t, r, zw);
+        if (c != rank) photo_load<kMixed>(d, level, c, lane0);
+        float2 r[2], zw[2];
 #pragma unroll
-        for (int m = 0; m < 4; m++) {
-            // one shared-memory atomic per distinct bin of the warp
-            int bin = mad_bin(r[m], nb);
-            unsigned int peers = __match_any_sync(kFull, bin);
-            if ((t & 31) == __ffs(peers) - 1) atomicAdd(&sh.hist[bin], __popc(peers));
+        for (int g = 0; g < 2; g++)
+            photo_pair(sh.photo, one, lane0.p[g], lane0.I[g], img, w, h, d.cur_z, d.W, d.H, r[g], zw[g]);
+#pragma unroll
+        for (int g = 0; g < 2; g++) {
+            atomicAdd(&sh.hist[mad_bin(r[g].x, nb)], 1);
+            atomicAdd(&sh.hist[mad_bin(r[g].y, nb)], 1);
             if (c == rank) {
-                r0[m] = r[m];
-                zw0[m] = zw[m];
+                r0[g] = r[g];
+                zw0[g] = zw[g];
             } else {  // later chunks of this CTA go through global scratch
-                int i = c * kChunk + t + kLanes * m;
-                d.ph_r[i] = r[m];
-                d.ph_zw[i] = zw[m];
+                int i = c * kChunk + t + 2 * g * kLanes;
+                d.ph_r[i] = r[g].x;
+                d.ph_r[i + kLanes] = r[g].y;
+                d.ph_zw[i] = zw[g].x;
+                d.ph_zw[i + kLanes] = zw[g].y;
             }
         }
     }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
-    cluster_arrive();
-    cluster_wait();  // every CTA's histogram is complete
+    cluster_wait();  // every CTA of the cluster has begun
     for (int k = t; k < nb; k += blockDim.x) {
-        int s = 0;
+        int v = sh.hist[k];
 #pragma unroll
-        for (int q = 0; q < kCluster; q++) s += *cluster_peer(&sh.hist[k], q);
-        sh.hist_all[k] = s;
+        for (int q = 0; q < kCluster; q++) *cluster_peer(&sh.peers[rank][k], q) = v;
     }
-    cluster_arrive();  // done reading the others' histograms; the wait is before this CTA leaves
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    cluster_arrive();
+    cluster_wait();  // every CTA's histogram is here (and no CTA touches another's memory from now on)
+    // thread k: the instance's count of bin k; the median bin is the first
+    // whose cumulative count exceeds P / 2
+    int cnt = 0;
+    if (t < nb) {
+#pragma unroll
+        for (int q = 0; q < kCluster; q++) cnt += sh.peers[q][t];
+    }
+    int incl = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+        int x = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += x;
+    }
+    if (lane == 31) sh.warp_tot[t >> 5] = incl;
+    if (t == 0) sh.median = 0;
     __syncthreads();
-    hist_median(sh, sh.hist_all, nb, P);
+#pragma unroll
+    for (int q = 0; q < kIterThreads / 32; q++)
+        if (q < (t >> 5)) incl += sh.warp_tot[q];
+    if (t < nb && incl > P / 2 && incl - cnt <= P / 2) sh.median = t;
     __syncthreads();
+    int median = sh.median;
     if (rank == 0) {
-        for (int k = t; k < nb; k += blockDim.x) d.ph_hist[256 + k] = sh.hist_all[k];  // for the trace
-        if (t == 0) d.ph_hist[512] = sh.median;
+        if (t < nb) d.ph_hist[256 + t] = cnt;  // for the trace
+        if (t == 0) d.ph_hist[512] = median;
     }
-    float s = mad_scale(sh.median, nb);
+    // Tukey weights with the divisions by the scale and by the constant exact
+    // (a quotient below the division's range leaves the weight as it is)
+    float sc = mad_scale(median, nb), rsc = rcp_rn(sc);
+    constexpr float kB = 4.6851f, kRb = 1.0f / 4.6851f;
+    auto weight = [&](float2 r, float2 zw) {
+        float2 u = div_rn2(make_float2(fabsf(r.x), fabsf(r.y)), dup2(-sc), dup2(rsc));
+        float2 ub = div_rn2(u, dup2(-kB), dup2(kRb));
+        float2 v = mul2(sub2(dup2(1.0f), mul2(ub, ub)), zw);
+        return make_float2(u.x <= kB ? v.x : 0.0f, u.y <= kB ? v.y : 0.0f);
+    };
+    const TJ *J = PhotoArrays<kMixed>::J(d, level);
     for (int c = rank; c < nph; c += kCluster) {
         float acc[27];
 #pragma unroll
         for (int q = 0; q < 27; q++) acc[q] = 0.0f;
 #pragma unroll
-        for (int m = 0; m < 4; m++) {
-            int i = c * kChunk + t + kLanes * m;
-            float r, zw, jv[6];
+        for (int g = 0; g < 2; g++) {
+            int i = t + 2 * g * kLanes;
+            float2 r, zw, j[6];
             if (c == rank) {
-                r = r0[m];
-                zw = zw0[m];
+                r = r0[g];
+                zw = zw0[g];
 #pragma unroll
-                for (int k = 0; k < 6; k++) jv[k] = (float)sJ[k][t + kLanes * m];
+                for (int k = 0; k < 6; k++)
+                    j[k] = make_float2((float)*photo_tile<TJ>(sh, k, i), (float)*photo_tile<TJ>(sh, k, i + kLanes));
             } else {
-                r = d.ph_r[i];  // written by this thread above
-                zw = d.ph_zw[i];
+                int x = c * kChunk + i;  // written by this thread above
+                r = make_float2(d.ph_r[x], d.ph_r[x + kLanes]);
+                zw = make_float2(d.ph_zw[x], d.ph_zw[x + kLanes]);
 #pragma unroll
-                for (int k = 0; k < 6; k++) jv[k] = ldf(J + k * P + i);
+                for (int k = 0; k < 6; k++) j[k] = make_float2(ldf(J + k * P + x), ldf(J + k * P + x + kLanes));
             }
-            float wv = tukey_weight(r, zw, s);
-            float jw[6];
+            float2 wv = weight(r, zw);
+            r = mul2(r, wv);
+            float a[6];
 #pragma unroll
-            for (int k = 0; k < 6; k++) jw[k] = jv[k] * wv;
-            acc27(acc, jw, r * wv);
+            for (int k = 0; k < 6; k++) {
+                j[k] = mul2(j[k], wv);
+                a[k] = j[k].x;
+            }
+            acc27(acc, a, r.x);
+#pragma unroll
+            for (int k = 0; k < 6; k++) a[k] = j[k].y;
+            acc27(acc, a, r.y);
         }
-        float v = warp_terms(acc);
-        if (lane < 27) fx_add_term(sh, lane, v);
+        fx_accumulate(sums, warp_terms(acc, sh.stage + (t & ~31)), bad);
     }
-    cluster_wait();
     return rank < nph;
 }
 
@@ -1548,62 +1826,87 @@ __device__ __forceinline__ void prefetch_l2(const void *p, unsigned bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(g), "r"(bytes) : "memory");
 }
 
-// Prefetches what ICP chunk c of the level reads: its reference points,
-// normals and weights (contiguous streams) and the rows of the current point
-// cloud that its bilinear taps read at small motion (the chunk's own rows and
-// the one below).  Issued by one thread, a chunk ahead of its use.
+// Prefetches what ICP chunk c of the level reads: its reference planes and
+// weights (contiguous) and the rows of the current points that its taps read at
+// small motion (the chunk's own rows and the one below).  Issued by one thread,
+// a chunk ahead of its use.
 __device__ __forceinline__ void icp_prefetch_chunk(const InstDesc &d, int level, int c, int npix) {
-    int i0 = c * kChunk;
-    if (c < 0 || i0 >= npix) return;
-    int n = min(kChunk, npix - i0);
-    prefetch_l2(d.ref_pts[level] + i0, (unsigned)n * 16u);
-    prefetch_l2(d.ref_nrm[level] + i0, (unsigned)n * 16u);
-    prefetch_l2(d.icp_w + i0, (unsigned)n * 4u);
-    int w = d.W >> level, h = d.H >> level;
-    int y0 = i0 / w, y1 = min((i0 + n - 1) / w + 1, h - 1);
-    prefetch_l2(d.cur_pts[level] + (size_t)y0 * w, (unsigned)((y1 - y0 + 1) * w) * 16u);
+    int w = d.W >> level, h = d.H >> level, i0 = c * kChunk;
+    if (i0 >= npix) return;
+    prefetch_l2(d.ref_pl[level] + (size_t)c * 6 * kChunk, 6 * kChunk * 4);
+    prefetch_l2(d.icp_w + i0, kChunk * 4);
+    int y0 = i0 / w, y1 = min((min(i0 + kChunk, npix) - 1) / w + 1, h - 1);
+    size_t first = (size_t)y0 * w, count = (size_t)(y1 - y0 + 1) * w;
+    if (level == 0) {
+        size_t down = first & 3;  // to a 16-byte boundary
+        prefetch_l2(d.cur_z + first - down, (unsigned)(count + down) * 4u);
+    } else {
+        prefetch_l2(d.cur_pts[level] + first, (unsigned)count * 16u);
+    }
 }
 
 // ICP chunks [c0, c1) of 1024 pixels of the level: lane t evaluates pixels
-// t + 256m of each chunk (icpResidualIndexKernel2 and the reference's per-point
-// Jacobian), the warp totals of each chunk go into the CTA's fixed-point sums.
-__device__ void icp_chunks(const InstDesc &d, IterShared &sh, int level, int c0, int c1, int npix) {
-    int t = threadIdx.x, lane = t & 31;
+// t + 256m of each chunk, kBatch at a time with their inputs and then their taps
+// in flight together, and leaves their terms in its own slots; the canonical
+// per-lane sums then take them in pixel order, and the warp totals of each chunk
+// go into the fixed-point sums that lane q keeps of term q.
+template <bool kDepth>
+__device__ void icp_chunks(const InstDesc &d, IterShared &sh, int level, int c0, int c1, int npix, uint32_t *sums,
+                           int &bad) {
+    // depths leave the registers for two pixels' taps at once (125 against 136 us
+    // a level-0 launch of 30 instances), points do not (52 against 54 at level 1)
+    constexpr int kBatch = kDepth ? 2 : 1;
+    int t = threadIdx.x;
+    const IcpLevel L(d, level);
+    const float opt_in = d.opt_in;
+    float *slot = sh.stage + t;
     for (int c = c0; c < c1; c++) {
         if (t == 0 && c + 1 < c1) icp_prefetch_chunk(d, level, c + 1, npix);
-        // Phase 1: the lane's four pixels with no accumulators live; each
-        // result goes to the lane's own shared slots.
+        const float *ref = d.ref_pl[level] + (size_t)c * 6 * kChunk + t, *wts = d.icp_w + c * kChunk + t;
+        // in registers: read from shared memory it would be read again after every
+        // store to the slots (124 against 131 us at level 0 of 30 instances)
+        float T[12];
 #pragma unroll
-        for (int g = 0; g < 2; g++) {
-            // two pixels at a time: both loads in flight, then both evaluated
-            float w[2];
-            float4 p[2], n[2];
+        for (int k = 0; k < 12; k++) T[k] = sh.T[k];
 #pragma unroll
-            for (int u = 0; u < 2; u++) icp_load(d, level, c * kChunk + t + kLanes * (2 * g + u), npix, w[u], p[u], n[u]);
+        for (int g = 0; g < 4; g += kBatch) {
+            IcpTaps<kDepth> tap[kBatch];
+            float p[kBatch][6], w[kBatch], q[kBatch][3], px[kBatch], py[kBatch];
+            bool in[kBatch];
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                int m = 2 * g + u;
+            for (int u = 0; u < kBatch; u++) {
+                w[u] = __ldg(wts + (g + u) * kLanes);
+#pragma unroll
+                for (int k = 0; k < 6; k++) p[u][k] = __ldg(ref + k * kChunk + (g + u) * kLanes);
+            }
+#pragma unroll
+            for (int u = 0; u < kBatch; u++) {
+                mul4(T, p[u][0], p[u][1], p[u][2], q[u][0], q[u][1], q[u][2]);
+                in[u] = w[u] > 0.0f && icp_project(L, q[u][0], q[u][1], q[u][2], px[u], py[u]);
+                tap[u].load(L, icp_tap_index(L, in[u], px[u], py[u]));
+            }
+#pragma unroll
+            for (int u = 0; u < kBatch; u++) {
                 float j[6], r;
-                icp_point(d, sh.T, level, w[u], p[u], n[u], j, r);
+                icp_point<kDepth>(L, T, opt_in, w[u], p[u], p[u] + 3, q[u], px[u], py[u], in[u], tap[u], j, r);
+                float *v = slot + (g + u) * kLanes;
 #pragma unroll
-                for (int k = 0; k < 6; k++) sh.J[k][t + kLanes * m] = j[k];
-                sh.R[t + kLanes * m] = r;
+                for (int k = 0; k < 6; k++) v[k * kChunk] = j[k];
+                v[6 * kChunk] = r;
             }
         }
-        // Phase 2: the canonical per-lane sums in point order, from the slots
-        // this thread wrote (no barrier needed).
         float acc[27];
 #pragma unroll
-        for (int q = 0; q < 27; q++) acc[q] = 0.0f;
+        for (int k = 0; k < 27; k++) acc[k] = 0.0f;
 #pragma unroll
         for (int m = 0; m < 4; m++) {
+            const float *v = slot + m * kLanes;
             float j[6];
 #pragma unroll
-            for (int k = 0; k < 6; k++) j[k] = sh.J[k][t + kLanes * m];
-            acc27(acc, j, sh.R[t + kLanes * m]);
+            for (int k = 0; k < 6; k++) j[k] = v[k * kChunk];
+            acc27(acc, j, v[6 * kChunk]);
         }
-        float v = warp_terms(acc);
-        if (lane < 27) fx_add_term(sh, lane, v);
+        fx_accumulate(sums, warp_terms(acc, sh.stage + (t & ~31)), bad);
     }
 }
 
@@ -1745,6 +2048,18 @@ __device__ __forceinline__ void finalize_iter(const InstDesc &d, SolveShared &sh
 // atomics, so the result does not depend on K or on the order in which CTAs
 // finish; k_solve then fuses, solves and updates the pose.
 //
+// What bounds it: at the fine levels the FP32 issue of about 300 operations a
+// pixel with the latency of its taps (a level-0 launch of 30 640x480 instances
+// reads 32 bytes a pixel, 44 us at the measured HBM rate, and takes 125 us,
+// 148 us before; level 1 52 us, before 57), at the coarse levels and for a single
+// instance the photometric chain (level 3 of 30 instances 15 us, before 18; a 320x240
+// photometric iteration with its solve 17.0 us, before 21.7).  Measured and not kept: two
+// pixels in packed arithmetic with the pose in shared memory (135 us: a third fewer
+// instructions, but the constants' loads and 80 registers), inputs copied two
+// blocks ahead into shared memory (3 CTAs an SM, of which clusters of 8 leave 11% of
+// the slots empty: 134 us), one share of the blocks for each resident CTA (151 us:
+// CTAs on SMs with fewer neighbours finish early).
+//
 // Even iterations visit the instances, and the chunks within each, in reverse
 // order (CTAs start roughly in block order): a level-0 pass streams several
 // times L2's capacity, and the lines it touched last (or k_icp_mask touched
@@ -1768,50 +2083,58 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kIterThreads,
         if (slot >= n_inst) return;  // rounding of the grid to whole clusters
     }
     __shared__ InstDesc sd;
+    __shared__ IterShared sh;
     load_desc(sd, D + (rev ? n_inst - 1 - slot : slot));
     __syncthreads();
     const InstDesc &d = sd;
     if (level >= d.L) return;
     if (it >= d.iters[d.L - 1 - level]) return;
-    if (role >= kCluster && threadIdx.x == 0 && d.mode != RECON_PHOTOMETRIC) {
-        // the first chunk's inputs, while the previous kernel finishes
-        int np = (d.W >> level) * (d.H >> level);
-        int nall = ((np + kChunk - 1) / kChunk + icp_per_cta - 1) / icp_per_cta;
-        int jj = role - kCluster;
-        if (jj < nall) icp_prefetch_chunk(d, level, (rev ? nall - 1 - jj : jj) * icp_per_cta, np);
-    }
-    pdl_wait();
-    // the instance left this level early (settle rule; uniform over a cluster)
-    if (d.settle_mm > 0.0f && __ldcg(d.stats + ST_SETTLED) == level + 1) return;
-    bool use_ph = d.mode != RECON_GEOMETRIC;
-    bool use_icp = d.mode != RECON_PHOTOMETRIC;
-    int nsel = use_icp ? __ldcg(d.icp_nsel + level) : 0;
+    const bool icp = role >= kCluster;
+    if (icp ? d.mode == RECON_PHOTOMETRIC : d.mode == RECON_GEOMETRIC) return;
     int npix = (d.W >> level) * (d.H >> level);
     int nchunks = (npix + kChunk - 1) / kChunk;
-    int nicp = nsel > 0 ? (nchunks + icp_per_cta - 1) / icp_per_cta : 0;
-    int set;  // which sums this CTA adds to: 0 photometric, 1 ICP
-    if (role < kCluster) {
-        if (!use_ph) return;
-        set = 0;
-    } else {
-        if (role - kCluster >= nicp) return;
-        set = 1;
+    int nicp = (nchunks + icp_per_cta - 1) / icp_per_cta;
+    int j = role - kCluster;
+    if (icp && j >= nicp) return;
+    int c0 = (rev ? nicp - 1 - j : j) * icp_per_cta, c1 = min(c0 + icp_per_cta, nchunks);
+    // what does not depend on the kernels before: the first chunk's inputs into
+    // L2, or the photometric term's constants, points and Jacobian
+    if (icp && threadIdx.x == 0) icp_prefetch_chunk(d, level, c0, npix);
+    const bool mixed = d.precision == RECON_PRECISION_MIXED;
+    PhotoLane first;
+    if (!icp) {
+        if (mixed) photo_begin<true>(d, sh, level, role, first);
+        else photo_begin<false>(d, sh, level, role, first);
     }
-    __shared__ IterShared sh;
-    if (threadIdx.x < 16) sh.T[threadIdx.x] = __ldcg(d.T + threadIdx.x);
-    fx_clear(sh);
+    if (threadIdx.x == 0) sh.bad = 0;
+    pdl_wait();
+    float pose = threadIdx.x < 16 ? __ldcg(d.T + threadIdx.x) : 0.0f;
+    // the instance left this level early (settle rule; uniform over a cluster),
+    // or it has no correspondence there
+    bool skip = d.settle_mm > 0.0f && __ldcg(d.stats + ST_SETTLED) == level + 1;
+    if (icp && __ldcg(d.icp_nsel + level) <= 0) skip = true;
+    if (threadIdx.x < 16) sh.T[threadIdx.x] = pose;
+    if (!icp) sh.photo.set_pose(pose);
     __syncthreads();
-    if (set == 0) {
-        bool had = d.precision == RECON_PRECISION_MIXED ? photo_cluster<true>(d, sh, level, role)
-                                                        : photo_cluster<false>(d, sh, level, role);
+    if (skip) {
+        if (!icp) {
+            cluster_wait();
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
+        }
+        return;
+    }
+    uint32_t sums[kFxLimbs] = {0u, 0u, 0u, 0u};
+    int bad = 0;
+    if (icp) {
+        if (level == 0) icp_chunks<true>(d, sh, level, c0, c1, npix, sums, bad);
+        else icp_chunks<false>(d, sh, level, c0, c1, npix, sums, bad);
+    } else {
+        bool had = mixed ? photo_cluster<true>(d, sh, level, role, first, sums, bad)
+                         : photo_cluster<false>(d, sh, level, role, first, sums, bad);
         if (!had) return;
-    } else {
-        int j = role - kCluster;
-        int c0 = (rev ? nicp - 1 - j : j) * icp_per_cta;
-        icp_chunks(d, sh, level, c0, min(c0 + icp_per_cta, nchunks), npix);
     }
-    __syncthreads();
-    fx_flush(sh, d.fx + set * kFxTerms, d.fx_bad + set);
+    int set = icp ? 1 : 0;  // which sums this CTA adds to: 0 photometric, 1 ICP
+    fx_flush(sh, sums, bad, d.fx + set * kFxTerms, d.fx_bad + set);
 }
 
 // The rest of a GN iteration, one CTA per instance after k_iter: the normal
@@ -1872,24 +2195,22 @@ __device__ __forceinline__ void student_body(const InstDesc *D, int level) {
         if (t < 16) sT[t] = __ldcg(d.T + t);
         if (rank == 0 && t == 0) d.work[2] += (unsigned long long)n;
         __syncthreads();
+        const IcpLevel L(d, level);
+        const float *pl = d.ref_pl[level];
         for (int i0 = rank * kStudentThreads + t; i0 < n; i0 += 2 * stride) {
             // two pixels at a time: point and normal loads in flight together
-            float4 p[2], rn[2];
+            float p[2][6];
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                int i = i0 + u * stride;
-                p[u] = rn[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (i < n) {
-                    p[u] = __ldg(d.ref_pts[level] + i);
-                    rn[u] = __ldg(d.ref_nrm[level] + i);
-                }
-            }
+            for (int u = 0; u < 2; u++)
+#pragma unroll
+                for (int k = 0; k < 6; k++)
+                    p[u][k] = i0 + u * stride < n ? __ldg(pl + ref_plane(i0 + u * stride, k)) : 0.0f;
 #pragma unroll
             for (int u = 0; u < 2; u++) {
                 int i = i0 + u * stride;
                 if (i >= n) continue;
                 float r2;
-                uint8_t ok = icp_mask_pixel(d, sT, level, p[u], rn[u], r2);
+                bool ok = level == 0 ? icp_mask_pixel<true>(L, sT, p[u], r2) : icp_mask_pixel<false>(L, sT, p[u], r2);
                 if (ok) v += trunc_prod(r2, student_w(r2, 100.0f));
                 d.icp_r2[i] = r2;
                 d.icp_mask[i] = ok;
@@ -1963,7 +2284,11 @@ __device__ __forceinline__ void student_body(const InstDesc *D, int level) {
                 vsum += trunc_prod(r, student_w(r, sigma2));
             }
         }
-        if (pass == 3) break;
+        if (pass == 3) {
+            // zero up to the end of the level's last block
+            for (int k = n + rank * kStudentThreads + t; k < (n + kChunk - 1) / kChunk * kChunk; k += stride) d.icp_w[k] = 0.0f;
+            break;
+        }
         for (int o = 16; o > 0; o >>= 1) vsum += __shfl_xor_sync(0xffffffffu, vsum, o);
         if (lane == 0) warp_sum[wid] = vsum;
         __syncthreads();
@@ -2190,7 +2515,7 @@ constexpr int kNoAllocMaxPoints = RECON_NOALLOC_MAX_POINTS;
 static __device__ __align__(256) float g_noalloc_scratch[2 * kNoAllocMaxPoints];
 
 __global__ void __launch_bounds__(256) k_photo_iter_noalloc(recon_photo_view v, float *scratch, float *T) {
-    __shared__ IterShared sh;
+    __shared__ PhotoShared sh;
     __shared__ InstDesc d;  // view of the caller's buffers in the layout photo_iteration reads
     if (threadIdx.x == 0) {
         d.W = v.depth_width;

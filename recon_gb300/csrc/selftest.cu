@@ -1,11 +1,12 @@
 // selftest.cu -- compares the truncation of the Student-t variance sums
-// (exact_arith.cuh) with the conversion it replaces, on the GPU the library
-// runs on.
+// (exact_arith.cuh) with the conversion it replaces, and the reciprocal and
+// division of pair_math.cuh with the compiler's, on the GPU the library runs on.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "../../include/recon_track.h"
 #include "exact_arith.cuh"
+#include "pair_math.cuh"
 
 namespace rt {
 
@@ -29,29 +30,84 @@ __global__ void k_check_trunc(unsigned long long *bad) {
     add_count(bad, c);
 }
 
+// every mantissa at the ends and the middle of the range, both signs: the
+// reciprocal against the correctly rounded one
+__global__ void k_check_rcp(unsigned long long *bad) {
+    unsigned long long c = 0;
+    uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < 0x800000u; m += stride)
+        for (uint32_t E = 127 - 60; E < 127 + 60; E += 20)
+            for (uint32_t sign = 0; sign < 2; sign++) {
+                float b = __uint_as_float(sign << 31 | E << 23 | m), y = __frcp_rn(b);
+                float2 y2 = rcp_rn2(dup2(b));
+                c += rcp_rn(b) != y || y2.x != y || y2.y != y;
+            }
+    add_count(bad, c);
+}
+
+// pseudo-random operands of the range (a linear congruential sequence a
+// thread): quotients against the compiler's division, and packed sums and
+// differences of products against separately rounded ones
+__global__ void k_check_div(unsigned long long *bad, int per_thread) {
+    unsigned long long c = 0, s = (blockIdx.x * blockDim.x + threadIdx.x) * 0x9E3779B97F4A7C15ull + 12345;
+    auto next = [&]() {
+        s = s * 6364136223846793005ull + 1442695040888963407ull;
+        uint32_t r = (uint32_t)(s >> 32);
+        s = s * 6364136223846793005ull + 1442695040888963407ull;
+        return __uint_as_float((r & 0x807fffffu) | ((127u - 60u + (uint32_t)(s >> 40) % 120u) << 23));
+    };
+    for (int i = 0; i < per_thread; i++) {
+        float a0 = next(), a1 = next(), b = next();
+        float2 q = div_rn2(make_float2(a0, a1), dup2(-b), rcp_rn2(dup2(b)));
+        // a product and a sum stay two roundings
+        float2 s2 = add2(mul2(make_float2(a0, a1), dup2(b)), make_float2(a1, a0), unseen_one());
+        float2 d2 = sub2(make_float2(a1, a0), mul2(make_float2(a0, a1), dup2(b)));
+        c += s2.x != __fadd_rn(__fmul_rn(a0, b), a1) || s2.y != __fadd_rn(__fmul_rn(a1, b), a0);
+        c += d2.x != __fsub_rn(a1, __fmul_rn(a0, b)) || d2.y != __fsub_rn(a0, __fmul_rn(a1, b));
+        c += !div_in_range(a0, a1, b) || div_rn(a0, -b, rcp_rn(b)) != a0 / b || q.x != a0 / b || q.y != a1 / b;
+    }
+    add_count(bad, c);
+}
+
 }  // namespace
 }  // namespace rt
 
-extern "C" int recon_selftest_exact_arith(int64_t *mismatches) {
-    using namespace rt;
+namespace {
+
+// runs `launch` on a zeroed counter and returns the count
+template <class Launch> int count_mismatches(int64_t *mismatches, const char *name, Launch launch) {
     if (!mismatches) {
-        set_last_error("recon_selftest_exact_arith: null argument");
+        rt::set_last_error(name);
         return RECON_ERR_INVALID_ARG;
     }
     unsigned long long *d = nullptr;
     cudaError_t e = cudaMalloc(&d, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(d, 0, sizeof(unsigned long long));
     if (e == cudaSuccess) {
-        k_check_trunc<<<152 * 8, 256>>>(d);
+        launch(d);
         e = cudaGetLastError();
     }
     unsigned long long h = 0;
     if (e == cudaSuccess) e = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost);
     if (d) cudaFree(d);
     if (e != cudaSuccess) {
-        set_last_error(cudaGetErrorString(e));
+        rt::set_last_error(cudaGetErrorString(e));
         return RECON_ERR_CUDA;
     }
     *mismatches = (int64_t)h;
     return RECON_OK;
+}
+
+}  // namespace
+
+extern "C" int recon_selftest_exact_arith(int64_t *mismatches) {
+    return count_mismatches(mismatches, "recon_selftest_exact_arith: null argument",
+                            [](unsigned long long *d) { rt::k_check_trunc<<<152 * 8, 256>>>(d); });
+}
+
+extern "C" int recon_selftest_division(int64_t *mismatches) {
+    return count_mismatches(mismatches, "recon_selftest_division: null argument", [](unsigned long long *d) {
+        rt::k_check_rcp<<<152 * 8, 256>>>(d);
+        rt::k_check_div<<<152 * 8, 256>>>(d, 4000);
+    });
 }

@@ -41,6 +41,10 @@ struct InstDesc {
     float *ref_col;               // W*H fused vertex colour (keyframe fusion), -1 where none
     float4 *ref_pts[kMaxLevels];  // x y z mask
     float4 *ref_nrm[kMaxLevels];  // nx ny nz 0
+    // the same for the ICP kernels, in blocks of 1024 pixels (ref_plane):
+    // [pixels / 1024][6][1024], x y z nx ny nz, z NaN where the pixel has no
+    // point; zero past the level's last pixel
+    float *ref_pl[kMaxLevels];
     float *gmag;                  // W*H: the keyframe pixels' gradient magnitudes
     int *grad_hist;               // select_bins
     int *seg;                     // segment tables, 6 * kSegments + 4
@@ -56,14 +60,14 @@ struct InstDesc {
     // current frame
     float *cur_gray[kMaxLevels];
     float *cur_z;
-    float4 *cur_pts[kMaxLevels];  // x y z mask
+    float4 *cur_pts[kMaxLevels];  // x y z mask; level 0 is not stored (formed from cur_z where it is read)
     // photometric scratch
     float *ph_r, *ph_zw;
     int *ph_hist;     // [256,512) the last histogram (for the trace), [512] its median bin
     // ICP scratch
     uint8_t *icp_mask;       // W*H: the pixel is a correspondence of the level
     float *icp_r2;           // W*H: its squared residual at the level's start pose
-    float *icp_w;            // W*H: its Student-t weight, 0 where not selected
+    float *icp_w;            // W*H: its Student-t weight, 0 where not selected and up to the end of the level's last block
     int *icp_blkcnt;         // per 1024-pixel block: correspondences
     long long *icp_blkvar;   // per 1024-pixel block: first variance sum
     long long *icp_part;     // per Student-t pass CTA (at most one per block): its partial sum
@@ -81,6 +85,9 @@ struct InstDesc {
     int trace_max;
     int *trace_count;
 };
+
+// Plane k of pixel i in a level's ref_pl
+__host__ __device__ constexpr size_t ref_plane(int i, int k) { return (size_t)(i / kChunk * 6 + k) * kChunk + i % kChunk; }
 
 // Programmatic dependent launch.  The kernels of the per-frame schedule are
 // launched so that the next kernel may start while this one finishes:

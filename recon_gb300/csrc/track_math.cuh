@@ -185,20 +185,4 @@ __device__ __forceinline__ void photo_residual(const float *calib, const float *
     zweight = zWeight;
 }
 
-// bilinearInterpolation6 of float4 (x,y,z,mask) cloud taps, kernelUtils.h:305-316
-__device__ __forceinline__ void bilin_pts(const float4 *cur, int off2, int width, float fx, float fy, float &cx,
-                                          float &cy, float &cz, float &m00, float &m10, float &m01, float &m11) {
-    float4 v0 = __ldg(cur + off2);
-    float4 v1 = __ldg(cur + off2 + 1);
-    float4 v2 = __ldg(cur + off2 + width);
-    float4 v3 = __ldg(cur + off2 + width + 1);
-    cx = (1 - fx) * (1 - fy) * v0.x + fx * (1 - fy) * v1.x + (1 - fx) * fy * v2.x + fx * fy * v3.x;
-    cy = (1 - fx) * (1 - fy) * v0.y + fx * (1 - fy) * v1.y + (1 - fx) * fy * v2.y + fx * fy * v3.y;
-    cz = (1 - fx) * (1 - fy) * v0.z + fx * (1 - fy) * v1.z + (1 - fx) * fy * v2.z + fx * fy * v3.z;
-    m00 = v0.w;
-    m10 = v1.w;
-    m01 = v2.w;
-    m11 = v3.w;
-}
-
 }  // namespace rt
