@@ -20,7 +20,7 @@
 //    records whether any voxel of the brick may be negative; the traversal
 //    steps through bricks without one using only its step arithmetic (the
 //    reference's coarse test, tsdf < 0, cannot pass there), so empty space
-//    costs no grid reads.  The byte is set whenever a negative value is
+//    costs no grid reads, and many such bricks are crossed at one go.  The byte is set whenever a negative value is
 //    stored and cleared only by a reset or a rebuild, so it never hides a
 //    negative voxel.
 //  * where the reference would read past the end of the grid array (its
@@ -30,6 +30,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
 #include <cmath>
 #include <string>
 #include <utility>
@@ -37,6 +38,7 @@
 
 #include "../../include/recon_track.h"
 #include "../../include/recon_tsdf.h"
+#include "pair_math.cuh"
 
 namespace rt {
 void set_last_error(const char *msg);
@@ -51,6 +53,8 @@ constexpr int kTileY = 8;
 constexpr int kRunZ = 8;
 constexpr int kRayTileX = 8;  // ray cast CTA: one warp on 8 x 4 pixels (rays differ widely in length;
 constexpr int kRayTileY = 4;  // one-warp CTAs let the block scheduler balance the SMs)
+constexpr int kRayCtas = 28;  // ray cast CTAs per SM: 72 registers.  32 (64 registers) spill more and 24 leave fewer
+                              // rays to switch between: 796, 779 and 791 us for six 640x480 frames on a 256^3 grid
 constexpr int kKinds = 5;     // timing kinds: update, ray cast, shading, distance map, reset / resample
 
 struct Geom {
@@ -65,6 +69,8 @@ struct Geom {
     float ib0x, ib0y, ib0z;         // interpolation origin
     float ivx, ivy, ivz;            // 1 / voxel spacing (voxelize's invVoxelDim)
     float min_dist, max_dist;
+    int mirror;      // 2^k - 1 >= R - 1
+    int exact_walk;  // every corner coordinate of a voxel walk is an exact sum
 };
 
 __device__ __forceinline__ unsigned f2u(float v) { return __float2uint_rz(v); }
@@ -228,8 +234,9 @@ __device__ __forceinline__ bool sample(const float2 *__restrict__ grid, const Ge
 __device__ __forceinline__ int empty_level(const uint8_t *__restrict__ flags, const Geom &g, int x, int y, int z) {
     const unsigned R = (unsigned)g.R;
     if (!((unsigned)x < R && (unsigned)y < R && (unsigned)z < R)) return 0;
-    if (__ldg(flags + super_of(g, x, y, z)) == 0) return 2;
-    return __ldg(flags + brick_of(g, x, y, z)) == 0 ? 1 : 0;
+    // both bytes are asked for at once: the second is no slower than the first
+    const uint8_t sup = __ldg(flags + super_of(g, x, y, z)), brick = __ldg(flags + brick_of(g, x, y, z));
+    return sup == 0 ? 2 : (brick == 0 ? 1 : 0);
 }
 
 // traverseVoxelsCuda's fine search once the coarse test passed
@@ -237,65 +244,141 @@ __device__ __forceinline__ int empty_level(const uint8_t *__restrict__ flags, co
 // trilinear value at the voxel is not negative (the traversal goes on)
 __device__ __forceinline__ int refine(const float2 *__restrict__ grid, const Geom &g, const Ray &r, float ivx,
                                       float ivy, float ivz, float vpx, float vpy, float vpz, float enterT,
-                                      float exitT, int iter, int max_back, float *t_hit) {
+                                      float exitT, int iter, int max_back, unsigned rays, float *t_hit) {
     const float dv = (vpx - r.ox) * r.dx + (vpy - r.oy) * r.dy + (vpz - r.oz) * r.dz;
     float t1 = fmaxf(enterT, fminf(dv, exitT));
     float e1;
-    if (!sample(grid, g, r, ivx, ivy, ivz, t1, &e1)) return 0;
-    if (!(e1 < 0.0f)) return 2;
-    float t0 = t1 - g.vx2 / 2;
-    int back = 0;
-    while (t0 > enterT) {
-        if (++back > max_back) return 0;
-        float e0;
-        if (!sample(grid, g, r, ivx, ivy, ivz, t0, &e0)) return 0;
-        if (e0 > 0.0f) {
-            float tx = linear_zero(t0, e0, t1, e1);
-            while (iter > 0) {
-                float ex;
-                if (!sample(grid, g, r, ivx, ivy, ivz, tx, &ex)) return 0;
-                if (ex < 0.0f) {
-                    t1 = tx;
-                    e1 = ex;
-                } else {
-                    t0 = tx;
-                    e0 = ex;
-                }
-                tx = linear_zero(t0, e0, t1, e1);
-                iter--;
-            }
-            *t_hit = tx;
-            return 1;
-        } else if (e0 > e1) {
+    int result = 0;
+    if (sample(grid, g, r, ivx, ivy, ivz, t1, &e1)) result = e1 < 0.0f ? 1 : 2;
+    // back in half-voxel steps to a positive value: a loop of its own, so that
+    // the rays of a warp go into the bisection together
+    float t0 = t1 - g.vx2 / 2, e0 = 0.0f;
+    bool found = false;
+    for (int back = 0; result == 1 && t0 > enterT && back < max_back; back++) {
+        if (!sample(grid, g, r, ivx, ivy, ivz, t0, &e0)) break;
+        found = e0 > 0.0f;
+        if (found) break;
+        if (e0 > e1) {
             t1 = t0;
             e1 = e0;
         }
         t0 -= g.vx2 * 0.5f;
     }
-    return 0;
+    if (result == 1 && !found) result = 0;
+    __syncwarp(rays);
+    if (result != 1) return result;
+    float tx = linear_zero(t0, e0, t1, e1);
+    for (; iter > 0; iter--) {
+        float ex;
+        if (!sample(grid, g, r, ivx, ivy, ivz, tx, &ex)) return 0;
+        if (ex < 0.0f) {
+            t1 = tx;
+            e1 = ex;
+        } else {
+            t0 = tx;
+            e0 = ex;
+        }
+        tx = linear_zero(t0, e0, t1, e1);
+    }
+    *t_hit = tx;
+    return 1;
 }
 
-// One axis of the voxel walk: the next plane-crossing time and its step, the
-// voxel corner coordinate and its step, the voxel index and its direction.
-struct Axis {
-    float tn, ts, vp, gs;
-    int c, d;
-    __device__ __forceinline__ void step() {
-        tn += ts;
-        vp += gs;
-        c = max(c + d, 0);
+// Repeated addition T += ts without taking every step.  While T stays in one
+// binade [2^e, 2^(e+1)) each sum is a multiple of the binade's unit u, so every
+// addition rounds ts to the same multiple d of u and k of them give T + k d,
+// one exact multiply-add.  Where ts lies half-way between two multiples the
+// sum is rounded to an even one: from an even T that is again the same d, from
+// an odd T only once (`even` is then false and one addition is taken).
+struct Binade {
+    float d, top;
+    bool even;
+    __device__ __forceinline__ Binade(float T, float ts) {
+        const unsigned b = __float_as_uint(T), e = b & 0x7f800000u;
+        top = __uint_as_float(e + 0x00800000u);
+        d = (T + ts) - T;
+        const float half = __uint_as_float(e - (24u << 23));
+        // T in [2^-101, 2^126], positive
+        even = b - (26u << 23) < 0x7e000000u - (26u << 23) && d > 0.0f && !((b & 1u) && fabsf(ts - d) == half);
     }
-    // events of this axis before the one that leaves the current S-block
-    // (S = 8 or 32, the block also ending at R); -1 when no event leaves it
-    // (the index saturates at 0 in block 0)
+    // T after k additions; at least top where not all of them stay below it
+    __device__ __forceinline__ float after(float T, int k) const { return __fmaf_rn((float)k, d, T); }
+};
+
+// One axis of the voxel walk: the next plane-crossing time, its step and the
+// step's reciprocal (an estimate); the voxel index, its direction, and the
+// events taken.
+struct Moment {
+    float tn, ts, rts;
+};
+struct Axis : Moment {
+    int c, d, n;
+    __device__ __forceinline__ void step(bool yes) {
+        if (yes) tn += ts;
+        took(yes);
+    }
+    __device__ __forceinline__ void took(int k) {
+        c = max(c + d * k, 0);
+        n += k;
+    }
+    // the events before the one that leaves the S-block (S = 8 or 32, the
+    // block also ending at R); -1 when none leaves it (the index saturates at 0
+    // in block 0)
     __device__ __forceinline__ int to_boundary(int S, int R) const {
         return d > 0 ? min(S - 1 - (c & (S - 1)), R - 1 - c) : (c >= S ? (c & (S - 1)) : -1);
     }
-    // the time of the event after b more events: the same additions as b steps
-    __device__ __forceinline__ float time_after(int b) const {
-        float T = tn;
-        for (int i = 0; i < b; i++) T += ts;
-        return T;
+};
+
+// the time of the event after `left` more events
+__device__ __forceinline__ float time_after(Moment A, int left) {
+    while (left > 0) {
+        const Binade B(A.tn, A.ts);
+        const int k = min(left, max((int)((B.top - A.tn) * A.rts), 0));
+        const float t = B.after(A.tn, k);
+        if (B.even && t < B.top) {
+            A.tn = t;
+            left -= k;
+        }
+        if (left > 0) {
+            A.tn += A.ts;
+            left--;
+        }
+    }
+    return A.tn;
+}
+
+// takes the events before time Te (those at Te too with `at`); how many, or
+// more than `most` where there are more than that
+__device__ __forceinline__ int pass(Moment &A, float Te, bool at, int most) {
+    int n = 0;
+    while ((A.tn < Te || (at && A.tn == Te)) && n <= most) {
+        const Binade B(A.tn, A.ts);
+        int k = min(max((int)((fminf(Te, B.top) - A.tn) * A.rts), 0), most);
+        float t = B.after(A.tn, k);
+        if (!(t < Te)) t = B.after(A.tn, --k);
+        if (B.even && t < B.top && t < Te && k > 0) {
+            A.tn = t;
+            n += k;
+        }
+        A.tn += A.ts;
+        n++;
+    }
+    return n;
+}
+
+// A voxel corner's coordinate after n steps, carried along when the fine
+// search asks for it.  exact: every such sum is exact (walk_is_exact), so the
+// steps are one multiply-add.
+struct Corner {
+    float vp, gs;
+    int n;
+    __device__ __forceinline__ float at(int k, bool exact) {
+        if (exact)
+            vp = __fmaf_rn((float)(k - n), gs, vp);
+        else
+            for (int i = n; i < k; i++) vp += gs;
+        n = k;
+        return vp;
     }
 };
 
@@ -307,49 +390,60 @@ struct Axis {
 // crossings at tn, tn + ts, ...; each value depends only on how many steps its
 // own axis took): at every step it takes the axis with the smallest tn, ties
 // going to z, then y, then x.  So the order of all events is the order of
-// (time, z < y < x).  A block of voxels (a 32^3 super brick or an 8^3 brick)
-// that holds no negative value is crossed axis by axis: the event that leaves
-// the block is the smallest (time, axis) among the three axes' boundary
-// events, and each axis takes exactly its events ordered before that one --
-// the same float additions in the same order as the reference's walk, and no
-// grid reads.  The boundary times are first estimated with one rounding; only
-// the axes whose estimate may be the smallest are summed exactly.  Other
-// voxels (blocks that may hold a negative value, voxels outside [0, R)^3) are
-// visited one by one, as the reference does.
-__device__ bool traverse(const float2 *__restrict__ grid, const uint8_t *__restrict__ flags, const Geom &g,
+// (time, z < y < x).  Where the walk is after an event therefore depends on
+// that event alone, not on how it got there, and while the voxels that it
+// passes hold no negative value nothing else of it matters.  So empty blocks
+// (32^3 super bricks and 8^3 bricks without a negative value) are crossed in
+// two parts: block after block by times estimated with one rounding, for as
+// long as the estimates' error bound leaves no doubt about the block that the
+// walk is in, and then to the event that enters the block where that ends,
+// exactly: its time, the other axes' events before it, and their times are
+// those of the reference's additions (time_after, pass).  Where two boundaries
+// are too close to call, the first of them is found by its exact time.  Voxels
+// that may hold a negative value, and those outside [0, R)^3, are visited one
+// by one, as the reference does.
+//
+// What bounds it is instruction issue (58% of the slots; DRAM 2%), so the rays
+// of a warp are kept on the same part of the walk: all cross empty blocks, then
+// all walk, and the fine search waits until none can walk on.  640x480 rays on
+// a 256^3 grid of a room: 95.6 million warp instructions with every block
+// crossed axis by axis in loops of additions, 57.4 million so; 193 -> 148 us
+// alone, and six frames of three streams 950 -> 779 us.
+__device__ bool traverse(bool in_grid, const float2 *__restrict__ grid, const uint8_t *__restrict__ flags, const Geom &g,
                          const Ray &r, float idx, float idy, float idz, int s0, int s1, int s2, float enterT,
                          float exitT, int iter, float *t_hit) {
     const float vdx = g.vx2, vdy = g.vy2, vdz = g.vz2;
     enterT += vdx * 2;
     exitT -= vdx * 2;
     if (enterT < 0) enterT = 0;
-    if (enterT + vdx * 2 > exitT) return false;
+    if (enterT + vdx * 2 > exitT) in_grid = false;
     const float ivx = g.ivx, ivy = g.ivy, ivz = g.ivz;
     const unsigned vx = f2u((r.ox + enterT * r.dx - g.ib0x) * ivx);
     const unsigned vy = f2u((r.oy + enterT * r.dy - g.ib0y) * ivy);
     const unsigned vz = f2u((r.oz + enterT * r.dz - g.ib0z) * ivz);
     // the start point lies in the grid box, so its voxel is in [0, R]^3
-    if (vx > (unsigned)g.R + 1 || vy > (unsigned)g.R + 1 || vz > (unsigned)g.R + 1) return false;
-    Axis X, Y, Z;
-    X.vp = g.ib0x + (float)vx * vdx;
-    Y.vp = g.ib0y + (float)vy * vdy;
-    Z.vp = g.ib0z + (float)vz * vdz;
+    if (vx > (unsigned)g.R + 1 || vy > (unsigned)g.R + 1 || vz > (unsigned)g.R + 1) in_grid = false;
     const float sgx = (float)(1 - 2 * s0), sgy = (float)(1 - 2 * s1), sgz = (float)(1 - 2 * s2);
-    X.gs = sgx * vdx;
-    Y.gs = sgy * vdy;
-    Z.gs = sgz * vdz;
-    X.tn = (X.vp + X.gs - r.ox) * idx;
-    Y.tn = (Y.vp + Y.gs - r.oy) * idy;
-    Z.tn = (Z.vp + Z.gs - r.oz) * idz;
-    X.ts = X.gs * idx;
-    Y.ts = Y.gs * idy;
-    Z.ts = Z.gs * idz;
+    Corner px = {g.ib0x + (float)vx * vdx, sgx * vdx, 0};
+    Corner py = {g.ib0y + (float)vy * vdy, sgy * vdy, 0};
+    Corner pz = {g.ib0z + (float)vz * vdz, sgz * vdz, 0};
+    Axis X, Y, Z;
+    X.tn = (px.vp + px.gs - r.ox) * idx;
+    Y.tn = (py.vp + py.gs - r.oy) * idy;
+    Z.tn = (pz.vp + pz.gs - r.oz) * idz;
+    X.ts = px.gs * idx;
+    Y.ts = py.gs * idy;
+    Z.ts = pz.gs * idz;
+    X.rts = rt::rcp_approx(X.ts);
+    Y.rts = rt::rcp_approx(Y.ts);
+    Z.rts = rt::rcp_approx(Z.ts);
     X.d = 1 - 2 * s0;
     Y.d = 1 - 2 * s1;
     Z.d = 1 - 2 * s2;
     X.c = (int)vx;
     Y.c = (int)vy;
     Z.c = (int)vz;
+    X.n = Y.n = Z.n = 0;
     const size_t R = (size_t)g.R, RR = R * R, nvox = RR * R;
     const float *gx = reinterpret_cast<const float *>(grid);
     // a ray crosses at most R + 2 voxel planes per axis inside the grid and
@@ -357,147 +451,174 @@ __device__ bool traverse(const float2 *__restrict__ grid, const uint8_t *__restr
     // loops only where float steps stall (a grid far from the origin with tiny
     // voxels), where the reference's loops would not end
     const int max_steps = 3 * g.R + 16, max_back = 4 * g.R + 16;
-    const float inf = __int_as_float(0x7f800000);
-    int steps = 0;
-    int lvl = empty_level(flags, g, X.c, Y.c, Z.c);
-    float t = enterT;
-    while (t < exitT) {
-        if (lvl > 0) {
-            const int S = lvl == 2 ? 32 : 8;
-            const int bx = X.to_boundary(S, g.R), by = Y.to_boundary(S, g.R), bz = Z.to_boundary(S, g.R);
-            if (bx >= 0 || by >= 0 || bz >= 0) {
-                // estimates E (one rounding) and bounds on their distance from
-                // the exact sums: b + 1 roundings of at most 2^-24 of the
-                // partial sums, taken four times over.  A NaN estimate (0 x inf)
-                // fails every comparison and is summed exactly.
-                const float Ex = bx >= 0 ? __fmaf_rn((float)bx, X.ts, X.tn) : inf;
-                const float Ey = by >= 0 ? __fmaf_rn((float)by, Y.ts, Y.tn) : inf;
-                const float Ez = bz >= 0 ? __fmaf_rn((float)bz, Z.ts, Z.tn) : inf;
-                const float ex = (float)(bx + 2) * 2.384185791e-7f * (fabsf(X.tn) + fabsf(Ex)) + 1e-30f;
-                const float ey = (float)(by + 2) * 2.384185791e-7f * (fabsf(Y.tn) + fabsf(Ey)) + 1e-30f;
-                const float ez = (float)(bz + 2) * 2.384185791e-7f * (fabsf(Z.tn) + fabsf(Ez)) + 1e-30f;
-                float thr = inf;
-                if (bx >= 0) thr = fminf(thr, Ex + ex);
-                if (by >= 0) thr = fminf(thr, Ey + ey);
-                if (bz >= 0) thr = fminf(thr, Ez + ez);
-                // exact boundary times of the candidates; the first in (time, z < y < x) order
-                int ea = -1;
-                float Te = 0.0f;
-                if (bz >= 0 && !(Ez - ez > thr)) {
-                    ea = 2;
-                    Te = Z.time_after(bz);
-                }
-                if (by >= 0 && !(Ey - ey > thr)) {
-                    const float Ty = Y.time_after(by);
-                    if (ea < 0 || Ty < Te) {
-                        ea = 1;
-                        Te = Ty;
-                    }
-                }
-                if (bx >= 0 && !(Ex - ex > thr)) {
-                    const float Tx = X.time_after(bx);
-                    if (ea < 0 || Tx < Te) {
-                        ea = 0;
-                        Te = Tx;
-                    }
-                }
-                // the walk ends inside this block: nothing can be hit there
-                if (!(Te < exitT)) return false;
-                int nx = 0, ny = 0, nz = 0;
-                if (ea == 0) {
-                    nx = bx + 1;
-                    for (int i = 0; i < nx; i++) {
-                        X.tn += X.ts;
-                        X.vp += X.gs;
-                    }
-                } else {
-                    while (X.tn < Te && nx <= max_steps) {
-                        X.tn += X.ts;
-                        X.vp += X.gs;
-                        nx++;
-                    }
-                }
-                if (ea == 1) {
-                    ny = by + 1;
-                    for (int i = 0; i < ny; i++) {
-                        Y.tn += Y.ts;
-                        Y.vp += Y.gs;
-                    }
-                } else {
-                    // y before x at equal times
-                    while ((Y.tn < Te || (Y.tn == Te && ea == 0)) && ny <= max_steps) {
-                        Y.tn += Y.ts;
-                        Y.vp += Y.gs;
-                        ny++;
-                    }
-                }
-                if (ea == 2) {
-                    nz = bz + 1;
-                    for (int i = 0; i < nz; i++) {
-                        Z.tn += Z.ts;
-                        Z.vp += Z.gs;
-                    }
-                } else {
-                    // z before x and y at equal times
-                    while (Z.tn <= Te && nz <= max_steps) {
-                        Z.tn += Z.ts;
-                        Z.vp += Z.gs;
-                        nz++;
-                    }
-                }
-                X.c = max(X.c + X.d * nx, 0);
-                Y.c = max(Y.c + Y.d * ny, 0);
-                Z.c = max(Z.c + Z.d * nz, 0);
-                steps += nx + ny + nz;
-                if (steps > max_steps) return false;
-                t = Te;
-                lvl = empty_level(flags, g, X.c, Y.c, Z.c);
-                continue;
-            }
-        }
-        if (++steps > max_steps) return false;
-        if (lvl == 0) {
-            const size_t off = (size_t)X.c + (size_t)Y.c * R + (size_t)Z.c * RR;
-            if (off >= nvox) return false;
-            if (__ldg(gx + 2 * off) < 0.0f) {
-                const int rr =
-                    refine(grid, g, r, ivx, ivy, ivz, X.vp, Y.vp, Z.vp, enterT, exitT, iter, max_back, t_hit);
-                if (rr != 2) return rr == 1;
-            }
-        }
-        // one event of the reference's walk (x when tnx < tny and tnx < tnz,
-        // y when tny <= tnx and tny < tnz, else z)
-        const int ox = X.c, oy = Y.c, oz = Z.c;
-        if (X.tn < Y.tn) {
-            if (X.tn < Z.tn) {
-                t = X.tn;
-                X.step();
-            } else {
-                t = Z.tn;
-                Z.step();
-            }
-        } else {
-            if (Y.tn < Z.tn) {
-                t = Y.tn;
-                Y.step();
-            } else {
-                t = Z.tn;
-                Z.step();
-            }
-        }
-        if (((ox ^ X.c) | (oy ^ Y.c) | (oz ^ Z.c)) >> 3) lvl = empty_level(flags, g, X.c, Y.c, Z.c);
+    int at_x = 0, at_y = 0, at_z = 0;
+    // voxels counted along the walk: w = c ^ m ascends on every axis, and 8 and
+    // 32 blocks stay blocks; the last one that the walk may leave on each axis
+    const int mx = s0 ? g.mirror : 0, my = s1 ? g.mirror : 0, mz = s2 ? g.mirror : 0;
+    // a bound on the distance of an estimated event time from its sum: R + 3
+    // roundings of at most 2^-24 of the largest, taken twice over.  It needs
+    // times of the ray's own size; a ray along a grid axis has others.
+    float err = (float)(g.R + 4) * 1.1920929e-7f * exitT;
+    const float voxel_err = (float)g.R * 5e-7f;  // of a position in voxels, by the reciprocal and the roundings
+    {
+        const auto plain = [&](const Axis &A) { return A.tn >= -exitT && A.tn < 1e30f && A.ts > 1e-30f && A.ts < 1e30f; };
+        if (!(plain(X) && plain(Y) && plain(Z))) err = __int_as_float(0x7f800000);
     }
-    return false;
+    int steps = 0;
+    float t = enterT;
+    enum { kWalk, kFine, kMiss, kHit };
+    int state = in_grid && t < exitT ? kWalk : kMiss;
+    int lvl = state == kWalk ? empty_level(flags, g, X.c, Y.c, Z.c) : 0;
+    while (true) {
+        // the fine search waits until no ray of the warp can walk on
+        if (!__any_sync(0xffffffffu, state == kWalk)) {
+            const unsigned rays = __ballot_sync(0xffffffffu, state == kFine);
+            if (!rays) break;
+            if (state == kFine) {
+                const int rr = refine(grid, g, r, ivx, ivy, ivz, px.at(at_x, g.exact_walk), py.at(at_y, g.exact_walk),
+                                      pz.at(at_z, g.exact_walk), enterT, exitT, iter, max_back, rays, t_hit);
+                state = rr == 1 ? kHit : (rr == 2 && t < exitT ? kWalk : kMiss);
+            }
+            continue;
+        }
+        // blocks without a negative value, by estimated times
+        bool fast = state == kWalk && lvl > 0;
+        bool stuck = false;
+        int ea = -1, left = 0;
+        float Te = 0.0f;
+        if (fast) {
+            const int cx = X.c ^ mx, cy = Y.c ^ my, cz = Z.c ^ mz;
+            const int lim_x = (g.R - 1) | mx, lim_y = (g.R - 1) | my, lim_z = (g.R - 1) | mz;
+            int wx = cx, wy = cy, wz = cz;
+            int S = lvl == 2 ? 32 : 8;
+            while (true) {
+                // the last voxel of the block on each axis, and the time of the event that leaves it
+                const int ux = min(wx | (S - 1), lim_x), uy = min(wy | (S - 1), lim_y), uz = min(wz | (S - 1), lim_z);
+                const float Ex = __fmaf_rn((float)(ux - cx), X.ts, X.tn), Ey = __fmaf_rn((float)(uy - cy), Y.ts, Y.tn),
+                            Ez = __fmaf_rn((float)(uz - cz), Z.ts, Z.tn);
+                const float E = fminf(fminf(Ex, Ey), Ez);
+                const float second = fmaxf(fminf(Ex, Ey), fminf(fmaxf(Ex, Ey), Ez));
+                if (E > exitT + err) {
+                    state = kMiss;
+                    break;
+                }
+                const bool isx = E == Ex, isy = E == Ey;
+                const int u = isx ? ux : (isy ? uy : uz), base = isx ? cx : (isy ? cy : cz);
+                if (!(E + 2.0f * err < fminf(second, exitT)) || u == (isx ? lim_x : (isy ? lim_y : lim_z))) break;
+                ea = isx ? 0 : (isy ? 1 : 2);
+                left = u - base;
+                // the other axes' voxels at that time, if all estimates within
+                // the error agree on the brick
+                const float qx = fmaxf(__fmaf_rn(E - X.tn, X.rts, (float)(cx + 1)), (float)cx),
+                            qy = fmaxf(__fmaf_rn(E - Y.tn, Y.rts, (float)(cy + 1)), (float)cy),
+                            qz = fmaxf(__fmaf_rn(E - Z.tn, Z.rts, (float)(cz + 1)), (float)cz);
+                const float dx = __fmaf_rn(err, X.rts, voxel_err), dy = __fmaf_rn(err, Y.rts, voxel_err),
+                            dz = __fmaf_rn(err, Z.rts, voxel_err);
+                wx = isx ? u + 1 : rt::index_of(rt::index_sum(qx + dx));
+                wy = !isx && isy ? u + 1 : rt::index_of(rt::index_sum(qy + dy));
+                wz = !isx && !isy ? u + 1 : rt::index_of(rt::index_sum(qz + dz));
+                int apart = 0;
+                if (!isx) apart |= wx ^ rt::index_of(rt::index_sum(fmaxf(qx - dx, 0.0f)));
+                if (isx || !isy) apart |= wy ^ rt::index_of(rt::index_sum(fmaxf(qy - dy, 0.0f)));
+                if (isx || isy) apart |= wz ^ rt::index_of(rt::index_sum(fmaxf(qz - dz, 0.0f)));
+                if (apart >> 3) break;
+                if (max(wx - lim_x, max(wy - lim_y, wz - lim_z)) > 0) break;
+                const int vx_ = wx ^ mx, vy_ = wy ^ my, vz_ = wz ^ mz;
+                const int ib = ((vz_ >> 3) * g.B + (vy_ >> 3)) * g.B + (vx_ >> 3);
+                const int is = ((vz_ >> 5) * g.SB + (vy_ >> 5)) * g.SB + (vx_ >> 5);
+                const uint8_t sup = __ldg(flags + g.nb + is), brick = __ldg(flags + ib);
+                S = sup == 0 ? 32 : 8;
+                if (sup != 0 && brick != 0) break;
+            }
+        }
+        __syncwarp();
+        fast = fast && state == kWalk;
+        if (fast) {
+            // the event that leaves the last of them, or the first in (time,
+            // z < y < x) order of those that may leave the first
+            if (ea < 0) {
+                const int S = lvl == 2 ? 32 : 8;
+                const int bx = X.to_boundary(S, g.R), by = Y.to_boundary(S, g.R), bz = Z.to_boundary(S, g.R);
+                const float inf = __int_as_float(0x7f800000);
+                const float Tx = bx < 0 ? inf : time_after(X, bx), Ty = by < 0 ? inf : time_after(Y, by),
+                            Tz = bz < 0 ? inf : time_after(Z, bz);
+                Te = Tz, ea = 2, left = bz;
+                if (Ty < Te) Te = Ty, ea = 1, left = by;
+                if (Tx < Te) Te = Tx, ea = 0, left = bx;
+                stuck = bx < 0 && by < 0 && bz < 0;
+                fast = !stuck && Te < exitT;
+                // the walk ends inside this block: nothing can be hit there
+                if (!stuck && !fast) state = kMiss;
+            } else {
+                Te = time_after(ea == 0 ? X : (ea == 1 ? Y : Z), left);
+            }
+        }
+        __syncwarp();
+        if (fast) {
+            // that axis takes this event as well, the other two, first in (x,
+            // y, z), their events before it: y before x and z before both at
+            // equal times
+            Moment A = ea == 0 ? Y : X, B = ea == 2 ? Y : Z;
+            const int na = pass(A, Te, ea == 0, max_steps), nb = pass(B, Te, ea != 2, max_steps);
+            const int nx = ea == 0 ? left + 1 : na, ny = ea == 1 ? left + 1 : (ea == 0 ? na : nb),
+                      nz = ea == 2 ? left + 1 : nb;
+            X.tn = ea == 0 ? Te + X.ts : A.tn;
+            Y.tn = ea == 1 ? Te + Y.ts : (ea == 0 ? A.tn : B.tn);
+            Z.tn = ea == 2 ? Te + Z.ts : B.tn;
+            X.took(nx);
+            Y.took(ny);
+            Z.took(nz);
+            steps += nx + ny + nz;
+            if (steps > max_steps) state = kMiss;
+            t = Te;
+            lvl = empty_level(flags, g, X.c, Y.c, Z.c);
+        }
+        // voxel by voxel
+        __syncwarp();
+        bool more = state == kWalk && (lvl == 0 || stuck);
+        while (more) {
+            if (++steps > max_steps) {
+                state = kMiss;
+                break;
+            }
+            float value = 1.0f;
+            if (lvl == 0) {
+                const size_t off = (size_t)X.c + (size_t)Y.c * R + (size_t)Z.c * RR;
+                if (off >= nvox) {
+                    state = kMiss;
+                    break;
+                }
+                value = __ldg(gx + 2 * off);
+            }
+            at_x = X.n; at_y = Y.n; at_z = Z.n;
+            // one event of the reference's walk (x when tnx < tny and tnx < tnz,
+            // y when tny <= tnx and tny < tnz, else z)
+            const int ox = X.c, oy = Y.c, oz = Z.c;
+            const bool ex = X.tn < Y.tn && X.tn < Z.tn, ey = !(X.tn < Y.tn) && Y.tn < Z.tn;
+            t = ex ? X.tn : (ey ? Y.tn : Z.tn);
+            X.step(ex);
+            Y.step(ey);
+            Z.step(!ex && !ey);
+            if (((ox ^ X.c) | (oy ^ Y.c) | (oz ^ Z.c)) >> 3) lvl = empty_level(flags, g, X.c, Y.c, Z.c);
+            if (value < 0.0f) {
+                state = kFine;
+                break;
+            }
+            if (!(t < exitT)) state = kMiss;
+            more = state == kWalk && lvl == 0;
+        }
+    }
+    return state == kHit;
 }
 
 // rayCastVoxelsKernel (VoxelGrid_cuda.cu:734-770) with initRay (118-141) and
 // intersectVoxelGridCuda (144-163); g.T = camera -> world
-__global__ void __launch_bounds__(kRayTileX * kRayTileY, 32)
+__global__ void __launch_bounds__(kRayTileX * kRayTileY, kRayCtas)
     k_raycast(const float2 *__restrict__ grid, const uint8_t *__restrict__ flags, Geom g, int iter,
               float4 *__restrict__ xyz) {
     const int xi = blockIdx.x * kRayTileX + (threadIdx.x % kRayTileX);
     const int yi = blockIdx.y * kRayTileY + (threadIdx.x / kRayTileX);
-    if (xi >= g.W || yi >= g.H) return;
+    const bool inside = xi < g.W && yi < g.H;
     const float pdx = (float)xi / g.Wf, pdy = (float)yi / g.Hf;
     float cx = -(pdx - g.K2) / g.K0, cy = -(pdy - g.K5) / g.K4, cz = -1;
     float len = 0.0f;
@@ -526,9 +647,10 @@ __global__ void __launch_bounds__(kRayTileX * kRayTileY, 32)
     const float tmax = fminf(x1, fminf(y1, z1));
     float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float th;
-    if (!(tmin >= tmax || tmax <= 0) && traverse(grid, flags, g, r, idx, idy, idz, s0, s1, s2, tmin, tmax, iter, &th))
+    if (traverse(inside && !(tmin >= tmax || tmax <= 0), grid, flags, g, r, idx, idy, idz, s0, s1, s2, tmin, tmax, iter,
+                 &th))
         out = make_float4(th * cx, th * cy, th * cz, (th > g.min_dist && th < g.max_dist) ? 1.0f : 0.0f);
-    xyz[(size_t)yi * g.W + xi] = out;
+    if (inside) xyz[(size_t)yi * g.W + xi] = out;
 }
 
 // shadingKernel (VoxelGrid_cuda.cu:844-891) with filter3 (772-789)
@@ -690,6 +812,21 @@ void invert_rt4(const float *M, float *Mi) {
 // the launch constants of SimParams (VoxelGrid.cpp:48-106; kernel prologues
 // VoxelGrid_cuda.cu:745-756, 957-965): T3x4 is the first three rows of the
 // pose the kernel uses
+// whether start + n * step is exact in float for every start on the axis' grid
+// (b0 + v * step) and every n that a walk of max_steps can take: b0 and step
+// are multiples of a power of two u, and the sums stay below 2^24 u
+bool walk_is_exact(float b0, float step, int R) {
+    if (!(std::fabs(b0) < 1e30f) || !(step > 1e-30f && step < 1e30f)) return false;
+    const auto unit = [](float v) {  // the exponent of the lowest bit set
+        int e;
+        int m = (int)std::ldexp(std::frexp(v, &e), 24);
+        for (e -= 24; !(m & 1); m >>= 1) e++;
+        return e;
+    };
+    const int u = b0 == 0.0f ? unit(step) : std::min(unit(std::fabs(b0)), unit(step));
+    return std::ldexp(std::fabs((double)b0) + (double)step * (4 * R + 32), -u) < 16777216.0;
+}
+
 Geom make_geom(const recon_tsdf_params &p, const float *T3x4, const float *K) {
     Geom g;
     memset(&g, 0, sizeof(g));
@@ -736,6 +873,9 @@ Geom make_geom(const recon_tsdf_params &p, const float *T3x4, const float *K) {
     g.ivz = 1.0f / g.vz2;
     g.min_dist = p.min_dist;
     g.max_dist = p.max_dist;
+    for (g.mirror = 31; g.mirror < R - 1;) g.mirror = 2 * g.mirror + 1;
+    g.exact_walk =
+        walk_is_exact(g.ib0x, g.vx2, R) && walk_is_exact(g.ib0y, g.vy2, R) && walk_is_exact(g.ib0z, g.vz2, R);
     return g;
 }
 
