@@ -9,13 +9,15 @@
 // float -> unsigned conversions saturate as the reference's make_uint3 and
 // `uint += float` do on the GPU.  What differs is how the work is mapped:
 //
-//  * update: one CTA per 32x8x8 block of voxels, each thread a run of 8 voxels
+//  * update: a CTA takes a 32x8x8 block of voxels, each thread a run of 8 voxels
 //    along z at one (x, y), so that a warp reads and writes 32 consecutive
 //    float2 (256 bytes).  A block whose voxel centres all project outside the
 //    image (tested at its 8 corners, with a margin for rounding) is skipped
 //    as a whole: the projection is a linear-fractional map, so over a box on
-//    one side of the camera plane its extremes lie at the corners.  A voxel is
-//    written only when its value changes.
+//    one side of the camera plane its extremes lie at the corners.  On large
+//    grids a block that lies behind all distances its pixels show is skipped
+//    too, and the blocks to visit are listed first.  A voxel is written only
+//    when its value changes.
 //  * ray cast: one thread per pixel, one warp per 8x4 tile.  A byte per 8x8x8 brick
 //    records whether any voxel of the brick may be negative; the traversal
 //    steps through bricks without one using only its step arithmetic (the
@@ -51,6 +53,15 @@ constexpr int kBrick = 8;    // voxels per side of a flag brick
 constexpr int kTileX = 32;   // update CTA: 32 x 8 columns of 8 voxels along z
 constexpr int kTileY = 8;
 constexpr int kRunZ = 8;
+constexpr int kFarTile = 16;    // distance map tiles of the update's test for blocks behind the surface
+constexpr int kFarMost = 256;   // tiles that a block may look at
+constexpr int kListCtas = 8;    // CTAs per SM of the update by list
+// From this many blocks on the update picks the blocks to visit first: two small
+// launches, which cost more than they save on a coarse grid.  640x480 frames, all
+// blocks / picked ones, four frames with their ray casts: 64^3 203 / 222 us,
+// 160^3 (2000 blocks) 340 / 361; six frames on 256^3 (8192) 785 / 758; two on
+// 512^3 (65536) 1014 / 812.
+constexpr int kListBlocks = 6144;
 constexpr int kRayTileX = 8;  // ray cast CTA: one warp on 8 x 4 pixels (rays differ widely in length;
 constexpr int kRayTileY = 4;  // one-warp CTAs let the block scheduler balance the SMs)
 constexpr int kRayCtas = 28;  // ray cast CTAs per SM: 72 registers.  32 (64 registers) spill more and 24 leave fewer
@@ -59,6 +70,7 @@ constexpr int kKinds = 5;     // timing kinds: update, ray cast, shading, distan
 
 struct Geom {
     int R, B, SB, W, H;             // voxels, 8^3 bricks and 32^3 super bricks per side, image size
+    int tiles_x, tiles_y;           // 16 x 16 tiles of the distance map
     int nb;                         // B^3: offset of the super-brick bytes
     float T[12];                    // update: world -> camera; ray cast / resample: camera -> world
     float K0, K2, K4, K5, Wf, Hf, Wm2, Hm2;
@@ -89,49 +101,104 @@ __device__ __forceinline__ void mark_negative(uint8_t *flags, const Geom &g, uns
 
 // ---------------------------------------------------------------- update --
 
-// updateVoxelsKernel (VoxelGrid_cuda.cu:944-1014).  counts (kCount): voxels
-// [projected into the image, fused, changed].
-template <bool kCount>
-__global__ void __launch_bounds__(kTileX * kTileY)
-    k_update(float2 *__restrict__ grid, uint8_t *__restrict__ flags, const float *__restrict__ dist, Geom g,
-             unsigned long long *__restrict__ counts) {
-    __shared__ int s_skip;
-    const int lane = threadIdx.x & 31;
-    const int x0 = blockIdx.x * kTileX, y0 = blockIdx.y * kTileY, z0 = blockIdx.z * kRunZ;
-    if (threadIdx.x < 32) {
-        // the block's corner voxel centres (lanes 8..31 repeat lanes 0..7)
-        const int c = lane & 7;
-        const int cx = min(x0 + ((c & 1) ? kTileX - 1 : 0), g.R - 1);
-        const int cy = y0 + ((c & 2) ? kTileY - 1 : 0), cz = z0 + ((c & 4) ? kRunZ - 1 : 0);
+// The largest distance in each 16 x 16 tile of the distance map (infinity where
+// the tile holds a NaN): one warp per tile.
+__global__ void __launch_bounds__(128) k_far_tiles(const float *__restrict__ dist, Geom g, float *__restrict__ far_tiles,
+                                                   int *__restrict__ count) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *count = 0;
+    const int tile = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (tile >= g.tiles_x * g.tiles_y) return;
+    const int x = (tile % g.tiles_x) * kFarTile + (lane & 15), y0 = (tile / g.tiles_x) * kFarTile + (lane >> 4);
+    float far = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kFarTile; k += 2) {
+        const float d = x < g.W && y0 + k < g.H ? __ldg(dist + (size_t)(y0 + k) * g.W + x) : 0.0f;
+        far = d == d ? fmaxf(far, d) : __int_as_float(0x7f800000);
+    }
+    for (int o = 16; o; o >>= 1) far = fmaxf(far, __shfl_xor_sync(0xffffffffu, far, o));
+    if (lane == 0) far_tiles[tile] = far;
+}
+
+// The 32 x 8 x 8 block of voxels at (x0, y0, z0), by its corner voxel centres:
+// one per lane of a group of 8 lanes (all 32 lanes take part).
+struct Block {
+    float lo_x, hi_x, lo_y, hi_y;  // pixels
+    float near;                    // the least depth, less what the roundings may add
+    bool outside;                  // no voxel projects into the image
+    bool sharp;                    // in front of the camera, projected to better than a pixel
+    __device__ __forceinline__ Block(const Geom &g, int x0, int y0, int z0) {
+        const int lane = threadIdx.x & 31, group = lane & 24;
+        const int cx = min(x0 + ((lane & 1) ? kTileX - 1 : 0), g.R - 1);
+        const int cy = y0 + ((lane & 2) ? kTileY - 1 : 0), cz = z0 + ((lane & 4) ? kRunZ - 1 : 0);
         const float px = g.sx + (float)cx * g.vx2, py = g.sy + (float)cy * g.vy2, pz = g.sz + (float)cz * g.vz2;
         const float rx = g.T[0] * px + g.T[1] * py + g.T[2] * pz + g.T[3];
         const float ry = g.T[4] * px + g.T[5] * py + g.T[6] * pz + g.T[7];
         const float rz = g.T[8] * px + g.T[9] * py + g.T[10] * pz + g.T[11];
-        float ux = (rx / rz * g.K0 + g.K2) * g.Wf, uy = (ry / rz * g.K4 + g.K5) * g.Hf;
-        float lo_x = ux, hi_x = ux, lo_y = uy, hi_y = uy;
+        lo_x = hi_x = (rx / rz * g.K0 + g.K2) * g.Wf;
+        lo_y = hi_y = (ry / rz * g.K4 + g.K5) * g.Hf;
+        const float off = 1e-6f * (fabsf(g.T[8] * px) + fabsf(g.T[9] * py) + fabsf(g.T[10] * pz) + fabsf(g.T[11]));
+        near = -rz - off;
+        const bool pixel = off * fmaxf(fabsf(g.K0) * g.Wf, fabsf(g.K4) * g.Hf) < near;
         for (int o = 1; o < 8; o <<= 1) {
             lo_x = fminf(lo_x, __shfl_xor_sync(0xffffffffu, lo_x, o));
             hi_x = fmaxf(hi_x, __shfl_xor_sync(0xffffffffu, hi_x, o));
             lo_y = fminf(lo_y, __shfl_xor_sync(0xffffffffu, lo_y, o));
             hi_y = fmaxf(hi_y, __shfl_xor_sync(0xffffffffu, hi_y, o));
+            near = fminf(near, __shfl_xor_sync(0xffffffffu, near, o));
         }
         // |rz| >= 16 mm at every corner keeps the rounding of the projected
         // coordinates far below the 4-pixel margin
-        const unsigned front = __ballot_sync(0xffffffffu, rz < -16.0f) & 0xffu;
-        const unsigned behind = __ballot_sync(0xffffffffu, rz > 16.0f) & 0xffu;
-        const bool one_side = (front == 0xffu) || (behind == 0xffu);
-        const bool outside = !(hi_x >= -3.0f) || !(lo_x < g.Wf + 2.0f) || !(hi_y >= -3.0f) || !(lo_y < g.Hf + 2.0f);
-        if (lane == 0) s_skip = one_side && outside;
+        const unsigned front = __ballot_sync(0xffffffffu, rz < -16.0f) >> group & 0xffu;
+        const unsigned behind = __ballot_sync(0xffffffffu, rz > 16.0f) >> group & 0xffu;
+        sharp = front == 0xffu && (__ballot_sync(0xffffffffu, pixel) >> group & 0xffu) == 0xffu;
+        outside = (front == 0xffu || behind == 0xffu) && (!(hi_x >= -3.0f) || !(lo_x < g.Wf + 2.0f) ||
+                                                          !(hi_y >= -3.0f) || !(lo_y < g.Hf + 2.0f));
     }
-    __syncthreads();
-    if (s_skip) return;
-    const int ix = x0 + lane, iy = y0 + (threadIdx.x >> 5);
-    if (ix >= g.R) return;
+    // Whether the block lies behind all that its pixels show: every distance
+    // that its voxels can see is too short for them to be fused.  A slack of 4
+    // pixels and of 1e-4 covers the roundings of the projection, of the
+    // interpolated distance and of the quotient.
+    __device__ __forceinline__ bool hidden(const Geom &g, const float *__restrict__ far_tiles) const {
+        const int lane = threadIdx.x & 31;
+        const int tx0 = (int)fmaxf(lo_x - 4.0f, 0.0f) / kFarTile, ty0 = (int)fmaxf(lo_y - 4.0f, 0.0f) / kFarTile;
+        const int tx1 = (int)fminf(hi_x + 6.0f, g.Wf - 1.0f) / kFarTile;
+        const int ty1 = (int)fminf(hi_y + 6.0f, g.Hf - 1.0f) / kFarTile;
+        const int nx = tx1 - tx0 + 1, n = nx * (ty1 - ty0 + 1);
+        const bool look = sharp && !outside && n <= kFarMost;
+        float far = 0.0f;
+        if (look)
+            for (int i = lane & 7; i < n; i += 8) far = fmaxf(far, __ldg(far_tiles + (ty0 + i / nx) * g.tiles_x + tx0 + i % nx));
+        for (int o = 1; o < 8; o <<= 1) far = fmaxf(far, __shfl_xor_sync(0xffffffffu, far, o));
+        return look && (far < g.lim || near - far > 1.25f * g.slope + 1e-4f * (near + g.slope));
+    }
+};
+
+// The blocks that the update has to visit: 8 lanes per block.  count was set
+// to 0 by k_far_tiles.  Their order in the list is of no matter: every voxel
+// is in one block.
+__global__ void __launch_bounds__(256)
+    k_pick_blocks(const float *__restrict__ far_tiles, Geom g, int bx, int by, int n, int *__restrict__ list,
+                  int *__restrict__ count) {
+    const int lane = threadIdx.x & 31, i = (blockIdx.x * 256 + threadIdx.x) >> 3, b = min(i, n - 1);
+    const Block block(g, b % bx * kTileX, b / bx % by * kTileY, b / bx / by * kRunZ);
+    const bool hidden = block.hidden(g, far_tiles);  // by all lanes
+    const bool visit = (lane & 7) == 0 && i < n && !hidden && !block.outside;
+    const unsigned all = __ballot_sync(0xffffffffu, visit);
+    int at = 0;
+    if (lane == 0 && all) at = atomicAdd(count, __popc(all));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (visit) list[at + __popc(all & ((1u << lane) - 1))] = b;
+}
+
+// updateVoxelsKernel (VoxelGrid_cuda.cu:944-1014) for the 8 voxels along z from
+// (ix, iy, z0)
+__device__ __forceinline__ void fuse_run(float2 *__restrict__ grid, uint8_t *__restrict__ flags,
+                                         const float *__restrict__ dist, const Geom &g, int ix, int iy, int z0,
+                                         unsigned &n_proj, unsigned &n_fused, unsigned &n_changed) {
     const float px = g.sx + (float)ix * g.vx2;
     const float py = g.sy + (float)iy * g.vy2;
     // T p summed left to right: the first two products do not depend on z
     const float ax = g.T[0] * px + g.T[1] * py, ay = g.T[4] * px + g.T[5] * py, az = g.T[8] * px + g.T[9] * py;
-    unsigned n_proj = 0, n_fused = 0, n_changed = 0;
     const int W = g.W;
 #pragma unroll 2
     for (int k = 0; k < kRunZ; k++) {
@@ -170,6 +237,27 @@ __global__ void __launch_bounds__(kTileX * kTileY)
         }
         if (nx < 0.0f) mark_negative(flags, g, ix, iy, iz);
     }
+}
+
+// All blocks of the grid.  counts (kCount): voxels [projected into the image,
+// fused, changed].
+template <bool kCount>
+__global__ void __launch_bounds__(kTileX * kTileY)
+    k_update(float2 *__restrict__ grid, uint8_t *__restrict__ flags, const float *__restrict__ dist, Geom g,
+             unsigned long long *__restrict__ counts) {
+    __shared__ int s_skip;
+    const int lane = threadIdx.x & 31;
+    const int x0 = blockIdx.x * kTileX, y0 = blockIdx.y * kTileY, z0 = blockIdx.z * kRunZ;
+    if (threadIdx.x < 32) {
+        const Block block(g, x0, y0, z0);
+        if (lane == 0) s_skip = block.outside;
+    }
+    __syncthreads();
+    if (s_skip) return;
+    const int ix = x0 + lane, iy = y0 + (threadIdx.x >> 5);
+    if (ix >= g.R) return;
+    unsigned n_proj = 0, n_fused = 0, n_changed = 0;
+    fuse_run(grid, flags, dist, g, ix, iy, z0, n_proj, n_fused, n_changed);
     if (kCount) {
         n_proj = __reduce_add_sync(0xffffffffu, n_proj);
         n_fused = __reduce_add_sync(0xffffffffu, n_fused);
@@ -179,6 +267,27 @@ __global__ void __launch_bounds__(kTileX * kTileY)
             atomicAdd(&counts[1], (unsigned long long)n_fused);
             atomicAdd(&counts[2], (unsigned long long)n_changed);
         }
+    }
+}
+
+// The blocks of k_pick_blocks' list, so many at a time as fit on the device.
+// What bounds it is the latency of each voxel's chain from the projection over
+// the four distances to the voxel itself, and the bytes of the voxels in front
+// of the surface.  A CTA for each block of a 512^3 grid spent 339 us on a frame,
+// of which 57% of the voxels are outside the image and 18 to 32% hidden behind
+// the surface; more voxels in flight per thread (2, 4 or 8 along z loaded
+// together) were slower (357 to 397 us), exact quotients by one reciprocal no
+// faster.
+__global__ void __launch_bounds__(kTileX * kTileY, kListCtas)
+    k_update_list(float2 *__restrict__ grid, uint8_t *__restrict__ flags, const float *__restrict__ dist, Geom g, int bx,
+                  int by, const int *__restrict__ list, const int *__restrict__ count) {
+    const int n = *count, lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+        const int b = list[i];
+        const int ix = b % bx * kTileX + lane;
+        unsigned n_proj = 0, n_fused = 0, n_changed = 0;
+        if (ix < g.R)
+            fuse_run(grid, flags, dist, g, ix, b / bx % by * kTileY + row, b / bx / by * kRunZ, n_proj, n_fused, n_changed);
     }
 }
 
@@ -752,6 +861,8 @@ struct recon_tsdf {
     float2 *grid = nullptr;
     uint8_t *flags = nullptr;
     float *dist = nullptr;
+    float *far_tiles = nullptr;  // of an update: the largest distance per tile of the map,
+    int *list = nullptr;         // and the blocks to visit, after their number
     float4 *xyz = nullptr, *shaded = nullptr, *normal = nullptr;
     void *staging = nullptr;  // device copy of a host measurement (uint16 or float4 frame)
     size_t staging_bytes = 0;
@@ -796,6 +907,13 @@ size_t n_flag_bytes(const recon_tsdf_params &p) {
     return n_bricks(p) + sb * sb * sb;
 }
 size_t n_pixels(const recon_tsdf_params &p) { return (size_t)p.width * p.height; }
+size_t n_blocks(const recon_tsdf_params &p) {
+    const size_t R = p.grid_resolution;
+    return (R + kTileX - 1) / kTileX * (R / kTileY) * (R / kRunZ);
+}
+size_t n_far_tiles(const recon_tsdf_params &p) {
+    return (size_t)((p.width + kFarTile - 1) / kFarTile) * ((p.height + kFarTile - 1) / kFarTile);
+}
 
 // invertRT4 (basic_math.cpp:355-368): VoxelGrid::setCameraParams's world ->
 // camera pose, in float, translation summed left to right
@@ -835,6 +953,8 @@ Geom make_geom(const recon_tsdf_params &p, const float *T3x4, const float *K) {
     g.B = R / kBrick;
     g.SB = (R + 31) / 32;
     g.nb = g.B * g.B * g.B;
+    g.tiles_x = (p.width + kFarTile - 1) / kFarTile;
+    g.tiles_y = (p.height + kFarTile - 1) / kFarTile;
     g.W = p.width;
     g.H = p.height;
     if (T3x4) memcpy(g.T, T3x4, sizeof(g.T));
@@ -1003,6 +1123,8 @@ int recon_tsdf_create(const recon_tsdf_params *p, void *stream, recon_tsdf **out
     alloc((void **)&v->grid, n_voxels(*p) * sizeof(float2));
     alloc((void **)&v->flags, n_flag_bytes(*p));
     alloc((void **)&v->dist, n_pixels(*p) * sizeof(float));
+    alloc((void **)&v->far_tiles, n_far_tiles(*p) * sizeof(float));
+    alloc((void **)&v->list, (1 + n_blocks(*p)) * sizeof(int));
     alloc((void **)&v->xyz, n_pixels(*p) * sizeof(float4));
     alloc((void **)&v->shaded, n_pixels(*p) * sizeof(float4));
     alloc((void **)&v->normal, n_pixels(*p) * sizeof(float4));
@@ -1034,6 +1156,8 @@ int recon_tsdf_destroy(recon_tsdf *v) {
     cudaFree(v->grid);
     cudaFree(v->flags);
     cudaFree(v->dist);
+    cudaFree(v->far_tiles);
+    cudaFree(v->list);
     cudaFree(v->xyz);
     cudaFree(v->shaded);
     cudaFree(v->normal);
@@ -1097,10 +1221,21 @@ int recon_tsdf_update(recon_tsdf *v, const float T[16], const float K[9]) {
     const int R = v->p.grid_resolution;
     dim3 grd((R + kTileX - 1) / kTileX, R / kTileY, R / kRunZ);
     Timed tm(v, 0);
+    // the counts are of all voxels that project into the image, hidden ones too
     if (v->counting)
         return launch(k_update<true>, grd, dim3(kTileX * kTileY), v->stream, v->grid, v->flags, v->dist, g, v->counts);
-    return launch(k_update<false>, grd, dim3(kTileX * kTileY), v->stream, v->grid, v->flags, v->dist, g,
-                  (unsigned long long *)nullptr);
+    const int n = (int)(grd.x * grd.y * grd.z);
+    if (n < kListBlocks)
+        return launch(k_update<false>, grd, dim3(kTileX * kTileY), v->stream, v->grid, v->flags, v->dist, g,
+                      (unsigned long long *)nullptr);
+    rc = launch(k_far_tiles, dim3((g.tiles_x * g.tiles_y + 3) / 4), dim3(128), v->stream, v->dist, g, v->far_tiles, v->list);
+    if (!rc)
+        rc = launch(k_pick_blocks, dim3((n + 31) / 32), dim3(256), v->stream, v->far_tiles, g, (int)grd.x, (int)grd.y, n,
+                    v->list + 1, v->list);
+    if (!rc)
+        rc = launch(k_update_list, dim3(152 * kListCtas), dim3(kTileX * kTileY), v->stream, v->grid, v->flags, v->dist, g,
+                    (int)grd.x, (int)grd.y, v->list + 1, v->list);
+    return rc;
 }
 
 int recon_tsdf_raycast(recon_tsdf *v, const float T[16], const float K[9], int32_t cubic_filter) {

@@ -56,3 +56,34 @@ def test_ray_cast_matches_voxel_walk(R, dim, fill):
     # a single negative voxel need not be met by a ray; none is met in an empty grid
     assert hits == 0 if fill == 0.0 else (hits > 0 or fill < 1e-3)
     v.close()
+
+
+@pytest.mark.parametrize("R,W,H", [(232, 160, 120), (256, 83, 61)])
+@pytest.mark.parametrize("view", ["room", "inside", "nan"])
+def test_update_of_picked_blocks_matches_oracle(R, W, H, view):
+    """A grid large enough for the update to list its blocks: blocks behind the
+    surface, a camera in the grid, missing, infinite and NaN distances, image
+    edges inside a tile."""
+    import recon_gb300 as rg
+    rng = np.random.default_rng(R + W)
+    dim = 1750.0 if view != "inside" else 600.0
+    origin, size = (0.0, 150.0, -2350.0 if view != "inside" else -300.0), (dim, dim, dim)
+    o = O.OracleTSDF(O.tsdf_params(R, W, H, origin=origin, dim=size))
+    v = rg.TSDF(rg.tsdf_params(R, W, H, cube_origin=origin, cube_dim=size))
+    y, x = np.mgrid[0:H, 0:W]
+    dist = (dim * (1.1 + 0.08 * np.sin(x / 40.0) * np.cos(y / 30.0) + 0.25 * (x > W // 2))).astype(np.float32)
+    dist[rng.random((H, W)) < 0.02] = 0.0
+    if view == "nan":
+        dist[H // 3: H // 3 + 9, W // 4: W // 4 + 9] = np.nan
+        dist[H // 2, W // 2] = np.inf
+    T = np.eye(4, dtype=np.float32)
+    T[:3, 3] = (20.0, -35.0, 10.0)
+    Kn = np.array([0.9, 0, 0.5, 0, -1.2, 0.5, 0, 0, 1], np.float32)
+    for _ in range(2):
+        v.set_dist_map(dist)
+        v.update(T, Kn)
+        o.update(dist, T, Kn)
+        assert np.array_equal(v.get("tsdf").view(np.uint32), o.grid.view(np.uint32))
+    changed = (o.grid.reshape(-1, 2)[:, 1] > 0).mean()
+    assert changed > 0.01  # voxels were fused
+    v.close()
