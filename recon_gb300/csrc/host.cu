@@ -31,7 +31,7 @@ __global__ void k_seg_count(const InstDesc *D, const int *active);
 __global__ void k_seg_scan(const InstDesc *D, const int *active);
 __global__ void k_seg_scatter(const InstDesc *D, const int *active);
 __global__ void k_attr_jac(const InstDesc *D, const int *active);
-__global__ void k_icp_mask(const InstDesc *D, int level);
+__global__ void k_icp_mask(const InstDesc *D, int level, int blocks_per_cta);
 constexpr int kPyrTile = 32;  // level-0 tile of k_prep_current_pyramid
 __global__ void k_prep_current_pyramid(const InstDesc *D, const uint8_t *const *in_gray,
                                        const uint16_t *const *in_depth, const float *const *in_rgbd, int tiles_x,
@@ -576,7 +576,9 @@ int launch_schedule(recon_batch *b, cudaStream_t s, bool in_graph) {
         } else if (any_icp) {
             {
                 TimedScope ts(b, s, TK_ICP_MASK, in_graph);
-                CK(launch_pdl(k_icp_mask, dim3(nchunk, n), dim3(kLanes), s, D, level));
+                // up to 4 blocks per CTA, as far as the device stays filled
+                int per = std::min(4, std::max(1, n * nchunk / kMaskCtaSlots));
+                CK(launch_pdl(k_icp_mask, dim3((nchunk + per - 1) / per, n), dim3(kLanes), s, D, level, per));
             }
             {
                 // about one wave of CTAs over the blocks of the instances that

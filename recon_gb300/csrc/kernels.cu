@@ -842,7 +842,34 @@ __device__ __forceinline__ long long trunc_prod(float r2, float w) {
 
 // The Student-t weight (rgb2gray.cu:537-540; the first pass's sigma^2 is 100,
 // rgb2gray.cu:827-850)
-__device__ __forceinline__ float student_w(float r2, float sigma2) { return 6 / (5 + r2 / sigma2); }
+// by the reciprocal of sigma^2, which all pixels of a pass share, and the exact
+// division of pair_math.cuh.  A squared residual below its range gives 5 + r^2 /
+// sigma^2 = 5 by either division.
+struct StudentW {
+    float sigma2, y;
+    bool plain;
+    __device__ __forceinline__ explicit StudentW(float s2)
+        : sigma2(s2), y(rcp_rn(s2)), plain(s2 >= 0x1p-20f && s2 <= 0x1p60f) {}
+    // whether near() serves squared residuals of this sum (NaN does not)
+    __device__ __forceinline__ bool in_range(float sum_r2) const { return plain && sum_r2 <= 0x1p40f; }
+    __device__ __forceinline__ float near(float r2) const {
+        float d = 5.0f + div_rn(r2, -sigma2, y);
+        return div_rn(6.0f, -d, rcp_rn(d));
+    }
+    __device__ __forceinline__ float far(float r2) const { return ieee_div(6.0f, 5.0f + ieee_div(r2, sigma2)); }
+    __device__ __forceinline__ float operator()(float r2) const { return in_range(r2) ? near(r2) : far(r2); }
+    // the truncated products r^2 w of four pixels, added up; a pixel that is no
+    // correspondence has r^2 = 0 and adds nothing
+    __device__ __forceinline__ long long products(float4 r) const {
+        if (in_range(((r.x + r.y) + r.z) + r.w)) {
+            float a = r.x * near(r.x), b = r.y * near(r.y), c = r.z * near(r.z), e = r.w * near(r.w);
+            if (fmaxf(fmaxf(a, b), fmaxf(c, e)) < 8388608.0f)
+                return trunc_small(a) + trunc_small(b) + trunc_small(c) + trunc_small(e);
+        }
+        return trunc_prod(r.x, (*this)(r.x)) + trunc_prod(r.y, (*this)(r.y)) + trunc_prod(r.z, (*this)(r.z)) +
+               trunc_prod(r.w, (*this)(r.w));
+    }
+};
 
 // What the ICP kernels need of a level for every pixel: the current frame's
 // points there and the projection into it.
@@ -1004,18 +1031,83 @@ __device__ __forceinline__ bool icp_last_block(const InstDesc &d, int nblk) {
     return s_last != 0;
 }
 
+// Blocks [b0, b1) of 1024 pixels, four per thread, kBatch at a time: a batch's
+// taps are in flight together, and meanwhile the next batch's points and normals.
+template <bool kDepth>
+__device__ __forceinline__ void icp_mask_blocks(const InstDesc &d, int level, const float *T, int b0, int b1, int n,
+                                                int &cnt, long long &vsum) {
+    constexpr int kBatch = kDepth ? 2 : 1;
+    const IcpLevel L(d, level);
+    const StudentW first(100.0f);
+    const float *pl = d.ref_pl[level] + (size_t)b0 * 6 * kChunk + threadIdx.x;
+    float next[kBatch][6];
+#pragma unroll
+    for (int u = 0; u < kBatch; u++)
+#pragma unroll
+        for (int k = 0; k < 6; k++) next[u][k] = __ldg(pl + k * kChunk + u * kLanes);
+    for (int b = b0; b < b1; b++, pl += 6 * kChunk) {
+        int i = b * kChunk + threadIdx.x;
+        float r4[4];
+#pragma unroll
+        for (int g = 0; g < 4; g += kBatch) {
+            // (past the last pixel the planes hold a point of depth 0: it is not stored)
+            float p[kBatch][6], q[kBatch][3], px[kBatch], py[kBatch];
+            bool in[kBatch];
+            IcpTaps<kDepth> tap[kBatch];
+#pragma unroll
+            for (int u = 0; u < kBatch; u++) {
+#pragma unroll
+                for (int k = 0; k < 6; k++) p[u][k] = next[u][k];
+                mul4(T, p[u][0], p[u][1], p[u][2], q[u][0], q[u][1], q[u][2]);
+                in[u] = p[u][2] == p[u][2] && i + (g + u) * kLanes < n && icp_project(L, q[u][0], q[u][1], q[u][2], px[u], py[u]);
+                tap[u].load(L, icp_tap_index(L, in[u], px[u], py[u]));
+            }
+            if (g + kBatch < 4 || b + 1 < b1) {
+                const float *nx = g + kBatch < 4 ? pl + (g + kBatch) * kLanes : pl + 6 * kChunk;
+#pragma unroll
+                for (int u = 0; u < kBatch; u++)
+#pragma unroll
+                    for (int k = 0; k < 6; k++) next[u][k] = __ldg(nx + k * kChunk + u * kLanes);
+            }
+#pragma unroll
+            for (int u = 0; u < kBatch; u++) {
+                float nx, ny, nz, cx, cy, cz;
+                bool ok = in[u] && tap[u].all();
+                float r2 = 0.0f;
+                if (ok) {
+                    rot4(T, p[u][3], p[u][4], p[u][5], nx, ny, nz);
+                    icp_blend<kDepth>(L, tap[u], px[u], py[u], cx, cy, cz);
+                    float res = (cx - q[u][0]) * nx + (cy - q[u][1]) * ny + (cz - q[u][2]) * nz;
+                    r2 = res * res;
+                }
+                int at = i + (g + u) * kLanes;
+                if (at < n) {
+                    d.icp_r2[at] = r2;
+                    d.icp_mask[at] = ok;
+                }
+                r4[g + u] = r2;
+                cnt += ok;
+            }
+        }
+        vsum += first.products(make_float4(r4[0], r4[1], r4[2], r4[3]));
+    }
+}
+
 // icpResidualKernel2 (rgb2gray.cu:223-260) with initWeightsKernel's first
 // Student-t weight (rgb2gray.cu:827-850): per pixel of the level, whether it is
 // a correspondence at the level's start pose and its squared residual; per
 // block of 1024 pixels the number of correspondences and the exact int64 sum
 // of the truncated r^2 w0 products (the first variance sum).  The ICP sums of
 // the iterations run over the pixel grid, so no compacted list is built.
-// 6 CTAs per SM (40 registers): more gathers in flight, 63 against 73 us per
-// 30-instance launch at 44 registers
-#ifndef RECON_MASK_MIN_BLOCKS
-#define RECON_MASK_MIN_BLOCKS 6
-#endif
-__global__ void __launch_bounds__(kLanes, RECON_MASK_MIN_BLOCKS) k_icp_mask(const InstDesc *D, int level) {
+// What bounds it is the latency of its two round trips per pixel (33 bytes of
+// DRAM traffic each at level 0: 3.4 TB/s), so a CTA takes blocks_per_cta blocks
+// in turn with the next pixels' points and normals on their way while these are
+// evaluated: level 0 of 30 640x480 instances 90 us against 105 us with a block
+// per CTA and one pixel after another, level 1 29 against 34.  More pixels at
+// once in fewer CTAs (4 pixels, 2 per SM: 103 us) or the other way round (1
+// pixel, 6 per SM: 94) is no better, nor are L2 prefetches of the next block.
+__global__ void __launch_bounds__(kLanes, kMaskCtas)
+    k_icp_mask(const InstDesc *D, int level, int blocks_per_cta) {
     pdl_trigger();
     __shared__ InstDesc sd;
     __shared__ float sT[16];
@@ -1029,31 +1121,17 @@ __global__ void __launch_bounds__(kLanes, RECON_MASK_MIN_BLOCKS) k_icp_mask(cons
     int n = (d.W >> level) * (d.H >> level);
     // the grid covers the batch's largest level; this instance has fewer blocks
     // (its per-block arrays hold exactly that many entries)
-    if ((int)blockIdx.x >= (n + kChunk - 1) / kChunk) return;
+    int nblk = (n + kChunk - 1) / kChunk;
+    int b0 = blockIdx.x * blocks_per_cta, b1 = min(b0 + blocks_per_cta, nblk);
+    if (b0 >= nblk) return;
     pdl_wait();
     if (threadIdx.x < 16) sT[threadIdx.x] = __ldcg(d.T + threadIdx.x);
     if (blockIdx.x == 0 && threadIdx.x == 0) d.work[2] += (unsigned long long)n;
     __syncthreads();
     int cnt = 0;
     long long vsum = 0;
-    const IcpLevel L(d, level);
-    const float *pl = d.ref_pl[level] + (size_t)blockIdx.x * 6 * kChunk + threadIdx.x;
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-        // (past the last pixel the planes hold 0, and the test on i ends it)
-        float p[6], r2;
-        bool ok;
-#pragma unroll
-        for (int k = 0; k < 6; k++) p[k] = __ldg(pl + k * kChunk + m * kLanes);
-        if (level == 0) ok = icp_mask_pixel<true>(L, sT, p, r2);
-        else ok = icp_mask_pixel<false>(L, sT, p, r2);
-        int i = blockIdx.x * kChunk + threadIdx.x + kLanes * m;
-        if (i >= n) continue;
-        if (ok) vsum += trunc_prod(r2, student_w(r2, 100.0f));
-        d.icp_r2[i] = r2;
-        d.icp_mask[i] = ok;
-        cnt += ok;
-    }
+    if (level == 0) icp_mask_blocks<true>(d, level, sT, b0, b1, n, cnt, vsum);
+    else icp_mask_blocks<false>(d, level, sT, b0, b1, n, cnt, vsum);
     cnt = __reduce_add_sync(0xffffffffu, cnt);
     for (int o = 16; o > 0; o >>= 1) vsum += __shfl_xor_sync(0xffffffffu, vsum, o);
     int wid = threadIdx.x >> 5;
@@ -1069,8 +1147,11 @@ __global__ void __launch_bounds__(kLanes, RECON_MASK_MIN_BLOCKS) k_icp_mask(cons
             c += s_cnt[k];
             v += s_var[k];
         }
-        d.icp_blkcnt[blockIdx.x] = c;
-        d.icp_blkvar[blockIdx.x] = v;
+        // the total of the CTA's blocks is its first block's
+        for (int b = b0; b < b1; b++) {
+            d.icp_blkcnt[b] = b == b0 ? c : 0;
+            d.icp_blkvar[b] = b == b0 ? v : 0;
+        }
     }
 }
 
@@ -1088,8 +1169,11 @@ __global__ void __launch_bounds__(kLanes, RECON_MASK_MIN_BLOCKS) k_icp_mask(cons
 // variance sum, which CTA 0 stores.  The sums are exact int64 sums, so the
 // result does not depend on how the pixels are split; one launch per pass
 // keeps every SM busy without any CTA waiting on another.  48 registers: five
-// CTAs per SM (kPassCtaSlots).
-__global__ void __launch_bounds__(kLanes) k_icp_student_pass(const InstDesc *D, int level, int pass,
+// CTAs per SM (kPassCtaSlots).  It was bound by the two IEEE divisions of the
+// weight: with the exact division by a reciprocal (StudentW), the three passes of
+// level 0 of 30 640x480 instances take 45 us against 63, level 1 23 against 27.
+// Passes 1 and 2 need no mask: a pixel that is no correspondence has r^2 = 0.
+__global__ void __launch_bounds__(kLanes, 5) k_icp_student_pass(const InstDesc *D, int level, int pass,
                                                              int blocks_per_cta) {
     pdl_trigger();
     __shared__ InstDesc sd;
@@ -1144,7 +1228,7 @@ __global__ void __launch_bounds__(kLanes) k_icp_student_pass(const InstDesc *D, 
     float Sf = (float)var;
     float minVal = (float)nsel;
     float vv = (nsel <= 1024) ? Sf : (Sf < minVal ? minVal : Sf);
-    float sigma2 = vv / (float)nsel;
+    const StudentW weight(vv / (float)nsel);
     long long vsum = 0;
     for (int b0 = b_first; b0 < b_last; b0 += 4) {
         float4 r[4];
@@ -1158,7 +1242,7 @@ __global__ void __launch_bounds__(kLanes) k_icp_student_pass(const InstDesc *D, 
             if (i + 3 < n) {
                 // 16- and 4-byte aligned: the arrays start on 256-byte boundaries
                 r[u] = __ldg(reinterpret_cast<const float4 *>(d.icp_r2 + i));
-                m[u] = __ldg(reinterpret_cast<const uchar4 *>(d.icp_mask + i));
+                if (pass == 3) m[u] = __ldg(reinterpret_cast<const uchar4 *>(d.icp_mask + i));
             } else {
                 // the instance's last pixels (n not a multiple of 4)
                 r[u].x = __ldg(d.icp_r2 + i);
@@ -1180,16 +1264,18 @@ __global__ void __launch_bounds__(kLanes) k_icp_student_pass(const InstDesc *D, 
             if (pass == 3) {
                 // pixels past the level's last one have mask 0: the weights
                 // are zero up to the end of the block
-                float4 w = make_float4(m[u].x ? fminf(student_w(r[u].x, sigma2), 1.0f) : 0.0f,
-                                       m[u].y ? fminf(student_w(r[u].y, sigma2), 1.0f) : 0.0f,
-                                       m[u].z ? fminf(student_w(r[u].z, sigma2), 1.0f) : 0.0f,
-                                       m[u].w ? fminf(student_w(r[u].w, sigma2), 1.0f) : 0.0f);
+                float4 w;
+                if (weight.in_range(((r[u].x + r[u].y) + r[u].z) + r[u].w))
+                    w = make_float4(weight.near(r[u].x), weight.near(r[u].y), weight.near(r[u].z), weight.near(r[u].w));
+                else
+                    w = make_float4(weight(r[u].x), weight(r[u].y), weight(r[u].z), weight(r[u].w));
+                w.x = m[u].x ? fminf(w.x, 1.0f) : 0.0f;
+                w.y = m[u].y ? fminf(w.y, 1.0f) : 0.0f;
+                w.z = m[u].z ? fminf(w.z, 1.0f) : 0.0f;
+                w.w = m[u].w ? fminf(w.w, 1.0f) : 0.0f;
                 *reinterpret_cast<float4 *>(d.icp_w + i) = w;
             } else {
-                if (m[u].x) vsum += trunc_prod(r[u].x, student_w(r[u].x, sigma2));
-                if (m[u].y) vsum += trunc_prod(r[u].y, student_w(r[u].y, sigma2));
-                if (m[u].z) vsum += trunc_prod(r[u].z, student_w(r[u].z, sigma2));
-                if (m[u].w) vsum += trunc_prod(r[u].w, student_w(r[u].w, sigma2));
+                vsum += weight.products(r[u]);
             }
         }
     }
@@ -2196,6 +2282,7 @@ __device__ __forceinline__ void student_body(const InstDesc *D, int level) {
         if (rank == 0 && t == 0) d.work[2] += (unsigned long long)n;
         __syncthreads();
         const IcpLevel L(d, level);
+        const StudentW first(100.0f);
         const float *pl = d.ref_pl[level];
         for (int i0 = rank * kStudentThreads + t; i0 < n; i0 += 2 * stride) {
             // two pixels at a time: point and normal loads in flight together
@@ -2211,7 +2298,7 @@ __device__ __forceinline__ void student_body(const InstDesc *D, int level) {
                 if (i >= n) continue;
                 float r2;
                 bool ok = level == 0 ? icp_mask_pixel<true>(L, sT, p[u], r2) : icp_mask_pixel<false>(L, sT, p[u], r2);
-                if (ok) v += trunc_prod(r2, student_w(r2, 100.0f));
+                if (ok) v += trunc_prod(r2, first(r2));
                 d.icp_r2[i] = r2;
                 d.icp_mask[i] = ok;
                 c += ok;
@@ -2261,7 +2348,7 @@ __device__ __forceinline__ void student_body(const InstDesc *D, int level) {
         float Sf = (float)var;
         float minVal = (float)nsel;
         float vv = (nsel <= 1024) ? Sf : (Sf < minVal ? minVal : Sf);
-        float sigma2 = vv / (float)nsel;
+        const StudentW weight(vv / (float)nsel);
         long long vsum = 0;
         int i = rank * kStudentThreads + t;
         float r_next = 0.0f;
@@ -2279,9 +2366,9 @@ __device__ __forceinline__ void student_body(const InstDesc *D, int level) {
                 m_next = __ldg(d.icp_mask + i + stride);
             }
             if (pass == 3) {
-                d.icp_w[i] = mk ? fminf(student_w(r, sigma2), 1.0f) : 0.0f;
+                d.icp_w[i] = mk ? fminf(weight(r), 1.0f) : 0.0f;
             } else if (mk) {
-                vsum += trunc_prod(r, student_w(r, sigma2));
+                vsum += trunc_prod(r, weight(r));
             }
         }
         if (pass == 3) {

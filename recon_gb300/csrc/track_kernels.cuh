@@ -18,6 +18,8 @@ constexpr int kVtxPlanes = 9;    // a vertex record: x y z px py gx gy gmag gray
 constexpr int kIterCluster = 8;  // CTAs of the photometric cluster of the GN iteration kernel
 constexpr int kIterBlock = 256;  // threads of a GN iteration CTA
 constexpr int kIterCtaSlots = 4 * 152;  // GN iteration CTAs resident on a 152-SM GB300
+constexpr int kMaskCtas = 4;  // 256-thread correspondence CTAs per SM (64 registers)
+constexpr int kMaskCtaSlots = kMaskCtas * 152;
 constexpr int kPassCtaSlots = 5 * 152;  // 256-thread Student-t pass CTAs resident on a 152-SM GB300
 constexpr int kSolveThreads = 64;        // threads of the per-instance solve CTA
 constexpr int kFxLimbs = 4;      // limbs of a fixed-point sum (fx.cuh)
