@@ -22,11 +22,11 @@
 
 namespace rt {
 __global__ void k_convert_level0(const InstDesc *D, const uint8_t *const *in_gray, const uint16_t *const *in_depth,
-                                 const float *const *in_rgbd);
+                                 const float *const *in_rgbd, int per_cta);
 __global__ void k_downsample(const InstDesc *D, int level, const int *active);
-__global__ void k_normals(const InstDesc *D, const int *active);
+__global__ void k_normals(const InstDesc *D, const int *active, int per_cta);
 __global__ void k_oriented_points(const InstDesc *D, const float *const *in_pts, const float *const *in_nrm);
-__global__ void k_xyz2cloud(const InstDesc *D, const int *active);
+__global__ void k_xyz2cloud(const InstDesc *D, const int *active, int per_cta);
 __global__ void k_seg_count(const InstDesc *D, const int *active);
 __global__ void k_seg_scan(const InstDesc *D, const int *active);
 __global__ void k_seg_scatter(const InstDesc *D, const int *active);
@@ -50,7 +50,6 @@ __global__ void k_store_pose(const InstDesc *D, float *dst);
 __global__ void k_gather_results(const InstDesc *D, int *dst);
 __global__ void k_fuse_depth(const InstDesc *D, int nframes, int n_inst, const uint16_t *const *depth,
                              const uint8_t *const *gray, const float *Tf, float gate, const int *active);
-__global__ void k_ref_from_z(const InstDesc *D, const int *active);
 __global__ void k_net_coarse(const InstDesc *D, const uint8_t *const *in_gray, const uint16_t *const *in_depth,
                              const __nv_bfloat16 *prev, __nv_bfloat16 *out, __nv_bfloat16 *net_in);
 __global__ void k_gate_twist(const InstDesc *D, const float *net_out, const float *scale, float *Dout);
@@ -465,16 +464,19 @@ int prepare_reference(recon_batch *b, bool from_inputs = true, bool reset_pose =
     auto D = b->d_desc;
     auto in = b->d_inptr;
     const int *active = active_flags ? active_flags : b->d_active;
+    // pixels per CTA of the keyframe's per-pixel kernels: more than one per thread
+    // where the batch fills the device several times over (fewer CTAs without
+    // pixels in a mixed batch, fewer histograms to add up), one where it does not
+    const int per = (long long)n * b->max_pix >= 4LL * 152 * 8 * 256 ? 1024 : 256;
+    const dim3 grid_prep((b->max_pix + per - 1) / per, n);
     if (from_inputs)
-        k_convert_level0<<<grid_pix(b->max_pix, n), 256, 0, s>>>(
-            D, (const uint8_t *const *)in, (const uint16_t *const *)(in + n), (const float *const *)(in + 2 * n));
-    else
-        k_ref_from_z<<<grid_pix(b->max_pix, n), 256, 0, s>>>(D, active);
-    k_normals<<<grid_pix(b->max_pix, n), 256, 0, s>>>(D, active);
+        k_convert_level0<<<grid_prep, 256, 0, s>>>(D, (const uint8_t *const *)in, (const uint16_t *const *)(in + n),
+                                                   (const float *const *)(in + 2 * n), per);
+    k_normals<<<grid_prep, 256, 0, s>>>(D, active, per);
     // the photometric vertex records take the points of the keyframe depth
     // (ref_z), not the level-0 ICP points that oriented points may replace
     k_clear_ref<<<dim3(1, n), 256, 0, s>>>(D, active);
-    k_xyz2cloud<<<grid_pix(b->max_pix, n), 256, 0, s>>>(D, active);
+    k_xyz2cloud<<<grid_prep, 256, 0, s>>>(D, active, per);
     if (oriented) {
         k_oriented_points<<<grid_pix(b->max_pix, n), 256, 0, s>>>(D, (const float *const *)(in + 3 * n),
                                                                    (const float *const *)(in + 4 * n));
@@ -487,7 +489,7 @@ int prepare_reference(recon_batch *b, bool from_inputs = true, bool reset_pose =
     k_seg_scatter<<<dim3(kSegments / 8, n), 256, 0, s>>>(D, active);
     k_attr_jac<<<grid_pix(b->max_P, n), 256, 0, s>>>(D, active);
     if (reset_pose) k_reset_pose<<<dim3(1, n), 32, 0, s>>>(D, active);
-    g_launches += 9 + (b->max_L - 1) + (reset_pose ? 1 : 0);
+    g_launches += (from_inputs ? 8 : 7) + (b->max_L - 1) + (reset_pose ? 1 : 0);
     CK(cudaGetLastError());
     return RECON_OK;
 }

@@ -35,12 +35,46 @@ __device__ __forceinline__ void load_desc(InstDesc &sd, const InstDesc *src_desc
 // input conversion and pyramids
 // ------------------------------------------------------------------
 
+// Back-projection with the IR camera, (x - cx) z / fx and (y - cy) z / fy: all
+// pixels divide by the same focal lengths, so by their reciprocals and the exact
+// division of pair_math.cuh.  (A pixel on the principal point's column or row, whose
+// quotient is -0, takes the division.)
+struct PixelRays {
+    float fx, fy, cx, cy, rfx, rfy;
+    bool plain;
+    __device__ __forceinline__ explicit PixelRays(const float *KL) : fx(KL[0]), fy(KL[4]), cx(KL[2]), cy(KL[5]) {
+        plain = div_in_range(fx, fy, fx);
+        rfx = rcp_rn(fx);
+        rfy = rcp_rn(fy);
+    }
+    __device__ __forceinline__ void point(int xi, int yi, float z, float &x, float &y) const {
+        float ax = ((float)xi - cx) * z, ay = ((float)yi - cy) * z;
+        x = div_rn(ax, -fx, rfx);
+        y = div_rn(ay, -fy, rfy);
+        if (!(plain && div_in_range(ax, ay, ax))) {
+            x = ieee_div(ax, fx);
+            y = ieee_div(ay, fy);
+        }
+    }
+};
+
+// three sums over ns = 1 .. 4 values into their means
+__device__ __forceinline__ void mean3(float ns, float &a, float &b, float &c) {
+    float y = rcp_rn(ns), qa = div_rn(a, -ns, y), qb = div_rn(b, -ns, y), qc = div_rn(c, -ns, y);
+    if (!(div_in_range(a) && div_in_range(b) && div_in_range(c))) {
+        qa = ieee_div(a, ns);
+        qb = ieee_div(b, ns);
+        qc = ieee_div(c, ns);
+    }
+    a = qa;
+    b = qb;
+    c = qc;
+}
+
 // The reference frame's level 0: uint8 gray -> [0,1], uint16 mm -> z = -mm
 // (rgb2gray.cu:64-76 for the u8/u16 form, or the float4 RGBA+depth frame with
-// its y-flip, rgbTex2GrayHdrZKernel), and its xyz + mask
-// (convertZMapToXYZ6Kernel, rgb2gray.cu:595-624; the same formula as
-// convertZMapToXYZKernel, 570-593).  The current frame uses
-// k_prep_current_pyramid.
+// its y-flip, rgbTex2GrayHdrZKernel); k_normals forms its points.  The current
+// frame uses k_prep_current_pyramid.
 __device__ __forceinline__ void convert_pixel(const InstDesc &d, const uint8_t *gp, const uint16_t *dp, const float *fp,
                                               int i, int xi, int yi, float &g, float &z) {
     if (fp) {
@@ -50,39 +84,30 @@ __device__ __forceinline__ void convert_pixel(const InstDesc &d, const uint8_t *
         float minDist = d.calib[RC_MIND], maxDist = d.calib[RC_MAXD];
         z = -(p.w * (maxDist - minDist) + minDist);
     } else {
-        g = (float)__ldg(gp + i) / 255.0f;
+        g = gray_unit(__ldg(gp + i));
         uint16_t dm = __ldg(dp + i);
         z = dm ? -(float)dm : 0.0f;
     }
 }
 
 __global__ void k_convert_level0(const InstDesc *D, const uint8_t *const *in_gray, const uint16_t *const *in_depth,
-                                 const float *const *in_rgbd) {
+                                 const float *const *in_rgbd, int per_cta) {
     INST_DESC;
     const uint8_t *gp = in_gray[blockIdx.y];
     const uint16_t *dp = in_depth[blockIdx.y];
     const float *fp = in_rgbd[blockIdx.y];
     if (!fp && (!gp || !dp)) return;  // instance not updated by this call
     int n = d.W * d.H;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int xi = i % d.W, yi = i / d.W;
-    float g, z;
-    convert_pixel(d, gp, dp, fp, i, xi, yi, g, z);
-    float fx = d.calib[RC_KL], fy = d.calib[RC_KL + 4];
-    float cx = d.calib[RC_KL + 2], cy = d.calib[RC_KL + 5];
-    d.ref_gray[0][i] = g;
-    d.ref_z[i] = z;
-    d.ref_col[i] = -1.0f;  // a new keyframe has no fused colour
-    float minDist = d.calib[RC_MIND], maxDist = d.calib[RC_MAXD];
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (z < -minDist && z > -maxDist) {
-        o.x = ((float)xi - cx) * z / fx;
-        o.y = ((float)yi - cy) * z / fy;
-        o.z = z;
-        o.w = 1.0f;
+#pragma unroll 4
+    for (int m = 0; m < per_cta; m += 256) {
+        int i = blockIdx.x * per_cta + m + threadIdx.x;
+        if (i >= n) return;
+        float g, z;
+        convert_pixel(d, gp, dp, fp, i, i % d.W, i / d.W, g, z);
+        d.ref_gray[0][i] = g;
+        d.ref_z[i] = z;
+        d.ref_col[i] = -1.0f;  // a new keyframe has no fused colour
     }
-    d.ref_pts[0][i] = o;
 }
 
 // The current frame's whole pyramid in one pass: the level-0 conversion
@@ -90,18 +115,16 @@ __global__ void k_convert_level0(const InstDesc *D, const uint8_t *const *in_gra
 // and the 2x2 reductions of fastDownSampleHdrKernel and downSampleCloud6Kernel
 // for the coarser levels (the expressions of k_downsample, in its order), so
 // every value is identical to the separate kernels'.  A CTA of 256 threads
-// takes a 32x32 tile of level 0: each thread converts one 2x2 block and
+// takes a 32x32 tile of level 0 (54 us for 30 640x480 frames, of which the bytes
+// take 24; 68 us with IEEE divisions and one pixel per access): each thread converts one 2x2 block and
 // reduces it to its level-1 pixel in registers; levels 2 and 3 come from the
 // level-1 tile in shared memory.  Level 0 is never read back.
 constexpr int kPyrTile = 32;
 
-__device__ __forceinline__ void cloud_point(const InstDesc &d, int xi, int yi, float z, float4 &o) {
-    float fx = d.calib[RC_KL], fy = d.calib[RC_KL + 4];
-    float cx = d.calib[RC_KL + 2], cy = d.calib[RC_KL + 5];
+__device__ __forceinline__ void cloud_point(const PixelRays &rays, int xi, int yi, float z, float4 &o) {
     o = make_float4(0.f, 0.f, 0.f, 0.f);
     if (z < 0) {
-        o.x = ((float)xi - cx) * z / fx;
-        o.y = ((float)yi - cy) * z / fy;
+        rays.point(xi, yi, z, o.x, o.y);
         o.z = z;
         o.w = 1.0f;
     }
@@ -121,7 +144,10 @@ __device__ __forceinline__ float4 down_points(const float4 &a, const float4 &b, 
         }
     }
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (ns > 0.0f) o = make_float4(p0 / ns, p1 / ns, p2 / ns, 1.0f);
+    if (ns > 0.0f) {
+        mean3(ns, p0, p1, p2);
+        o = make_float4(p0, p1, p2, 1.0f);
+    }
     return o;
 }
 
@@ -137,6 +163,9 @@ __global__ void __launch_bounds__(256) k_prep_current_pyramid(const InstDesc *D,
     __shared__ float sg[2][256];   // gray of levels 1 (16x16) and 2 (8x8)
     __shared__ float4 sp[2][256];  // points of levels 1 and 2
     load_desc(sd, D + blockIdx.y);
+    const uint8_t *gp = in_gray[blockIdx.y];
+    const uint16_t *dp = in_depth[blockIdx.y];
+    const float *fp = in_rgbd[blockIdx.y];
     __syncthreads();
     const InstDesc &d = sd;
     if (blockIdx.x == 0) {
@@ -152,9 +181,6 @@ __global__ void __launch_bounds__(256) k_prep_current_pyramid(const InstDesc *D,
             if (t < 2) d.fx_bad[t] = 0;
         }
     }
-    const uint8_t *gp = in_gray[blockIdx.y];
-    const uint16_t *dp = in_depth[blockIdx.y];
-    const float *fp = in_rgbd[blockIdx.y];
     if (!fp && (!gp || !dp)) return;  // instance not updated by this call
     int W = d.W, H = d.H;
     int tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
@@ -166,7 +192,28 @@ __global__ void __launch_bounds__(256) k_prep_current_pyramid(const InstDesc *D,
     float g[4];
     float4 pt[4];
     bool in0 = x0 < W && y0 < H;
-    if (in0) {
+    const PixelRays rays(d.calib + RC_KL);
+    // pixels in pairs where the width is even and the inputs are aligned to it
+    if (in0 && !fp && !(W & 1) && !(reinterpret_cast<uintptr_t>(gp) & 1) && !(reinterpret_cast<uintptr_t>(dp) & 3)) {
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            g[2 * r] = g[2 * r + 1] = 0.0f;
+            pt[2 * r] = pt[2 * r + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (y0 + r >= H) continue;
+            int i = x0 + (y0 + r) * W;
+            uchar2 gg = __ldg(reinterpret_cast<const uchar2 *>(gp + i));
+            ushort2 dd = __ldg(reinterpret_cast<const ushort2 *>(dp + i));
+            float2 gf = make_float2(gray_unit(gg.x), gray_unit(gg.y));
+            float2 z = make_float2(dd.x ? -(float)dd.x : 0.0f, dd.y ? -(float)dd.y : 0.0f);
+            *reinterpret_cast<float2 *>(d.cur_gray[0] + i) = gf;
+            *reinterpret_cast<float2 *>(d.cur_z + i) = z;
+            if (d.cur_grayh[0]) *reinterpret_cast<__half2 *>(d.cur_grayh[0] + i) = __floats2half2_rn(gf.x, gf.y);
+            g[2 * r] = gf.x;
+            g[2 * r + 1] = gf.y;
+            cloud_point(rays, x0, y0 + r, z.x, pt[2 * r]);
+            cloud_point(rays, x0 + 1, y0 + r, z.y, pt[2 * r + 1]);
+        }
+    } else if (in0) {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             int xi = x0 + (k & 1), yi = y0 + (k >> 1);
@@ -176,7 +223,7 @@ __global__ void __launch_bounds__(256) k_prep_current_pyramid(const InstDesc *D,
             int i = xi + yi * W;
             float z;
             convert_pixel(d, gp, dp, fp, i, xi, yi, g[k], z);
-            cloud_point(d, xi, yi, z, pt[k]);
+            cloud_point(rays, xi, yi, z, pt[k]);
             d.cur_gray[0][i] = g[k];
             if (d.cur_grayh[0]) d.cur_grayh[0][i] = __float2half_rn(g[k]);  // mixed precision
             d.cur_z[i] = z;
@@ -268,12 +315,8 @@ __global__ void k_downsample(const InstDesc *D, int level, const int *active) {
         }
     }
     if (ns > 0.0f) {
-        p0 /= ns;
-        p1 /= ns;
-        p2 /= ns;
-        n0 /= ns;
-        n1 /= ns;
-        n2 /= ns;
+        mean3(ns, p0, p1, p2);
+        mean3(ns, n0, n1, n2);
         normalize3(n0, n1, n2);
         d.ref_nrm[level][i] = make_float4(n0, n1, n2, 0.0f);
         d.ref_pts[level][i] = make_float4(p0, p1, p2, 1.0f);
@@ -286,6 +329,12 @@ __global__ void k_downsample(const InstDesc *D, int level, const int *active) {
     }
 }
 
+// 1 / v, rounded once
+__device__ __forceinline__ float reciprocal(float v) {
+    float a = fabsf(v);
+    return a >= kDivLo && a <= kDivHi ? rcp_rn(v) : ieee_div(1.0f, v);
+}
+
 // Gray value the RGB camera sees at point (qx, qy, qz) of its rig's IR frame
 // (TLR, distortPoint and the bilinear color1 tap of xyz2CloudKernel,
 // d2z.cu:235-331, with the perspective division as one reciprocal and two
@@ -296,7 +345,7 @@ __device__ __forceinline__ float rgb_sample(const float *calib, float qx, float 
                                             int H) {
     float rx, ry, rz;
     mul4(calib + RC_TLR, qx, qy, qz, rx, ry, rz);
-    float irz = 1.0f / rz;
+    float irz = reciprocal(rz);
     float pux = rx * irz, puy = ry * irz;
     float px, py;
     distort(pux, puy, calib + RC_KCR, calib + RC_KR, px, py);
@@ -323,7 +372,8 @@ __device__ __forceinline__ float rgb_sample(const float *calib, float qx, float 
 // depth / gray: nframes x n_inst frame pointers (gray may be null: depth only,
 // colours kept); Tf: nframes x n_inst x 16 poses.
 // 8 CTAs per SM (32 registers, a few bytes of spill): more warps to hide the
-// per-frame gathers, 447 against 496 us per 30 x 5-frame launch at 44 registers
+// per-frame gathers, 402 us per 30 x 5-frame launch (471 us with IEEE reciprocals and
+// divisions by 255)
 #ifndef RECON_FUSE_MIN_BLOCKS
 #define RECON_FUSE_MIN_BLOCKS 8
 #endif
@@ -370,7 +420,7 @@ __global__ void __launch_bounds__(256, RECON_FUSE_MIN_BLOCKS) k_fuse_depth(const
     for (int f = 0; f < nframes && f < 8; f++) {
         float qx, qy, qz;
         mul4(sT[f], px3, py3, pz3, qx, qy, qz);
-        float iqz = 1.0f / qz;
+        float iqz = reciprocal(qz);
         float q2x = qx * iqz, q2y = qy * iqz;
         float pxl = KL[0] * q2x + KL[1] * q2y + KL[2];
         float pyl = KL[3] * q2x + KL[4] * q2y + KL[5];
@@ -399,27 +449,6 @@ __global__ void __launch_bounds__(256, RECON_FUSE_MIN_BLOCKS) k_fuse_depth(const
     if (colour) d.ref_col[idx] = cw > 0.0f ? csum / cw : -1.0f;
 }
 
-// reference level-0 points from ref_z (convertZMapToXYZ6Kernel, rgb2gray.cu:595-624)
-__global__ void k_ref_from_z(const InstDesc *D, const int *active) {
-    INST_DESC;
-    if (!active[blockIdx.y]) return;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.W * d.H) return;
-    int xi = i % d.W, yi = i / d.W;
-    float fx = d.calib[RC_KL], fy = d.calib[RC_KL + 4];
-    float cx = d.calib[RC_KL + 2], cy = d.calib[RC_KL + 5];
-    float minDist = d.calib[RC_MIND], maxDist = d.calib[RC_MAXD];
-    float z = d.ref_z[i];
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (z < -minDist && z > -maxDist) {
-        o.x = ((float)xi - cx) * z / fx;
-        o.y = ((float)yi - cy) * z / fy;
-        o.z = z;
-        o.w = 1.0f;
-    }
-    d.ref_pts[0][i] = o;
-}
-
 // genOrientedPoints6Kernel (d2z.cu:471-501): the filtered reference's level-0
 // ICP points and normals from a ray-cast point image and its normals (float4
 // maps of the keyframe's pixels, camera frame); replaces what k_normals wrote
@@ -444,38 +473,55 @@ __global__ void k_oriented_points(const InstDesc *D, const float *const *in_pts,
     }
 }
 
-// computeNormalsCudaKernel, d2z.cu:503-537 (reference level 0)
-__global__ void k_normals(const InstDesc *D, const int *active) {
+// The reference's level-0 ICP point of a keyframe pixel of depth z
+// (convertZMapToXYZ6Kernel, rgb2gray.cu:595-624; the same formula as
+// convertZMapToXYZKernel, 570-593): zero out of range.
+__device__ __forceinline__ float4 ref_point(const InstDesc &d, const PixelRays &rays, int xi, int yi, float z) {
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (z < -d.calib[RC_MIND] && z > -d.calib[RC_MAXD]) {
+        rays.point(xi, yi, z, o.x, o.y);
+        o.z = z;
+        o.w = 1.0f;
+    }
+    return o;
+}
+
+// The reference's level 0 from the keyframe depth: the points, and their normals
+// and masks (computeNormalsCudaKernel, d2z.cu:503-537).  It is bound by the 56
+// bytes that it writes per pixel; a pixel's four neighbours are formed from their
+// depths again, which costs less than reading points that another kernel wrote
+// (30 640x480 frames: 108 us here and 39 for the conversion, against 105 and 80,
+// and no launch of its own, 52 us, to form the points of a fused depth).
+__global__ void k_normals(const InstDesc *D, const int *active, int per_cta) {
     INST_DESC;
     if (!active[blockIdx.y]) return;
     int W = d.W, H = d.H;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= W * H) return;
-    int xi = i % W, yi = i / W;
-    float4 me = d.ref_pts[0][i];
-    float4 nrm = make_float4(0.f, 0.f, 0.f, 0.f);
-    float mask = me.w;
-    if (xi < 1 || yi < 1 || xi > W - 2 || yi > H - 2) {
-        mask = 0.0f;
-    } else {
-        float4 x1 = d.ref_pts[0][i - 1], x2 = d.ref_pts[0][i + 1];
-        float4 y1 = d.ref_pts[0][i - W], y2 = d.ref_pts[0][i + W];
-        if (x1.z < 0 && x2.z < 0 && y1.z < 0 && y2.z < 0) {
-            float ux = x2.x - x1.x, uy = x2.y - x1.y, uz = x2.z - x1.z;
-            float vx = y2.x - y1.x, vy = y2.y - y1.y, vz = y2.z - y1.z;
-            float nx = uy * vz - uz * vy;
-            float ny = -(ux * vz - uz * vx);
-            float nz = ux * vy - uy * vx;
-            normalize3(nx, ny, nz);
-            nrm = make_float4(nx, ny, nz, 0.0f);
-        } else {
-            mask = 0.0f;
+    const PixelRays rays(d.calib + RC_KL);
+    const float *z = d.ref_z;
+    for (int m = 0; m < per_cta; m += 256) {
+        int i = blockIdx.x * per_cta + m + threadIdx.x;
+        if (i >= W * H) return;
+        int xi = i % W, yi = i / W;
+        float4 me = ref_point(d, rays, xi, yi, z[i]), nrm = make_float4(0.f, 0.f, 0.f, 0.f);
+        float mask = 0.0f;
+        if (!(xi < 1 || yi < 1 || xi > W - 2 || yi > H - 2)) {
+            float4 x1 = ref_point(d, rays, xi - 1, yi, z[i - 1]), x2 = ref_point(d, rays, xi + 1, yi, z[i + 1]);
+            float4 y1 = ref_point(d, rays, xi, yi - 1, z[i - W]), y2 = ref_point(d, rays, xi, yi + 1, z[i + W]);
+            if (x1.z < 0 && x2.z < 0 && y1.z < 0 && y2.z < 0) {
+                float ux = x2.x - x1.x, uy = x2.y - x1.y, uz = x2.z - x1.z;
+                float vx = y2.x - y1.x, vy = y2.y - y1.y, vz = y2.z - y1.z;
+                float nx = uy * vz - uz * vy;
+                float ny = -(ux * vz - uz * vx);
+                float nz = ux * vy - uy * vx;
+                normalize3(nx, ny, nz);
+                nrm = make_float4(nx, ny, nz, 0.0f);
+                mask = me.w;
+            }
         }
+        d.ref_nrm[0][i] = nrm;
+        d.ref_pts[0][i] = make_float4(me.x, me.y, me.z, mask);
+        store_ref_planes(d.ref_pl[0], i, me.x, me.y, me.z, mask, nrm.x, nrm.y, nrm.z);
     }
-    d.ref_nrm[0][i] = nrm;
-    // only .w changes; neighbours read x/y/z of this element, which stay the same
-    d.ref_pts[0][i].w = mask;
-    store_ref_planes(d.ref_pl[0], i, me.x, me.y, me.z, mask, nrm.x, nrm.y, nrm.z);
 }
 
 // ------------------------------------------------------------------
@@ -488,8 +534,8 @@ __global__ void k_normals(const InstDesc *D, const int *active) {
 // evaluate it twice with the same operations: for every pixel to find the
 // gradient magnitude that selects the points, and again for the selected
 // points only (so that the other eight planes are never stored).  The point
-// is the back-projection of the keyframe depth ref_z, formed as
-// k_convert_level0 and k_ref_from_z form the level-0 ICP points (zero out of
+// is the back-projection of the keyframe depth ref_z, formed as k_normals forms
+// the level-0 ICP points (zero out of
 // range: xyz alone carries the validity), so a filtered reference's oriented
 // points, which later replace those, do not enter it.
 __device__ __forceinline__ void vertex_record(const InstDesc &d, int i, int W, int H, float *v) {
@@ -500,10 +546,7 @@ __device__ __forceinline__ void vertex_record(const InstDesc &d, int i, int W, i
         float z = d.ref_z[i];
         float minDist = d.calib[RC_MIND], maxDist = d.calib[RC_MAXD];
         if (z < -minDist && z > -maxDist) {
-            float fx = d.calib[RC_KL], fy = d.calib[RC_KL + 4];
-            float cx = d.calib[RC_KL + 2], cy = d.calib[RC_KL + 5];
-            p3x = ((float)(i % W) - cx) * z / fx;
-            p3y = ((float)(i / W) - cy) * z / fy;
+            PixelRays(d.calib + RC_KL).point(i % W, i / W, z, p3x, p3y);
             p3z = z;
         }
     }
@@ -511,20 +554,41 @@ __device__ __forceinline__ void vertex_record(const InstDesc &d, int i, int W, i
         const float *T = d.calib + RC_TLR;
         float rx, ry, rz;
         mul4(T, p3x, p3y, p3z, rx, ry, rz);
-        float pux = rx / rz, puy = ry / rz;
+        float irz = rcp_rn(rz), pux = div_rn(rx, -rz, irz), puy = div_rn(ry, -rz, irz);
+        if (!div_in_range(rx, ry, rz)) {
+            pux = ieee_div(rx, rz);
+            puy = ieee_div(ry, rz);
+        }
         float px, py;
         distort(pux, puy, d.calib + RC_KCR, d.calib + RC_KR, px, py);
         if (in_bounds10(px, py, W, H)) {
             const float *img = d.ref_gray[0];
             int xdi = ftoi(px), ydi = ftoi(py);
             float fx = px - xdi, fy = py - ydi;
-            float color1 = bilin(xdi, ydi, fx, fy, W, img);
+            float color1, colorN, colorE, colorW, colorS;
+            if (ftoi(px + 1.0f) == xdi + 1 && ftoi(px - 1.0f) == xdi - 1 && ftoi(py + 1.0f) == ydi + 1 &&
+                ftoi(py - 1.0f) == ydi - 1) {
+                // the five interpolations share 12 taps and their weights
+                float w0 = (1 - fx) * (1 - fy), w1 = fx * (1 - fy), w2 = (1 - fx) * fy, w3 = fx * fy;
+                const float *q = img + xdi + ydi * W;
+                float a1 = __ldg(q - W), a2 = __ldg(q - W + 1);
+                float b0 = __ldg(q - 1), b1 = __ldg(q), b2 = __ldg(q + 1), b3 = __ldg(q + 2);
+                float c0 = __ldg(q + W - 1), c1 = __ldg(q + W), c2 = __ldg(q + W + 1), c3 = __ldg(q + W + 2);
+                float e1 = __ldg(q + 2 * W), e2 = __ldg(q + 2 * W + 1);
+                color1 = w0 * b1 + w1 * b2 + w2 * c1 + w3 * c2;
+                colorN = w0 * a1 + w1 * a2 + w2 * b1 + w3 * b2;
+                colorE = w0 * b2 + w1 * b3 + w2 * c2 + w3 * c3;
+                colorW = w0 * b0 + w1 * b1 + w2 * c0 + w3 * c1;
+                colorS = w0 * c1 + w1 * c2 + w2 * e1 + w3 * e2;
+            } else {  // a coordinate that one more rounding takes to the next pixel
+                color1 = bilin(xdi, ydi, fx, fy, W, img);
+                colorN = bilin(ftoi(px), ftoi(py - 1.0f), fx, fy, W, img);
+                colorE = bilin(ftoi(px + 1.0f), ftoi(py), fx, fy, W, img);
+                colorW = bilin(ftoi(px - 1.0f), ftoi(py), fx, fy, W, img);
+                colorS = bilin(ftoi(px), ftoi(py + 1.0f), fx, fy, W, img);
+            }
             float fused = d.ref_col[i];  // the keyframe fusion's vertex colour, if any
             if (fused >= 0.0f) color1 = fused;
-            float colorN = bilin(ftoi(px), ftoi(py - 1.0f), fx, fy, W, img);
-            float colorE = bilin(ftoi(px + 1.0f), ftoi(py), fx, fy, W, img);
-            float colorW = bilin(ftoi(px - 1.0f), ftoi(py), fx, fy, W, img);
-            float colorS = bilin(ftoi(px), ftoi(py + 1.0f), fx, fy, W, img);
             float gradX1 = (colorE - colorW) / 2.0f;
             float gradY1 = (colorS - colorN) / 2.0f;
             float gm = fabsf(gradY1) + fabsf(gradX1);
@@ -539,8 +603,10 @@ __device__ __forceinline__ void vertex_record(const InstDesc &d, int i, int W, i
 
 // The gradient magnitude of every keyframe pixel (xyz2CloudKernel's gmag
 // plane) and its 256-bin histogram (gpu_hist.cu:136, cuda_hist.cu:100-152)
-// with privatised shared-memory integer atomics.
-__global__ void k_xyz2cloud(const InstDesc *D, const int *active) {
+// with privatised shared-memory integer atomics.  Bound by the gathers of its 12
+// taps and by the bins that each CTA adds to the instance's: 256 mixed frames
+// 272 us with four pixels a thread, 466 with one, 20 taps and IEEE divisions.
+__global__ void k_xyz2cloud(const InstDesc *D, const int *active, int per_cta) {
     INST_DESC;
     if (!active[blockIdx.y]) return;
     __shared__ int sh[1024];
@@ -548,8 +614,7 @@ __global__ void k_xyz2cloud(const InstDesc *D, const int *active) {
     for (int k = threadIdx.x; k < nb; k += blockDim.x) sh[k] = 0;
     __syncthreads();
     int W = d.W, H = d.H, n = W * H;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
+    for (int i = blockIdx.x * per_cta + threadIdx.x; i < min(n, ((int)blockIdx.x + 1) * per_cta); i += blockDim.x) {
         float v[kVtxPlanes];
         vertex_record(d, i, W, H, v);
         d.gmag[i] = v[7];
@@ -576,18 +641,32 @@ __global__ void k_seg_count(const InstDesc *D, const int *active) {
     // search (from the top bin down) then reads shared memory only
     for (int k = threadIdx.x; k < nb; k += blockDim.x) s_hist[k] = __ldcg(d.grad_hist + k);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned int thr = 0;
-        int sel = 0;
-        for (int k = nb - 1; k >= 0; k--) {
-            sel += s_hist[k];
-            if (sel > P) { thr = (unsigned)k; break; }
+    if (threadIdx.x < 32) {
+        // from the top bin down, 32 bins at a time: the first at which the running
+        // count passes P (bin 0 when none does)
+        int above = 0, thr = 0, sel = 0, l = threadIdx.x;
+        for (int top = nb - 1;; top -= 32) {
+            int k = top - l, incl = k >= 0 ? s_hist[k] : 0;
+            for (int o = 1; o < 32; o <<= 1) {
+                int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (l >= o) incl += t;
+            }
+            unsigned past = __ballot_sync(0xffffffffu, above + incl > P);
+            if (past || top < 32) {
+                int first = past ? __ffs(past) - 1 : 31;
+                sel = above + __shfl_sync(0xffffffffu, incl, first);
+                thr = past ? top - first : 0;
+                break;
+            }
+            above += __shfl_sync(0xffffffffu, incl, 31);
         }
-        s_thr = thr;
-        s_excess = sel - P;
-        if (blockIdx.x == 0) {
-            d.seg[3072] = (int)thr;
-            d.seg[3073] = sel - P;
+        if (l == 0) {
+            s_thr = (unsigned)thr;
+            s_excess = sel - P;
+            if (blockIdx.x == 0) {
+                d.seg[3072] = thr;
+                d.seg[3073] = sel - P;
+            }
         }
     }
     __syncthreads();
@@ -599,15 +678,16 @@ __global__ void k_seg_count(const InstDesc *D, const int *active) {
     const float *grad = d.gmag;
     unsigned int thr = s_thr;
     int cnt = 0, mcnt = 0;
+#pragma unroll 4
     for (int base = warp * ppt; base < warp * ppt + ppt; base += 32) {
         int i = base + lane;
         bool in = i < warp * ppt + ppt;
-        unsigned int q = in ? (unsigned int)(grad[i] * (nb - 1) + 0.5f) : 0u;
-        unsigned int ab = __ballot_sync(0xffffffffu, in && q > thr);
-        unsigned int me = __ballot_sync(0xffffffffu, in && q == thr);
-        cnt += __popc(ab);
-        mcnt += __popc(me);
+        unsigned int q = in ? (unsigned int)(__ldg(grad + i) * (nb - 1) + 0.5f) : 0u;
+        cnt += in && q > thr;
+        mcnt += in && q == thr;
     }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    mcnt = __reduce_add_sync(0xffffffffu, mcnt);
     if (lane == 0) {
         d.seg[warp] = cnt;
         d.seg[512 + warp] = mcnt;
@@ -699,10 +779,11 @@ __global__ void k_seg_scatter(const InstDesc *D, const int *active) {
     int kept = d.seg[2048 + warp];
     int m = 0;
     unsigned int lower = (1u << lane) - 1u;
+#pragma unroll 4
     for (int base = warp * ppt; base < warp * ppt + ppt; base += 32) {
         int i = base + lane;
         bool in = i < warp * ppt + ppt;
-        unsigned int q = in ? (unsigned int)(grad[i] * (nb - 1) + 0.5f) : 0u;
+        unsigned int q = in ? (unsigned int)(__ldg(grad + i) * (nb - 1) + 0.5f) : 0u;
         bool ia = in && q > thr, im = in && q == thr;
         unsigned int ab = __ballot_sync(0xffffffffu, ia);
         unsigned int me = __ballot_sync(0xffffffffu, im);

@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "pair_math.cuh"
+
 #define RC_KR 0
 #define RC_KCR 18
 #define RC_TLR 26
@@ -64,8 +66,10 @@ __device__ __forceinline__ void distort(float pux, float puy, const float *kc, c
 __device__ __forceinline__ float ldf(const float *p) { return __ldg(p); }
 __device__ __forceinline__ float ldf(const __half *p) { return __half2float(__ldg(p)); }
 __device__ __forceinline__ float ldf(const __nv_bfloat16 *p) { return __bfloat162float(__ldg(p)); }
-// a uint8 gray value in [0, 1] (the input conversion's (float)g / 255)
-__device__ __forceinline__ float ldf(const uint8_t *p) { return (float)__ldg(p) / 255.0f; }
+// a uint8 gray value in [0, 1] (the input conversion's (float)g / 255): 0x1.010102p-8
+// is RN(1 / 255), and the quotient of all 256 values is the rounded one
+__device__ __forceinline__ float gray_unit(uint8_t g) { return div_rn((float)g, -255.0f, 0x1.010102p-8f); }
+__device__ __forceinline__ float ldf(const uint8_t *p) { return gray_unit(__ldg(p)); }
 
 // bilinearInterpolation(int,int,float,float,...), kernelUtils.h:298-303
 template <typename TImg>
