@@ -68,34 +68,38 @@ __device__ __forceinline__ void fx_accumulate(uint32_t *a, float v, int &bad) {
 }
 
 __device__ __forceinline__ double fx_to_double(const long long *L) {
-    unsigned __int128 Q = 0;
-#pragma unroll
-    for (int k = kFxLimbs - 1; k >= 0; k--) Q = (Q << 32) + (unsigned __int128)(__int128)L[k];
-    bool neg = (uint64_t)(Q >> 127) != 0;
-    unsigned __int128 U = neg ? (unsigned __int128)0 - Q : Q;
-    if (U == 0) return 0.0;
-    uint64_t hi = (uint64_t)(U >> 64), lo = (uint64_t)U;
-    int n = hi ? 127 - __clzll((long long)hi) : 63 - __clzll((long long)lo);
-    uint64_t mant;
-    int e2;
-    if (n <= 52) {
-        mant = (uint64_t)U << (52 - n);
-        e2 = -64 - (52 - n);
-    } else {
-        int sh = n - 52;
-        mant = (uint64_t)(U >> sh);
-        unsigned __int128 rem = U - ((unsigned __int128)mant << sh);
-        unsigned __int128 half = (unsigned __int128)1 << (sh - 1);
-        if (rem > half || (rem == half && (mant & 1))) mant++;
-        if (mant >> 53) {
-            mant >>= 1;
-            sh++;
-        }
-        e2 = sh - 64;
+    // the sum modulo 2^128, limb by limb, and its magnitude
+    static_assert(kFxLimbs == 4, "a 128-bit sum");
+    long long c = L[0];
+    unsigned long long lo = (uint32_t)c;
+    c = (c >> 32) + L[1];
+    lo |= (unsigned long long)c << 32;
+    c = (c >> 32) + L[2];
+    unsigned long long hi = (uint32_t)c;
+    c = (c >> 32) + L[3];
+    hi |= (unsigned long long)c << 32;
+    unsigned long long sign = hi & (1ull << 63);
+    if (sign) {
+        lo = 0ull - lo;
+        hi = ~hi + (lo == 0);
     }
-    uint64_t out = ((uint64_t)(e2 + 52 + 1023) << 52) | (mant & ((1ull << 52) - 1));
-    if (neg) out |= 1ull << 63;
-    return __longlong_as_double((long long)out);
+    if ((hi | lo) == 0) return 0.0;
+    // its first one to the top bit; 53 bits are the mantissa, the others round it
+    int lead = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo), s = lead & 63;
+    if (lead >= 64) {
+        hi = lo;
+        lo = 0;
+    }
+    if (s) {
+        hi = hi << s | lo >> (64 - s);
+        lo <<= s;
+    }
+    unsigned long long mant = hi >> 11;
+    uint32_t rest = (uint32_t)hi & 0x7ffu;
+    mant += rest > 0x400u || (rest == 0x400u && (lo != 0 || (mant & 1)));
+    // (a mantissa that rounding takes to 2^53 carries into the exponent)
+    return __longlong_as_double(
+        (long long)(sign | (((unsigned long long)(1023 + 63 - lead) << 52) + (mant - (1ull << 52)))));
 }
 
 }  // namespace rt
