@@ -33,7 +33,7 @@ constexpr int kWd[kLayers + 1] = {80, 40, 20, 10, 5, 3, 2};
 constexpr int kFeat = 128;
 constexpr int kOut = RECON_NET_OUT;
 
-constexpr int kpad(int cin) { return (9 * cin + 15) / 16 * 16; }
+__host__ __device__ constexpr int kpad(int cin) { return (9 * cin + 15) / 16 * 16; }
 
 struct Offsets {
     int64_t w[kLayers], b[kLayers], wfc, bfc, scale, total;
@@ -60,91 +60,116 @@ Offsets offsets() {
 
 __device__ __forceinline__ float bf(const __nv_bfloat16 *p) { return __bfloat162float(*p); }
 
+// 16 bytes from global to shared memory, zeros where `yes` is false
+__device__ __forceinline__ void copy16_or_zero(void *dst, const void *src, bool yes) {
+    unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(yes ? 16 : 0) : "memory");
+}
+
 // out[m][co] = relu(bias[co] + sum_k A[m][k] W[co][k]) with A the 3x3 / stride 2
-// / pad 1 patches of `in` (k = tap * Cin + c).  One CTA of 16 warps per 16
+// / pad 1 patches of `in` (k = tap * Cin + c).  One CTA of 16 warps per 16 MT
 // output pixels and K split (blockIdx.y of gridDim.y): the split covers a
 // contiguous range of 16-wide K steps, warp w takes output-channel group
-// w % NG and the steps j0 + w / NG, + KS, ...; the KS partial tiles are added in
-// ascending order in shared memory.  With one split the CTA adds the bias,
-// applies the ReLU and stores BF16; with several it stores its FP32 tile to
-// `partial` and k_conv_split_finish adds the splits in ascending order.  Every
-// order is fixed, so the result does not depend on scheduling.
+// w % NG and the steps j0 + w / NG, + KS, ... of all the CTA's pixels; the KS
+// partial tiles are added in ascending order in shared memory.  With one split
+// the CTA adds the bias, applies the ReLU and stores BF16; with several it stores
+// its FP32 tile to `partial` and k_conv_split_finish adds the splits in ascending
+// order.  Every order is fixed, so the result does not depend on scheduling, nor
+// on MT.
+//
+// The CTA copies its pixels' patches into shared memory once (16 bytes a copy,
+// rows padded so that ldmatrix meets no bank twice); reading them as fragments
+// from global memory took every warp of the NG through the same 4-byte loads
+// and their index arithmetic (a batch of 256: 32 to 64 channels at 8x10 72 -> 14 us,
+// 64 to 64 at 4x5 50 -> 14).  MT is as large as 38 KB of patches allow where that
+// still leaves a CTA per SM: the weights' fragments then serve MT tiles.
 constexpr int kConvWarps = 16;
+constexpr int conv_tiles(int cin) { return cin >= 128 ? 1 : cin >= 64 ? 2 : 4; }
 
-template <int COUT>
-__global__ void __launch_bounds__(kConvWarps * 32) k_conv_fwd(const __nv_bfloat16 *in, int N, int H, int W, int Cin,
-                                                              int Kp, const __nv_bfloat16 *w, const float *bias,
+template <int COUT, int CIN, int MT>
+__global__ void __launch_bounds__(kConvWarps * 32) k_conv_fwd(const __nv_bfloat16 *in, int N, int H, int W,
+                                                              const __nv_bfloat16 *w, const float *bias,
                                                               __nv_bfloat16 *out, int Ho, int Wo, float *partial) {
     constexpr int NF = COUT / 8;             // 8-column fragments
     constexpr int NG = NF < 8 ? NF : 8;      // warps across the columns
     constexpr int FPW = NF / NG;             // fragments per warp
     constexpr int KS = kConvWarps / NG;      // warps across K
-    __shared__ float red[KS][16][COUT];
+    constexpr int K = 9 * CIN, R = 16 * MT, LD = 2 * K + 16;  // LD: bytes per row of patches
+    static_assert(CIN % 16 == 0, "a 16-wide K step lies in one tap");
+    constexpr int kBytes = R * LD > KS * R * COUT * 4 ? R * LD : KS * R * COUT * 4;
+    __shared__ alignas(16) unsigned char mem[kBytes];  // the patches, then the partial tiles
+    __shared__ int s_n[R], s_y[R], s_x[R];
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int ng = warp % NG, ks = warp / NG;
     long long M = (long long)N * Ho * Wo;
-    long long m0 = (long long)blockIdx.x * 16;
+    long long m0 = (long long)blockIdx.x * R;
     int g = lane >> 2, tig = lane & 3;
-    long long rr[2] = {m0 + g, m0 + g + 8};
-    bool rv[2];
-    int rn[2], ry[2], rx[2];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        rv[h] = rr[h] < M;
-        long long mm = rv[h] ? rr[h] : 0;
-        rx[h] = (int)(mm % Wo);
-        ry[h] = (int)((mm / Wo) % Ho);
-        rn[h] = (int)(mm / ((long long)Wo * Ho));
-    }
-    float acc[FPW][4];
-#pragma unroll
-    for (int f = 0; f < FPW; f++) acc[f][0] = acc[f][1] = acc[f][2] = acc[f][3] = 0.0f;
-    int K = 9 * Cin, nk = Kp / 16;
+    constexpr int nk = K / 16;
     int S = gridDim.y, per = (nk + S - 1) / S;
     int j0 = blockIdx.y * per, j1 = min(nk, j0 + per);
-#pragma unroll 2
-    for (int j = j0 + ks; j < j1; j += KS) {
-        int kb = 16 * j;
-        // A fragment: a0 (row g, k 2t..2t+1), a1 (row g+8), a2 (row g, k+8), a3 (row g+8, k+8)
-        uint32_t a[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            int h = q & 1;
-            int k = kb + 2 * tig + ((q >> 1) ? 8 : 0);
-            uint32_t v = 0;
-            if (rv[h] && k < K) {
-                int tap = k / Cin, c = k - tap * Cin;
-                int ky = tap / 3, kx = tap - ky * 3;
-                int iy = 2 * ry[h] - 1 + ky, ix = 2 * rx[h] - 1 + kx;
-                if (iy >= 0 && iy < H && ix >= 0 && ix < W)
-                    v = *reinterpret_cast<const uint32_t *>(in + (((long long)rn[h] * H + iy) * W + ix) * Cin + c);
-            }
-            a[q] = v;
-        }
-#pragma unroll
-        for (int f = 0; f < FPW; f++) {
-            // B fragment: b0 (k 2t..2t+1, n g), b1 (k + 8)
-            const __nv_bfloat16 *wr = w + (long long)((ng * FPW + f) * 8 + g) * Kp + kb + 2 * tig;
-            uint32_t b0 = *reinterpret_cast<const uint32_t *>(wr);
-            uint32_t b1 = *reinterpret_cast<const uint32_t *>(wr + 8);
-            asm volatile(
-                "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-                "{%0,%1,%2,%3};\n"
-                : "+f"(acc[f][0]), "+f"(acc[f][1]), "+f"(acc[f][2]), "+f"(acc[f][3])
-                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-        }
-    }
-    // C fragment: c0 c1 (row g, cols 2t, 2t+1), c2 c3 (row g+8)
-#pragma unroll
-    for (int f = 0; f < FPW; f++) {
-        int col = (ng * FPW + f) * 8 + 2 * tig;
-        red[ks][g][col] = acc[f][0];
-        red[ks][g][col + 1] = acc[f][1];
-        red[ks][g + 8][col] = acc[f][2];
-        red[ks][g + 8][col + 1] = acc[f][3];
+    if (threadIdx.x < R) {
+        long long m = m0 + threadIdx.x;
+        s_n[threadIdx.x] = m < M ? (int)(m / ((long long)Wo * Ho)) : -1;
+        s_y[threadIdx.x] = 2 * (int)((m / Wo) % Ho) - 1;
+        s_x[threadIdx.x] = 2 * (int)(m % Wo) - 1;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < 16 * COUT / 2; e += blockDim.x) {
+    int per_row = 2 * (j1 - j0);
+    for (int e = threadIdx.x; e < R * per_row; e += kConvWarps * 32) {
+        int row = e / per_row, k8 = e - row * per_row, k = 16 * j0 + 8 * k8;
+        int tap = k / CIN, c = k % CIN, ky = tap / 3, kx = tap - 3 * ky;
+        int n = s_n[row], iy = s_y[row] + ky, ix = s_x[row] + kx;
+        bool yes = n >= 0 && iy >= 0 && iy < H && ix >= 0 && ix < W;
+        copy16_or_zero(mem + row * LD + 16 * k8, in + (yes ? (((long long)n * H + iy) * W + ix) * CIN + c : 0), yes);
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    float acc[MT][FPW][4];
+#pragma unroll
+    for (int t = 0; t < MT; t++)
+#pragma unroll
+        for (int f = 0; f < FPW; f++) acc[t][f][0] = acc[t][f][1] = acc[t][f][2] = acc[t][f][3] = 0.0f;
+    const __nv_bfloat16 *wr = w + (long long)(ng * FPW * 8 + g) * K + 2 * tig;
+    // ldmatrix: lane l gives the address of row l % 16, columns 8 (l / 16) ..
+    unsigned pa = (unsigned)__cvta_generic_to_shared(mem) + (lane & 15) * LD + (lane >> 4) * 16;
+#pragma unroll 4
+    for (int j = j0 + ks; j < j1; j += KS) {
+        // B fragments: b0 (k 2t..2t+1, n g), b1 (k + 8)
+        uint32_t b[FPW][2];
+#pragma unroll
+        for (int f = 0; f < FPW; f++) {
+            b[f][0] = __ldg(reinterpret_cast<const unsigned *>(wr + f * 8 * K + 16 * j));
+            b[f][1] = __ldg(reinterpret_cast<const unsigned *>(wr + f * 8 * K + 16 * j + 8));
+        }
+#pragma unroll
+        for (int t = 0; t < MT; t++) {
+            // A fragment: a0 (row g, k 2t..2t+1), a1 (row g+8), a2 (row g, k+8), a3 (row g+8, k+8)
+            uint32_t a[4];
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                         : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
+                         : "r"(pa + t * 16 * LD + (j - j0) * 32));
+#pragma unroll
+            for (int f = 0; f < FPW; f++)
+                asm volatile(
+                    "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                    "{%0,%1,%2,%3};\n"
+                    : "+f"(acc[t][f][0]), "+f"(acc[t][f][1]), "+f"(acc[t][f][2]), "+f"(acc[t][f][3])
+                    : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[f][0]), "r"(b[f][1]));
+        }
+    }
+    __syncthreads();  // the patches are consumed
+    float(*red)[R][COUT] = reinterpret_cast<float(*)[R][COUT]>(mem);
+    // C fragment: c0 c1 (row g, cols 2t, 2t+1), c2 c3 (row g+8)
+#pragma unroll
+    for (int t = 0; t < MT; t++)
+#pragma unroll
+        for (int f = 0; f < FPW; f++) {
+            int col = (ng * FPW + f) * 8 + 2 * tig;
+            *reinterpret_cast<float2 *>(&red[ks][16 * t + g][col]) = make_float2(acc[t][f][0], acc[t][f][1]);
+            *reinterpret_cast<float2 *>(&red[ks][16 * t + g + 8][col]) = make_float2(acc[t][f][2], acc[t][f][3]);
+        }
+    __syncthreads();
+    for (int e = threadIdx.x; e < R * COUT / 2; e += blockDim.x) {
         int row = e / (COUT / 2), col = 2 * (e % (COUT / 2));
         long long m = m0 + row;
         if (m >= M) continue;
@@ -174,12 +199,11 @@ __global__ void __launch_bounds__(kConvWarps * 32) k_conv_fwd(const __nv_bfloat1
 // no partial tiles are added.  8 warps (128 pixels) per CTA.
 constexpr int kConvPxWarps = 8;
 
-template <int COUT>
+template <int COUT, int CIN>
 __global__ void __launch_bounds__(kConvPxWarps * 32) k_conv_fwd_px(const __nv_bfloat16 *in, int N, int H, int W,
-                                                                   int Cin, int Kp, const __nv_bfloat16 *w,
-                                                                   const float *bias, __nv_bfloat16 *out, int Ho,
-                                                                   int Wo) {
-    constexpr int NF = COUT / 8;
+                                                                   const __nv_bfloat16 *w, const float *bias,
+                                                                   __nv_bfloat16 *out, int Ho, int Wo) {
+    constexpr int NF = COUT / 8, K = 9 * CIN, Kp = kpad(CIN), nk = Kp / 16;
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     long long M = (long long)N * Ho * Wo;
     long long m0 = ((long long)blockIdx.x * kConvPxWarps + warp) * 16;
@@ -199,7 +223,11 @@ __global__ void __launch_bounds__(kConvPxWarps * 32) k_conv_fwd_px(const __nv_bf
     float acc[NF][4];
 #pragma unroll
     for (int f = 0; f < NF; f++) acc[f][0] = acc[f][1] = acc[f][2] = acc[f][3] = 0.0f;
-    int K = 9 * Cin, nk = Kp / 16;
+    const __nv_bfloat16 *patch[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+        patch[h] = in + (((long long)rn[h] * H + 2 * ry[h] - 1) * W + 2 * rx[h] - 1) * CIN;
+#pragma unroll(nk < 4 ? nk : 3)
     for (int j = 0; j < nk; j++) {
         int kb = 16 * j;
         uint32_t a[4];
@@ -209,19 +237,19 @@ __global__ void __launch_bounds__(kConvPxWarps * 32) k_conv_fwd_px(const __nv_bf
             int k = kb + 2 * tig + ((q >> 1) ? 8 : 0);
             uint32_t v = 0;
             if (rv[h] && k < K) {
-                int tap = k / Cin, c = k - tap * Cin;
+                int tap = k / CIN, c = k % CIN;
                 int ky = tap / 3, kx = tap - ky * 3;
                 int iy = 2 * ry[h] - 1 + ky, ix = 2 * rx[h] - 1 + kx;
                 if (iy >= 0 && iy < H && ix >= 0 && ix < W)
-                    v = *reinterpret_cast<const uint32_t *>(in + (((long long)rn[h] * H + iy) * W + ix) * Cin + c);
+                    v = __ldg(reinterpret_cast<const unsigned *>(patch[h] + (ky * W + kx) * CIN + c));
             }
             a[q] = v;
         }
 #pragma unroll
         for (int f = 0; f < NF; f++) {
             const __nv_bfloat16 *wr = w + (long long)(f * 8 + g) * Kp + kb + 2 * tig;
-            uint32_t b0 = *reinterpret_cast<const uint32_t *>(wr);
-            uint32_t b1 = *reinterpret_cast<const uint32_t *>(wr + 8);
+            uint32_t b0 = __ldg(reinterpret_cast<const unsigned *>(wr));
+            uint32_t b1 = __ldg(reinterpret_cast<const unsigned *>(wr + 8));
             asm volatile(
                 "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
                 "{%0,%1,%2,%3};\n"
@@ -307,6 +335,7 @@ __global__ void k_head_grad(const float *y, const float *t, const float *feat, i
             sdy[e] = d * inv;
         }
         __syncthreads();
+#pragma unroll 16
         for (int n = 0; n < cnt; n++) {
             float dy = sdy[n * kOut + j];
             s += dy * feat[(long long)(n0 + n) * kFeat + c];
@@ -367,33 +396,44 @@ __device__ __forceinline__ void mma_bf16(float *c, const uint32_t *a, uint32_t b
 // Split s covers pixels [s per, (s + 1) per).  Writes partial[e][s] for the
 // entries e = co (Kp + 1) + k, k < Kp, and, from CTA column 0, the bias
 // gradient at k = Kp: the split's FP32 sum of dz (each thread adds its pixel
-// pairs in order, the threads of a co are then added in thread order).
+// pairs in order, the threads of a co are then added in thread order).  It is
+// bound by staging the patches: with a tap's bit and an offset per pixel and
+// column instead of the whole index arithmetic per element, and four channels a
+// load, the six layers of a batch of 256 take 166 us against 274.
+// four channels: the network's own activations are aligned to 8 bytes, the
+// caller's input (the layer of 4 channels) to 4
+template <int CIN> __device__ __forceinline__ uint2 load4(const __nv_bfloat16 *p) {
+    if constexpr (CIN > 4) return __ldg(reinterpret_cast<const uint2 *>(p));
+    const unsigned *q = reinterpret_cast<const unsigned *>(p);
+    return make_uint2(__ldg(q), __ldg(q + 1));
+}
+
 constexpr int kWgKT = 64, kWgMS = 64, kWgThreads = 128;
-template <int COUT>
+// where row k's words of the staged patches lie: their index with these bits
+// turned, alike for the 8 rows of a fragment (the stores of 16 rows' words then
+// share a bank 4 times instead of 8)
+__device__ __forceinline__ constexpr int wg_swizzle(int k) { return 8 * ((k >> 3) & 3); }
+template <int COUT, int CIN>
 __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad_tc(const float *dz, const __nv_bfloat16 *in, int N,
-                                                              int H, int W, int Cin, int Kp, int Ho, int Wo,
-                                                              int nsplit, int per, float *partial) {
+                                                              int H, int W, int Ho, int Wo, int nsplit, int per,
+                                                              float *partial) {
+    constexpr int K = 9 * CIN, Kp = kpad(CIN);
     constexpr int RT = COUT / 16, FPW = RT * 2;  // 8 column fragments per row tile, over 4 warps
     constexpr int LD = kWgMS / 2 + 4;            // words per staged row
     constexpr int TPC = kWgThreads / COUT;       // threads per co in the staging of dz
     static_assert(kWgThreads % COUT == 0 && RT * 8 == 4 * FPW, "tile split");
     __shared__ uint32_t sD[COUT][LD];
     __shared__ uint32_t sX[kWgKT][LD];
-    __shared__ int s_n[kWgMS], s_oy[kWgMS], s_ox[kWgMS];
-    __shared__ int s_c[kWgKT], s_ky[kWgKT], s_kx[kWgKT];
+    __shared__ long long s_at[kWgMS];  // a pixel's patch: its first element, and a bit per tap
+    __shared__ unsigned s_taps[kWgMS]; // that lies inside the image
     __shared__ float s_bias[kWgThreads];
-    const uint16_t *inb = reinterpret_cast<const uint16_t *>(in);
     int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    int K = 9 * Cin, kb = blockIdx.x * kWgKT, s = blockIdx.y;
+    int kb = blockIdx.x * kWgKT, s = blockIdx.y;
     long long M = (long long)N * Ho * Wo;
     long long mb = (long long)per * s, me = mb + per < M ? mb + per : M;
-    if (tid < kWgKT) {
-        int k = kb + tid;
-        int tap = k / Cin;
-        s_c[tid] = k < K ? k - tap * Cin : -1;
-        s_ky[tid] = tap / 3;
-        s_kx[tid] = tap - (tap / 3) * 3;
-    }
+    // the thread's four columns of the patches (k = kb + 4 (tid % 16) ..; one tap, since Cin is a multiple of 4)
+    int kq = tid & 15, k = kb + 4 * kq, tap = k / CIN, koff = ((tap / 3) * W + tap % 3) * CIN + k % CIN;
+    unsigned tap_bit = k < K ? 1u << tap : 0u;
     float acc[FPW][4];
 #pragma unroll
     for (int q = 0; q < FPW; q++) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.0f;
@@ -402,12 +442,15 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad_tc(const float *dz, c
         __syncthreads();  // the previous stage is consumed
         if (tid < kWgMS) {
             long long m = m0 + tid;
-            s_n[tid] = -1;
-            if (m < me) {
-                s_ox[tid] = (int)(m % Wo);
-                s_oy[tid] = (int)((m / Wo) % Ho);
-                s_n[tid] = (int)(m / ((long long)Wo * Ho));
-            }
+            int oy = (int)((m / Wo) % Ho), ox = (int)(m % Wo), n = (int)(m / ((long long)Wo * Ho));
+            unsigned taps = 0;
+            if (m < me)
+                for (int q = 0; q < 9; q++) {
+                    int iy = 2 * oy - 1 + q / 3, ix = 2 * ox - 1 + q % 3;
+                    if (iy >= 0 && iy < H && ix >= 0 && ix < W) taps |= 1u << q;
+                }
+            s_taps[tid] = taps;
+            s_at[tid] = (((long long)n * H + 2 * oy - 1) * W + 2 * ox - 1) * CIN;
         }
         // dz^T: thread tid always stages co = tid % COUT
         for (int e = tid; e < COUT * (kWgMS / 2); e += kWgThreads) {
@@ -420,21 +463,17 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad_tc(const float *dz, c
             sD[co][mp] = pack_bf16(v0, v1);
         }
         __syncthreads();  // the pixel decode is visible
-        for (int e = tid; e < kWgKT * (kWgMS / 2); e += kWgThreads) {
-            int kk = e % kWgKT, mp = e / kWgKT;
-            int c = s_c[kk];
-            uint32_t word = 0;
-            if (c >= 0) {
+        // X^T: four channels (8 bytes) of two pixels at a time
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    int i = 2 * mp + h, n = s_n[i];
-                    if (n < 0) continue;
-                    int iy = 2 * s_oy[i] - 1 + s_ky[kk], ix = 2 * s_ox[i] - 1 + s_kx[kk];
-                    if (iy >= 0 && iy < H && ix >= 0 && ix < W)
-                        word |= (uint32_t)inb[(((long long)n * H + iy) * W + ix) * Cin + c] << (16 * h);
-                }
-            }
-            sX[kk][mp] = word;
+        for (int mp = tid >> 4; mp < kWgMS / 2; mp += kWgThreads / 16) {
+            uint2 p0 = make_uint2(0u, 0u), p1 = make_uint2(0u, 0u);
+            if (s_taps[2 * mp] & tap_bit) p0 = load4<CIN>(in + s_at[2 * mp] + koff);
+            if (s_taps[2 * mp + 1] & tap_bit) p1 = load4<CIN>(in + s_at[2 * mp + 1] + koff);
+            int at = mp ^ wg_swizzle(4 * kq);
+            sX[4 * kq][at] = __byte_perm(p0.x, p1.x, 0x5410);
+            sX[4 * kq + 1][at] = __byte_perm(p0.x, p1.x, 0x7632);
+            sX[4 * kq + 2][at] = __byte_perm(p0.y, p1.y, 0x5410);
+            sX[4 * kq + 3][at] = __byte_perm(p0.y, p1.y, 0x7632);
         }
         __syncthreads();
 #pragma unroll
@@ -444,7 +483,8 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad_tc(const float *dz, c
                 int qq = warp * FPW + q, r = qq / 8, f = qq % 8;
                 uint32_t a[4] = {sD[16 * r + g][ks * 8 + t], sD[16 * r + g + 8][ks * 8 + t],
                                  sD[16 * r + g][ks * 8 + t + 4], sD[16 * r + g + 8][ks * 8 + t + 4]};
-                mma_bf16(acc[q], a, sX[8 * f + g][ks * 8 + t], sX[8 * f + g][ks * 8 + t + 4]);
+                int sw = wg_swizzle(8 * f);
+                mma_bf16(acc[q], a, sX[8 * f + g][(ks * 8 + t) ^ sw], sX[8 * f + g][(ks * 8 + t + 4) ^ sw]);
             }
         }
     }
@@ -452,13 +492,13 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad_tc(const float *dz, c
 #pragma unroll
     for (int q = 0; q < FPW; q++) {
         int qq = warp * FPW + q, r = qq / 8, f = qq % 8;
-        int k = kb + 8 * f + 2 * t;
+        int kc = kb + 8 * f + 2 * t;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             int co = 16 * r + g + 8 * h;
-            long long e = (long long)co * row + k;
-            if (k < Kp) partial[e * nsplit + s] = acc[q][2 * h];
-            if (k + 1 < Kp) partial[(e + 1) * nsplit + s] = acc[q][2 * h + 1];
+            long long e = (long long)co * row + kc;
+            if (kc < Kp) partial[e * nsplit + s] = acc[q][2 * h];
+            if (kc + 1 < Kp) partial[(e + 1) * nsplit + s] = acc[q][2 * h + 1];
         }
     }
     if (blockIdx.x == 0) {
@@ -514,10 +554,10 @@ __global__ void k_wgrad_reduce(const float *partial, int nsplit, int Cout, int K
 // reduced by KS warps (warp group kg takes the co steps kg, kg + KS, ... of
 // every tap), whose tiles are then added in group order (the deep layers
 // have few rows and long reductions).
-template <int CIN, int KS>
+template <int CIN, int Cout, int KS>
 __global__ void __launch_bounds__(128) k_conv_dgrad_tc(const float *dz, const __nv_bfloat16 *wt,
-                                                       const __nv_bfloat16 *a_prev, int N, int H, int W, int Cout,
-                                                       int Ho, int Wo, float *dz_prev) {
+                                                       const __nv_bfloat16 *a_prev, int N, int H, int W, int Ho, int Wo,
+                                                       float *dz_prev) {
     constexpr int NF = CIN / 8;
     static_assert(KS == 1 || KS == 2 || KS == 4, "4 warps per CTA");
     __shared__ float red[KS > 1 ? 4 : 1][KS > 1 ? 16 : 1][KS > 1 ? CIN : 1];
@@ -565,12 +605,13 @@ __global__ void __launch_bounds__(128) k_conv_dgrad_tc(const float *dz, const __
         }
         if (!__any_sync(0xffffffffu, v[0] || v[1])) continue;
         const uint32_t *wtap = reinterpret_cast<const uint32_t *>(wt + (long long)tap * CIN * Cout);
+#pragma unroll 2
         for (int co0 = 16 * kg; co0 < Cout; co0 += 16 * KS) {
             uint32_t a[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 int h = q & 1, col = co0 + 2 * t + ((q >> 1) ? 8 : 0);
-                float2 d = v[h] ? *reinterpret_cast<const float2 *>(dz + o[h] + col) : make_float2(0.0f, 0.0f);
+                float2 d = v[h] ? __ldg(reinterpret_cast<const float2 *>(dz + o[h] + col)) : make_float2(0.0f, 0.0f);
                 a[q] = pack_bf16(d.x, d.y);
             }
 #pragma unroll
@@ -762,38 +803,76 @@ bool pixel_parallel(int l, int n) {
     return kpad(kCin[l]) / 16 < KS || tiles >= 4096;
 }
 
-template <int COUT>
-void conv_launch(recon_initnet *net, int l, const __nv_bfloat16 *in, int n) {
-    int Cin = kCin[l], Kp = kpad(Cin);
-    long long M = (long long)n * kHt[l + 1] * kWd[l + 1];
-    if (pixel_parallel(l, n)) {
-        long long tiles = (M + 15) / 16;
-        k_conv_fwd_px<COUT><<<(unsigned)((tiles + kConvPxWarps - 1) / kConvPxWarps), kConvPxWarps * 32, 0,
-                               net->stream>>>(in, n, kHt[l], kWd[l], Cin, Kp, net->pbf + net->off.w[l],
-                                              net->params + net->off.b[l], net->act[l], kHt[l + 1], kWd[l + 1]);
-        return;
+template <int L, int MT>
+void conv_tiled(recon_initnet *net, const __nv_bfloat16 *in, int n, long long M, int S) {
+    k_conv_fwd<kCout[L], kCin[L], MT><<<dim3((unsigned)((M + 16 * MT - 1) / (16 * MT)), (unsigned)S), kConvWarps * 32, 0,
+                                        net->stream>>>(in, n, kHt[L], kWd[L], net->pbf + net->off.w[L],
+                                                       net->params + net->off.b[L], net->act[L], kHt[L + 1], kWd[L + 1],
+                                                       net->fpart);
+}
+
+template <int L>
+void conv_launch(recon_initnet *net, const __nv_bfloat16 *in, int n) {
+    constexpr int COUT = kCout[L], CIN = kCin[L];
+    long long M = (long long)n * kHt[L + 1] * kWd[L + 1];
+    const float *b = net->params + net->off.b[L];
+    if constexpr (CIN % 16 == 0) {
+        if (!pixel_parallel(L, n)) {
+            int S = fsplit_for(L, n);
+            constexpr int MT = conv_tiles(CIN);
+            // several tiles per CTA as long as every SM has one
+            if (M >= 16LL * MT * 152) conv_tiled<L, MT>(net, in, n, M, S);
+            else conv_tiled<L, 1>(net, in, n, M, S);
+            if (S > 1) {
+                long long pairs = M * (COUT / 2);
+                k_conv_split_finish<COUT><<<(unsigned)((pairs + 255) / 256), 256, 0, net->stream>>>(net->fpart, S, M, b,
+                                                                                                   net->act[L]);
+            }
+            return;
+        }
     }
-    int S = fsplit_for(l, n);
-    dim3 grid((unsigned)((M + 15) / 16), (unsigned)S);
-    const __nv_bfloat16 *w = net->pbf + net->off.w[l];
-    const float *b = net->params + net->off.b[l];
-    k_conv_fwd<COUT><<<grid, kConvWarps * 32, 0, net->stream>>>(in, n, kHt[l], kWd[l], Cin, Kp, w, b, net->act[l],
-                                                                kHt[l + 1], kWd[l + 1], net->fpart);
-    if (S > 1) {
-        long long pairs = M * (COUT / 2);
-        k_conv_split_finish<COUT><<<(unsigned)((pairs + 255) / 256), 256, 0, net->stream>>>(net->fpart, S, M, b,
-                                                                                           net->act[l]);
-    }
+    long long tiles = (M + 15) / 16;
+    k_conv_fwd_px<COUT, CIN><<<(unsigned)((tiles + kConvPxWarps - 1) / kConvPxWarps), kConvPxWarps * 32, 0, net->stream>>>(
+        in, n, kHt[L], kWd[L], net->pbf + net->off.w[L], b, net->act[L], kHt[L + 1], kWd[L + 1]);
 }
 
 int conv_forward(recon_initnet *net, int l, const __nv_bfloat16 *in, int n) {
-    switch (kCout[l]) {
-        case 16: conv_launch<16>(net, l, in, n); break;
-        case 32: conv_launch<32>(net, l, in, n); break;
-        case 64: conv_launch<64>(net, l, in, n); break;
-        default: conv_launch<128>(net, l, in, n); break;
+    switch (l) {
+        case 0: conv_launch<0>(net, in, n); break;
+        case 1: conv_launch<1>(net, in, n); break;
+        case 2: conv_launch<2>(net, in, n); break;
+        case 3: conv_launch<3>(net, in, n); break;
+        case 4: conv_launch<4>(net, in, n); break;
+        default: conv_launch<5>(net, in, n); break;
     }
     return RECON_OK;
+}
+
+// the weight gradient's partial sums, and for l > 0 the input gradient
+template <int L>
+void wgrad_launch(recon_initnet *net, const __nv_bfloat16 *in, int n, int ns, int per) {
+    dim3 grid((kpad(kCin[L]) + kWgKT - 1) / kWgKT, ns);
+    k_conv_wgrad_tc<kCout[L], kCin[L]><<<grid, kWgThreads, 0, net->stream>>>(net->dz[L], in, n, kHt[L], kWd[L], kHt[L + 1],
+                                                                             kWd[L + 1], ns, per, net->partial);
+}
+template <int L, int KS>
+void dgrad_tiled(recon_initnet *net, int n, long long tiles) {
+    k_conv_dgrad_tc<kCin[L], kCout[L], KS><<<(unsigned)((tiles + 4 / KS - 1) / (4 / KS)), 128, 0, net->stream>>>(
+        net->dz[L], net->wt + net->wt_lay.dst[L], net->act[L - 1], n, kHt[L], kWd[L], kHt[L + 1], kWd[L + 1],
+        net->dz[L - 1]);
+}
+template <int L>
+void dgrad_launch(recon_initnet *net, int n) {
+    // rows of 16 per tile; the reduction split over 2 or 4 warps when the
+    // layer has fewer than 8 or 4 tiles per SM (and co steps to share)
+    long long tiles = ((long long)n * kHt[L] * kWd[L] + 15) / 16;
+    int ks = 1;
+    if (tiles < 8 * 152) ks = 2;
+    if (tiles < 4 * 152) ks = 4;
+    while (ks > 1 && kCout[L] / 16 < ks) ks >>= 1;
+    if (ks == 4) dgrad_tiled<L, 4>(net, n, tiles);
+    else if (ks == 2) dgrad_tiled<L, 2>(net, n, tiles);
+    else dgrad_tiled<L, 1>(net, n, tiles);
 }
 
 int forward(recon_initnet *net, const __nv_bfloat16 *in, int n) {
@@ -817,42 +896,27 @@ int backward(recon_initnet *net, const __nv_bfloat16 *in, const float *target, i
                                               net->dz[kLayers - 1]);
     for (int l = kLayers - 1; l >= 0; l--) {
         int Cin = kCin[l], Cout = kCout[l], Kp = kpad(Cin);
-        int H = kHt[l], W = kWd[l], Ho = kHt[l + 1], Wo = kWd[l + 1];
         const __nv_bfloat16 *lin = l ? net->act[l - 1] : in;
         int ns = nsplit_for(l, n), per = wg_per_split(l, n);
         int row = Kp + 1;
-        dim3 g1((Kp + kWgKT - 1) / kWgKT, ns);
-        switch (Cout) {
-            case 16: k_conv_wgrad_tc<16><<<g1, kWgThreads, 0, net->stream>>>(net->dz[l], lin, n, H, W, Cin, Kp, Ho, Wo, ns, per, net->partial); break;
-            case 32: k_conv_wgrad_tc<32><<<g1, kWgThreads, 0, net->stream>>>(net->dz[l], lin, n, H, W, Cin, Kp, Ho, Wo, ns, per, net->partial); break;
-            case 64: k_conv_wgrad_tc<64><<<g1, kWgThreads, 0, net->stream>>>(net->dz[l], lin, n, H, W, Cin, Kp, Ho, Wo, ns, per, net->partial); break;
-            default: k_conv_wgrad_tc<128><<<g1, kWgThreads, 0, net->stream>>>(net->dz[l], lin, n, H, W, Cin, Kp, Ho, Wo, ns, per, net->partial); break;
+        switch (l) {
+            case 0: wgrad_launch<0>(net, lin, n, ns, per); break;
+            case 1: wgrad_launch<1>(net, lin, n, ns, per); break;
+            case 2: wgrad_launch<2>(net, lin, n, ns, per); break;
+            case 3: wgrad_launch<3>(net, lin, n, ns, per); break;
+            case 4: wgrad_launch<4>(net, lin, n, ns, per); break;
+            default: wgrad_launch<5>(net, lin, n, ns, per); break;
         }
         long long red_threads = (long long)Cout * row * (ns <= 8 ? 1 : 32);
         k_wgrad_reduce<<<(unsigned)((red_threads + 127) / 128), 128, 0, net->stream>>>(
             net->partial, ns, Cout, Kp, grad + net->off.w[l], grad + net->off.b[l]);
-        if (l > 0) {
-            // rows of 16 per tile; the reduction split over 2 or 4 warps when the
-            // layer has fewer than 8 or 4 tiles per SM (and co steps to share)
-            long long rows = (long long)n * H * W, tiles = (rows + 15) / 16;
-            int ks = 1;
-            if (tiles < 8 * 152) ks = 2;
-            if (tiles < 4 * 152) ks = 4;
-            while (ks > 1 && Cout / 16 < ks) ks >>= 1;
-            unsigned blocks = (unsigned)((tiles + 4 / ks - 1) / (4 / ks));
-            const __nv_bfloat16 *wt = net->wt + net->wt_lay.dst[l];
-            const __nv_bfloat16 *ap = net->act[l - 1];
-            float *dp = net->dz[l - 1];
-#define RECON_DGRAD(CI, K) k_conv_dgrad_tc<CI, K><<<blocks, 128, 0, net->stream>>>(net->dz[l], wt, ap, n, H, W, Cout, Ho, Wo, dp)
-#define RECON_DGRAD_KS(CI) (ks == 4 ? RECON_DGRAD(CI, 4) : ks == 2 ? RECON_DGRAD(CI, 2) : RECON_DGRAD(CI, 1))
-            switch (Cin) {
-                case 16: RECON_DGRAD_KS(16); break;
-                case 32: RECON_DGRAD_KS(32); break;
-                case 64: RECON_DGRAD_KS(64); break;
-                default: RECON_DGRAD_KS(128); break;
-            }
-#undef RECON_DGRAD_KS
-#undef RECON_DGRAD
+        switch (l) {
+            case 0: break;
+            case 1: dgrad_launch<1>(net, n); break;
+            case 2: dgrad_launch<2>(net, n); break;
+            case 3: dgrad_launch<3>(net, n); break;
+            case 4: dgrad_launch<4>(net, n); break;
+            default: dgrad_launch<5>(net, n); break;
         }
     }
     NCK(cudaMemsetAsync(grad + net->off.scale, 0, kOut * sizeof(float), net->stream));
