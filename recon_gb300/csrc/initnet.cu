@@ -25,6 +25,8 @@ void set_last_error(const char *msg);
 
 namespace nn {
 
+// Pixel numbers of a layer fit 32 bits: 2^32 of them would take more memory than the device has.
+
 constexpr int kLayers = 6;
 constexpr int kCin[kLayers] = {4, 16, 32, 64, 64, 128};
 constexpr int kCout[kLayers] = {16, 32, 64, 64, 128, 128};
@@ -86,10 +88,10 @@ __device__ __forceinline__ void copy16_or_zero(void *dst, const void *src, bool 
 constexpr int kConvWarps = 16;
 constexpr int conv_tiles(int cin) { return cin >= 128 ? 1 : cin >= 64 ? 2 : 4; }
 
-template <int COUT, int CIN, int MT>
-__global__ void __launch_bounds__(kConvWarps * 32) k_conv_fwd(const __nv_bfloat16 *in, int N, int H, int W,
-                                                              const __nv_bfloat16 *w, const float *bias,
-                                                              __nv_bfloat16 *out, int Ho, int Wo, float *partial) {
+template <int L, int MT>
+__global__ void __launch_bounds__(kConvWarps * 32) k_conv_fwd(const __nv_bfloat16 *in, int N, const __nv_bfloat16 *w,
+                                                              const float *bias, __nv_bfloat16 *out, float *partial) {
+    constexpr int COUT = kCout[L], CIN = kCin[L], H = kHt[L], W = kWd[L], Ho = kHt[L + 1], Wo = kWd[L + 1];
     constexpr int NF = COUT / 8;             // 8-column fragments
     constexpr int NG = NF < 8 ? NF : 8;      // warps across the columns
     constexpr int FPW = NF / NG;             // fragments per warp
@@ -108,9 +110,9 @@ __global__ void __launch_bounds__(kConvWarps * 32) k_conv_fwd(const __nv_bfloat1
     int S = gridDim.y, per = (nk + S - 1) / S;
     int j0 = blockIdx.y * per, j1 = min(nk, j0 + per);
     if (threadIdx.x < R) {
-        long long m = m0 + threadIdx.x;
-        s_n[threadIdx.x] = m < M ? (int)(m / ((long long)Wo * Ho)) : -1;
-        s_y[threadIdx.x] = 2 * (int)((m / Wo) % Ho) - 1;
+        unsigned m = (unsigned)m0 + threadIdx.x;
+        s_n[threadIdx.x] = m < M ? (int)(m / (Wo * Ho)) : -1;
+        s_y[threadIdx.x] = 2 * (int)(m / Wo % Ho) - 1;
         s_x[threadIdx.x] = 2 * (int)(m % Wo) - 1;
     }
     __syncthreads();
@@ -129,18 +131,15 @@ __global__ void __launch_bounds__(kConvWarps * 32) k_conv_fwd(const __nv_bfloat1
     for (int t = 0; t < MT; t++)
 #pragma unroll
         for (int f = 0; f < FPW; f++) acc[t][f][0] = acc[t][f][1] = acc[t][f][2] = acc[t][f][3] = 0.0f;
-    const __nv_bfloat16 *wr = w + (long long)(ng * FPW * 8 + g) * K + 2 * tig;
+    const uint2 *wf = reinterpret_cast<const uint2 *>(w) + ng * FPW * 32 + lane;
     // ldmatrix: lane l gives the address of row l % 16, columns 8 (l / 16) ..
     unsigned pa = (unsigned)__cvta_generic_to_shared(mem) + (lane & 15) * LD + (lane >> 4) * 16;
 #pragma unroll 4
     for (int j = j0 + ks; j < j1; j += KS) {
         // B fragments: b0 (k 2t..2t+1, n g), b1 (k + 8)
-        uint32_t b[FPW][2];
+        uint2 b[FPW];
 #pragma unroll
-        for (int f = 0; f < FPW; f++) {
-            b[f][0] = __ldg(reinterpret_cast<const unsigned *>(wr + f * 8 * K + 16 * j));
-            b[f][1] = __ldg(reinterpret_cast<const unsigned *>(wr + f * 8 * K + 16 * j + 8));
-        }
+        for (int f = 0; f < FPW; f++) b[f] = __ldg(wf + (j * NF + f) * 32);
 #pragma unroll
         for (int t = 0; t < MT; t++) {
             // A fragment: a0 (row g, k 2t..2t+1), a1 (row g+8), a2 (row g, k+8), a3 (row g+8, k+8)
@@ -154,7 +153,7 @@ __global__ void __launch_bounds__(kConvWarps * 32) k_conv_fwd(const __nv_bfloat1
                     "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
                     "{%0,%1,%2,%3};\n"
                     : "+f"(acc[t][f][0]), "+f"(acc[t][f][1]), "+f"(acc[t][f][2]), "+f"(acc[t][f][3])
-                    : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[f][0]), "r"(b[f][1]));
+                    : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[f].x), "r"(b[f].y));
         }
     }
     __syncthreads();  // the patches are consumed
@@ -199,11 +198,11 @@ __global__ void __launch_bounds__(kConvWarps * 32) k_conv_fwd(const __nv_bfloat1
 // no partial tiles are added.  8 warps (128 pixels) per CTA.
 constexpr int kConvPxWarps = 8;
 
-template <int COUT, int CIN>
-__global__ void __launch_bounds__(kConvPxWarps * 32) k_conv_fwd_px(const __nv_bfloat16 *in, int N, int H, int W,
-                                                                   const __nv_bfloat16 *w, const float *bias,
-                                                                   __nv_bfloat16 *out, int Ho, int Wo) {
-    constexpr int NF = COUT / 8, K = 9 * CIN, Kp = kpad(CIN), nk = Kp / 16;
+template <int L>
+__global__ void __launch_bounds__(kConvPxWarps * 32) k_conv_fwd_px(const __nv_bfloat16 *in, int N, const __nv_bfloat16 *w,
+                                                                   const float *bias, __nv_bfloat16 *out) {
+    constexpr int COUT = kCout[L], CIN = kCin[L], H = kHt[L], W = kWd[L], Ho = kHt[L + 1], Wo = kWd[L + 1];
+    constexpr int NF = COUT / 8, K = 9 * CIN, nk = kpad(CIN) / 16;
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     long long M = (long long)N * Ho * Wo;
     long long m0 = ((long long)blockIdx.x * kConvPxWarps + warp) * 16;
@@ -215,10 +214,10 @@ __global__ void __launch_bounds__(kConvPxWarps * 32) k_conv_fwd_px(const __nv_bf
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         rv[h] = rr[h] < M;
-        long long mm = rv[h] ? rr[h] : 0;
+        unsigned mm = rv[h] ? (unsigned)rr[h] : 0u;
         rx[h] = (int)(mm % Wo);
-        ry[h] = (int)((mm / Wo) % Ho);
-        rn[h] = (int)(mm / ((long long)Wo * Ho));
+        ry[h] = (int)(mm / Wo % Ho);
+        rn[h] = (int)(mm / (Wo * Ho));
     }
     float acc[NF][4];
 #pragma unroll
@@ -247,14 +246,12 @@ __global__ void __launch_bounds__(kConvPxWarps * 32) k_conv_fwd_px(const __nv_bf
         }
 #pragma unroll
         for (int f = 0; f < NF; f++) {
-            const __nv_bfloat16 *wr = w + (long long)(f * 8 + g) * Kp + kb + 2 * tig;
-            uint32_t b0 = __ldg(reinterpret_cast<const unsigned *>(wr));
-            uint32_t b1 = __ldg(reinterpret_cast<const unsigned *>(wr + 8));
+            const uint2 b = __ldg(reinterpret_cast<const uint2 *>(w) + (j * NF + f) * 32 + lane);
             asm volatile(
                 "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
                 "{%0,%1,%2,%3};\n"
                 : "+f"(acc[f][0]), "+f"(acc[f][1]), "+f"(acc[f][2]), "+f"(acc[f][3])
-                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
         }
     }
 #pragma unroll
@@ -311,19 +308,20 @@ __global__ void k_head_fwd(const __nv_bfloat16 *a6, int P, const float *wfc, con
     }
 }
 
-// loss, and the gradients of the linear layer (one CTA of kOut*kFeat
-// threads): the output gradients of kHeadChunk samples at a time are staged
-// in shared memory, thread (j, c) adds its products over the samples in order,
-// and the loss is every thread's squared errors (its entries in order) added
-// by a fixed tree.
-constexpr int kHeadChunk = 128;
+// loss, and the gradients of the linear layer (CTA j: output j): the output
+// gradients of kHeadChunk samples at a time and the features of kHeadTile of them
+// are staged in shared memory by all threads, thread c adds its products over
+// the samples in order.  CTA 0 adds the loss: every thread's squared errors (its
+// entries in order), then a fixed tree.  One CTA that read its features one
+// sample after another took 27 us for 256 samples.
+constexpr int kHeadChunk = 128, kHeadTile = 64;
 __global__ void k_head_grad(const float *y, const float *t, const float *feat, int N, float *gwfc, float *gbfc,
                             float *loss) {
     static_assert(kOut * kFeat == 768, "the loss tree folds 3 x 256 partial sums");
     __shared__ float sdy[kHeadChunk * kOut];
+    __shared__ float4 tile[kHeadTile][kFeat / 4];
     __shared__ float red[kOut * kFeat];
-    int i = threadIdx.x;  // j * kFeat + c
-    int j = i / kFeat, c = i % kFeat;
+    int i = threadIdx.x, j = blockIdx.x;
     float inv = 2.0f / (float)(kOut * N);
     float s = 0.0f, sb = 0.0f, l = 0.0f;
     for (int n0 = 0; n0 < N; n0 += kHeadChunk) {
@@ -334,16 +332,26 @@ __global__ void k_head_grad(const float *y, const float *t, const float *feat, i
             l += d * d;
             sdy[e] = d * inv;
         }
-        __syncthreads();
-#pragma unroll 16
-        for (int n = 0; n < cnt; n++) {
-            float dy = sdy[n * kOut + j];
-            s += dy * feat[(long long)(n0 + n) * kFeat + c];
-            sb += dy;
+        for (int q0 = 0; q0 < cnt; q0 += kHeadTile) {
+            int c = cnt - q0 < kHeadTile ? cnt - q0 : kHeadTile;
+            __syncthreads();  // the output gradients are there, the previous tile is consumed
+            const float4 *src = reinterpret_cast<const float4 *>(feat + (long long)(n0 + q0) * kFeat);
+            for (int e = i; e < c * (kFeat / 4); e += blockDim.x) (&tile[0][0])[e] = __ldg(src + e);
+            __syncthreads();
+            if (i < kFeat) {
+                const float *f = reinterpret_cast<const float *>(&tile[0][0]) + i;
+#pragma unroll 8
+                for (int n = 0; n < c; n++) {
+                    float dy = sdy[(q0 + n) * kOut + j];
+                    s += dy * f[n * kFeat];
+                    sb += dy;
+                }
+            }
         }
     }
-    gwfc[i] = s;
-    if (c == 0) gbfc[j] = sb;
+    if (i < kFeat) gwfc[j * kFeat + i] = s;
+    if (i == 0) gbfc[j] = sb;
+    if (j != 0) return;
     red[i] = l;
     __syncthreads();
     if (i < 256) red[i] = (red[i] + red[i + 256]) + red[i + 512];
@@ -413,10 +421,10 @@ constexpr int kWgKT = 64, kWgMS = 64, kWgThreads = 128;
 // turned, alike for the 8 rows of a fragment (the stores of 16 rows' words then
 // share a bank 4 times instead of 8)
 __device__ __forceinline__ constexpr int wg_swizzle(int k) { return 8 * ((k >> 3) & 3); }
-template <int COUT, int CIN>
-__global__ void __launch_bounds__(kWgThreads) k_conv_wgrad_tc(const float *dz, const __nv_bfloat16 *in, int N,
-                                                              int H, int W, int Ho, int Wo, int nsplit, int per,
-                                                              float *partial) {
+template <int L>
+__global__ void __launch_bounds__(kWgThreads) k_conv_wgrad_tc(const float *dz, const __nv_bfloat16 *in, int N, int nsplit,
+                                                              int per, float *partial) {
+    constexpr int COUT = kCout[L], CIN = kCin[L], H = kHt[L], W = kWd[L], Ho = kHt[L + 1], Wo = kWd[L + 1];
     constexpr int K = 9 * CIN, Kp = kpad(CIN);
     constexpr int RT = COUT / 16, FPW = RT * 2;  // 8 column fragments per row tile, over 4 warps
     constexpr int LD = kWgMS / 2 + 4;            // words per staged row
@@ -441,8 +449,8 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad_tc(const float *dz, c
     for (long long m0 = mb; m0 < me; m0 += kWgMS) {
         __syncthreads();  // the previous stage is consumed
         if (tid < kWgMS) {
-            long long m = m0 + tid;
-            int oy = (int)((m / Wo) % Ho), ox = (int)(m % Wo), n = (int)(m / ((long long)Wo * Ho));
+            unsigned m = (unsigned)m0 + tid;
+            int oy = (int)(m / Wo % Ho), ox = (int)(m % Wo), n = (int)(m / (Wo * Ho));
             unsigned taps = 0;
             if (m < me)
                 for (int q = 0; q < 9; q++) {
@@ -453,11 +461,12 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad_tc(const float *dz, c
             s_at[tid] = (((long long)n * H + 2 * oy - 1) * W + 2 * ox - 1) * CIN;
         }
         // dz^T: thread tid always stages co = tid % COUT
+#pragma unroll 8
         for (int e = tid; e < COUT * (kWgMS / 2); e += kWgThreads) {
             int co = e % COUT, mp = e / COUT;
             long long m = m0 + 2 * mp;
-            float v0 = m < me ? dz[m * COUT + co] : 0.0f;
-            float v1 = m + 1 < me ? dz[(m + 1) * COUT + co] : 0.0f;
+            float v0 = m < me ? __ldg(dz + m * COUT + co) : 0.0f;
+            float v1 = m + 1 < me ? __ldg(dz + (m + 1) * COUT + co) : 0.0f;
             bsum += v0;
             bsum += v1;
             sD[co][mp] = pack_bf16(v0, v1);
@@ -515,26 +524,34 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad_tc(const float *dz, c
 
 // Sums the splits of every entry of partial[e][s] (e = co (Kp + 1) + k) in a
 // fixed order into the flat gradient (weights, then the bias): with few
-// splits a thread per entry adds them in order; with many a warp per entry,
-// lane q adding splits q, q + 32, ... in order and the lanes then added by a
-// fixed butterfly.
-__global__ void k_wgrad_reduce(const float *partial, int nsplit, int Cout, int Kp, float *gw, float *gb) {
+// splits a thread per entry adds them in order; with more as 32 sums, sum q of
+// the splits q, q + 32, ... in order, added by halves (q and q + 16, then q and
+// q + 8, ...).  `lanes` threads take an entry (reduce_lanes): 32, a sum each, or
+// 8, thread u the sums u, u + 8, u + 16 and u + 24 (256 samples, 8 lanes against
+// 32: 24 splits of the fifth layer 5 us against 12, 80 of the fourth 6 against
+// 11, 300 of the second 7 against 4, 960 of the first 16 against 6).
+constexpr int reduce_lanes(int nsplit) { return nsplit <= 8 ? 1 : nsplit <= 192 ? 8 : 32; }
+__global__ void k_wgrad_reduce(const float *partial, int nsplit, int lanes, int Cout, int Kp, float *gw, float *gb) {
     int row = Kp + 1;
-    long long ne = (long long)Cout * row;
-    long long e;
+    unsigned ne = Cout * row, e = (blockIdx.x * blockDim.x + threadIdx.x) >> (__ffs(lanes) - 1);
+    const float *p = partial + (long long)(e < ne ? e : 0) * nsplit;
     float v = 0.0f;
-    if (nsplit <= 8) {
-        e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-        if (e >= ne) return;
-        for (int q = 0; q < nsplit; q++) v += partial[e * nsplit + q];
+    if (lanes == 1) {
+        for (int q = 0; q < nsplit; q++) v += p[q];
+    } else if (lanes == 8) {
+        int u = threadIdx.x & 7;
+        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int q0 = 0; q0 < nsplit; q0 += 32)
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (q0 + 8 * k + u < nsplit) s[k] += p[q0 + 8 * k + u];
+        v = (s[0] + s[2]) + (s[1] + s[3]);
     } else {
-        e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-        int lane = threadIdx.x & 31;
-        if (e >= ne) return;  // uniform over the warp
-        for (int q = lane; q < nsplit; q += 32) v += partial[e * nsplit + q];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane) return;
+        for (int q = threadIdx.x & 31; q < nsplit; q += 32) v += p[q];
     }
+    if (lanes > 1)
+        for (int o = lanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (e >= ne || threadIdx.x & (lanes - 1)) return;
     int co = (int)(e / row), k = (int)(e % row);
     if (k == Kp) gb[co] = v;
     else gw[(long long)co * Kp + k] = v;
@@ -546,7 +563,7 @@ __global__ void k_wgrad_reduce(const float *partial, int nsplit, int Cout, int K
 // o(p, tap) the output pixel that pixel p feeds through the tap (stride 2: by
 // the parity of p's coordinates only 1, 2 or 4 of the 9 taps exist).  A GEMM
 // of the input pixels (rows) by Cin (columns) with BF16 operands (dz rounded to
-// nearest even, the weights as [9][Cin][Cout] in wt) and FP32 accumulation,
+// nearest even, the weights as k_weight_fragments leaves them in wt) and FP32 accumulation,
 // the taps and co in ascending order.  The rows are the input pixels in parity
 // class order ((y & 1, x & 1) outermost, then image, row, column), so the 16
 // rows of a warp almost always share their taps and a tap that none of them
@@ -554,10 +571,10 @@ __global__ void k_wgrad_reduce(const float *partial, int nsplit, int Cout, int K
 // reduced by KS warps (warp group kg takes the co steps kg, kg + KS, ... of
 // every tap), whose tiles are then added in group order (the deep layers
 // have few rows and long reductions).
-template <int CIN, int Cout, int KS>
+template <int L, int KS>
 __global__ void __launch_bounds__(128) k_conv_dgrad_tc(const float *dz, const __nv_bfloat16 *wt,
-                                                       const __nv_bfloat16 *a_prev, int N, int H, int W, int Ho, int Wo,
-                                                       float *dz_prev) {
+                                                       const __nv_bfloat16 *a_prev, int N, float *dz_prev) {
+    constexpr int Cout = kCout[L], CIN = kCin[L], H = kHt[L], W = kWd[L], Ho = kHt[L + 1], Wo = kWd[L + 1];
     constexpr int NF = CIN / 8;
     static_assert(KS == 1 || KS == 2 || KS == 4, "4 warps per CTA");
     __shared__ float red[KS > 1 ? 4 : 1][KS > 1 ? 16 : 1][KS > 1 ? CIN : 1];
@@ -569,24 +586,24 @@ __global__ void __launch_bounds__(128) k_conv_dgrad_tc(const float *dz, const __
     bool ok[2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        long long r = rbase + g + 8 * h;
+        unsigned r = (unsigned)rbase + g + 8 * h;
         ok[h] = false;
         pix[h] = 0;
         yy[h] = xx[h] = nn[h] = 0;
+        bool past = false;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            int py = q >> 1, px = q & 1;
-            int hq = (H + 1 - py) / 2, wq = (W + 1 - px) / 2;
-            long long cnt = (long long)N * hq * wq;
-            if (!ok[h] && r >= 0 && r < cnt) {
-                int n = (int)(r / ((long long)hq * wq));
-                int rem = (int)(r - (long long)n * hq * wq);
+            const int py = q >> 1, px = q & 1, hq = (H + 1 - py) / 2, wq = (W + 1 - px) / 2;
+            unsigned cnt = (unsigned)N * (hq * wq);
+            if (!past && !ok[h] && r < cnt) {
+                int n = (int)(r / (hq * wq)), rem = (int)(r % (hq * wq));
                 nn[h] = n;
                 yy[h] = 2 * (rem / wq) + py;
                 xx[h] = 2 * (rem % wq) + px;
                 pix[h] = ((long long)n * H + yy[h]) * W + xx[h];
                 ok[h] = true;
             }
+            past |= r < cnt;
             r -= cnt;
         }
     }
@@ -604,7 +621,7 @@ __global__ void __launch_bounds__(128) k_conv_dgrad_tc(const float *dz, const __
             o[h] = v[h] ? (((long long)nn[h] * Ho + (ty >> 1)) * Wo + (tx >> 1)) * Cout : 0;
         }
         if (!__any_sync(0xffffffffu, v[0] || v[1])) continue;
-        const uint32_t *wtap = reinterpret_cast<const uint32_t *>(wt + (long long)tap * CIN * Cout);
+        const uint4 *wtap = reinterpret_cast<const uint4 *>(wt + (long long)tap * CIN * Cout) + lane;
 #pragma unroll 2
         for (int co0 = 16 * kg; co0 < Cout; co0 += 16 * KS) {
             uint32_t a[4];
@@ -615,9 +632,10 @@ __global__ void __launch_bounds__(128) k_conv_dgrad_tc(const float *dz, const __
                 a[q] = pack_bf16(d.x, d.y);
             }
 #pragma unroll
-            for (int f = 0; f < NF; f++) {
-                int wi = ((8 * f + g) * Cout + co0 + 2 * t) >> 1;
-                mma_bf16(acc[f], a, __ldg(wtap + wi), __ldg(wtap + wi + 4));
+            for (int f = 0; f < NF; f += 2) {
+                const uint4 b = __ldg(wtap + (co0 / 16 * NF + f) * 16);
+                mma_bf16(acc[f], a, b.x, b.y);
+                mma_bf16(acc[f + 1], a, b.z, b.w);
             }
         }
     }
@@ -656,19 +674,32 @@ __global__ void __launch_bounds__(128) k_conv_dgrad_tc(const float *dz, const __
     }
 }
 
-// The convolution weights of every layer as [9][Cin][Cout] (BF16) for the
-// input-gradient kernel: wt[tap][c][co] = w[co][tap Cin + c].
-struct WtLayout {
-    int64_t src[kLayers], dst[kLayers];
+// The convolution weights in the order of mma.sync's B fragments, so that a warp
+// reads a fragment with one load of consecutive words (from rows of weights a
+// fragment took eight separate 16-byte pieces, twice).  Lane (g, t) = (lane / 4,
+// lane % 4) of a fragment holds k = 2t, 2t + 1 and 2t + 8, 2t + 9 of column g.
+// Forward (wf): w[co][k], [K step][co / 8][lane][2 words].  Input gradient (wt,
+// layers of 16 and more input channels): w[co][tap Cin + c] as columns c and
+// k = co, [tap][co / 16][c / 16][lane][c / 8 % 2][2 words].
+struct WeightLayout {
+    int64_t src[kLayers], wf[kLayers], wt[kLayers];
     int cin[kLayers], cout[kLayers];
 };
-__global__ void k_wt_transpose(const __nv_bfloat16 *pbf, __nv_bfloat16 *wt, WtLayout lay) {
+__global__ void k_weight_fragments(const __nv_bfloat16 *pbf, __nv_bfloat16 *wf, __nv_bfloat16 *wt, WeightLayout lay) {
     int l = blockIdx.y;
-    int Cin = lay.cin[l], Cout = lay.cout[l], Kp = (9 * Cin + 15) / 16 * 16;
-    int tot = 9 * Cin * Cout;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += gridDim.x * blockDim.x) {
-        int co = e % Cout, k = e / Cout;  // k = tap * Cin + c
-        wt[lay.dst[l] + e] = pbf[lay.src[l] + (int64_t)co * Kp + k];
+    int Cin = lay.cin[l], Cout = lay.cout[l], Kp = kpad(Cin);
+    const __nv_bfloat16 *w = pbf + lay.src[l];
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < Kp * Cout; e += gridDim.x * blockDim.x) {
+        int half = e & 1, word = e >> 1 & 1, lane = e >> 2 & 31, q = e >> 7;
+        int co = q % (Cout / 8) * 8 + (lane >> 2), k = q / (Cout / 8) * 16 + 2 * (lane & 3) + 8 * word + half;
+        wf[lay.wf[l] + e] = w[(int64_t)co * Kp + k];
+    }
+    if (Cin % 16) return;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 9 * Cin * Cout; e += gridDim.x * blockDim.x) {
+        int half = e & 1, word = e >> 1 & 1, odd = e >> 2 & 1, lane = e >> 3 & 31, q = e >> 8;
+        int c = q % (Cin / 16) * 16 + 8 * odd + (lane >> 2);
+        int r = q / (Cin / 16), co = r % (Cout / 16) * 16 + 2 * (lane & 3) + 8 * word + half, tap = r / (Cout / 16);
+        wt[lay.wt[l] + e] = w[(int64_t)co * Kp + tap * Cin + c];
     }
 }
 
@@ -737,8 +768,8 @@ struct recon_initnet {
     Offsets off;
     float *params = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
     __nv_bfloat16 *pbf = nullptr;
-    __nv_bfloat16 *wt = nullptr;  // the convolution weights as [9][Cin][Cout] per layer
-    WtLayout wt_lay;
+    __nv_bfloat16 *wf = nullptr, *wt = nullptr;  // the convolution weights as fragments (k_weight_fragments)
+    WeightLayout frag;
     __nv_bfloat16 *act[kLayers] = {nullptr};
     float *dz[kLayers] = {nullptr};
     float *feat = nullptr, *y = nullptr, *partial = nullptr, *loss = nullptr;
@@ -805,10 +836,8 @@ bool pixel_parallel(int l, int n) {
 
 template <int L, int MT>
 void conv_tiled(recon_initnet *net, const __nv_bfloat16 *in, int n, long long M, int S) {
-    k_conv_fwd<kCout[L], kCin[L], MT><<<dim3((unsigned)((M + 16 * MT - 1) / (16 * MT)), (unsigned)S), kConvWarps * 32, 0,
-                                        net->stream>>>(in, n, kHt[L], kWd[L], net->pbf + net->off.w[L],
-                                                       net->params + net->off.b[L], net->act[L], kHt[L + 1], kWd[L + 1],
-                                                       net->fpart);
+    k_conv_fwd<L, MT><<<dim3((unsigned)((M + 16 * MT - 1) / (16 * MT)), (unsigned)S), kConvWarps * 32, 0, net->stream>>>(
+        in, n, net->wf + net->frag.wf[L], net->params + net->off.b[L], net->act[L], net->fpart);
 }
 
 template <int L>
@@ -832,8 +861,8 @@ void conv_launch(recon_initnet *net, const __nv_bfloat16 *in, int n) {
         }
     }
     long long tiles = (M + 15) / 16;
-    k_conv_fwd_px<COUT, CIN><<<(unsigned)((tiles + kConvPxWarps - 1) / kConvPxWarps), kConvPxWarps * 32, 0, net->stream>>>(
-        in, n, kHt[L], kWd[L], net->pbf + net->off.w[L], b, net->act[L], kHt[L + 1], kWd[L + 1]);
+    k_conv_fwd_px<L><<<(unsigned)((tiles + kConvPxWarps - 1) / kConvPxWarps), kConvPxWarps * 32, 0, net->stream>>>(
+        in, n, net->wf + net->frag.wf[L], b, net->act[L]);
 }
 
 int conv_forward(recon_initnet *net, int l, const __nv_bfloat16 *in, int n) {
@@ -852,14 +881,12 @@ int conv_forward(recon_initnet *net, int l, const __nv_bfloat16 *in, int n) {
 template <int L>
 void wgrad_launch(recon_initnet *net, const __nv_bfloat16 *in, int n, int ns, int per) {
     dim3 grid((kpad(kCin[L]) + kWgKT - 1) / kWgKT, ns);
-    k_conv_wgrad_tc<kCout[L], kCin[L]><<<grid, kWgThreads, 0, net->stream>>>(net->dz[L], in, n, kHt[L], kWd[L], kHt[L + 1],
-                                                                             kWd[L + 1], ns, per, net->partial);
+    k_conv_wgrad_tc<L><<<grid, kWgThreads, 0, net->stream>>>(net->dz[L], in, n, ns, per, net->partial);
 }
 template <int L, int KS>
 void dgrad_tiled(recon_initnet *net, int n, long long tiles) {
-    k_conv_dgrad_tc<kCin[L], kCout[L], KS><<<(unsigned)((tiles + 4 / KS - 1) / (4 / KS)), 128, 0, net->stream>>>(
-        net->dz[L], net->wt + net->wt_lay.dst[L], net->act[L - 1], n, kHt[L], kWd[L], kHt[L + 1], kWd[L + 1],
-        net->dz[L - 1]);
+    k_conv_dgrad_tc<L, KS><<<(unsigned)((tiles + 4 / KS - 1) / (4 / KS)), 128, 0, net->stream>>>(
+        net->dz[L], net->wt + net->frag.wt[L], net->act[L - 1], n, net->dz[L - 1]);
 }
 template <int L>
 void dgrad_launch(recon_initnet *net, int n) {
@@ -890,7 +917,7 @@ int forward(recon_initnet *net, const __nv_bfloat16 *in, int n) {
 
 int backward(recon_initnet *net, const __nv_bfloat16 *in, const float *target, int n, float *grad, float *loss) {
     int P = kHt[kLayers] * kWd[kLayers];
-    k_head_grad<<<1, kOut * kFeat, 0, net->stream>>>(net->y, target, net->feat, n, grad + net->off.wfc,
+    k_head_grad<<<kOut, kOut * kFeat, 0, net->stream>>>(net->y, target, net->feat, n, grad + net->off.wfc,
                                                     grad + net->off.bfc, loss);
     k_head_back<<<n, kFeat, 0, net->stream>>>(net->y, target, net->params + net->off.wfc, net->act[kLayers - 1], n, P,
                                               net->dz[kLayers - 1]);
@@ -907,9 +934,10 @@ int backward(recon_initnet *net, const __nv_bfloat16 *in, const float *target, i
             case 4: wgrad_launch<4>(net, lin, n, ns, per); break;
             default: wgrad_launch<5>(net, lin, n, ns, per); break;
         }
-        long long red_threads = (long long)Cout * row * (ns <= 8 ? 1 : 32);
+        int lanes = reduce_lanes(ns);
+        long long red_threads = (long long)Cout * row * lanes;
         k_wgrad_reduce<<<(unsigned)((red_threads + 127) / 128), 128, 0, net->stream>>>(
-            net->partial, ns, Cout, Kp, grad + net->off.w[l], grad + net->off.b[l]);
+            net->partial, ns, lanes, Cout, Kp, grad + net->off.w[l], grad + net->off.b[l]);
         switch (l) {
             case 0: break;
             case 1: dgrad_launch<1>(net, n); break;
@@ -933,7 +961,7 @@ int check_batch(recon_initnet *net, int n) {
 void refresh_bf16(recon_initnet *net) {
     int64_t tot = net->off.total;
     k_to_bf16<<<(unsigned)((tot + 255) / 256), 256, 0, net->stream>>>(net->params, net->pbf, tot);
-    k_wt_transpose<<<dim3(64, kLayers), 256, 0, net->stream>>>(net->pbf, net->wt, net->wt_lay);
+    k_weight_fragments<<<dim3(64, kLayers), 256, 0, net->stream>>>(net->pbf, net->wf, net->wt, net->frag);
 }
 
 }  // namespace
@@ -973,12 +1001,14 @@ int recon_initnet_create(int32_t max_batch, void *stream, recon_initnet **out) {
     net->off = offsets();
     net->stream = (cudaStream_t)stream;  // NULL: the legacy default stream
     int64_t P = net->off.total;
-    int64_t nwt = 0;
+    int64_t nwf = 0, nwt = 0;
     for (int l = 0; l < kLayers; l++) {
-        net->wt_lay.src[l] = net->off.w[l];
-        net->wt_lay.dst[l] = nwt;
-        net->wt_lay.cin[l] = kCin[l];
-        net->wt_lay.cout[l] = kCout[l];
+        net->frag.src[l] = net->off.w[l];
+        net->frag.wf[l] = nwf;
+        net->frag.wt[l] = nwt;
+        net->frag.cin[l] = kCin[l];
+        net->frag.cout[l] = kCout[l];
+        nwf += (int64_t)kpad(kCin[l]) * kCout[l];
         nwt += 9LL * kCin[l] * kCout[l];
     }
     int64_t part = 0;
@@ -997,7 +1027,8 @@ int recon_initnet_create(int32_t max_batch, void *stream, recon_initnet **out) {
         }
     bool ok = cudaMalloc(&net->params, P * 4) == cudaSuccess && cudaMalloc(&net->grad, P * 4) == cudaSuccess &&
               cudaMalloc(&net->m, P * 4) == cudaSuccess && cudaMalloc(&net->v, P * 4) == cudaSuccess &&
-              cudaMalloc(&net->pbf, P * 2) == cudaSuccess && cudaMalloc(&net->wt, nwt * 2) == cudaSuccess &&
+              cudaMalloc(&net->pbf, P * 2) == cudaSuccess && cudaMalloc(&net->wf, nwf * 2) == cudaSuccess &&
+              cudaMalloc(&net->wt, nwt * 2) == cudaSuccess &&
               cudaMalloc(&net->feat, (int64_t)max_batch * kFeat * 4) == cudaSuccess &&
               cudaMalloc(&net->y, (int64_t)max_batch * kOut * 4) == cudaSuccess &&
               cudaMalloc(&net->partial, part * 4) == cudaSuccess && cudaMalloc(&net->fpart, fpart * 4) == cudaSuccess &&
@@ -1031,6 +1062,7 @@ int recon_initnet_destroy(recon_initnet *net) {
     cudaFree(net->m);
     cudaFree(net->v);
     cudaFree(net->pbf);
+    cudaFree(net->wf);
     cudaFree(net->wt);
     cudaFree(net->feat);
     cudaFree(net->y);
