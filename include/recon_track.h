@@ -302,6 +302,10 @@ int recon_selftest_exact_arith(int64_t *mismatches);
  * (pseudo-random operands) against the compiler's IEEE division. */
 int recon_selftest_division(int64_t *mismatches);
 
+/* Makes `consumer` wait for the work queued so far on `producer` (two streams
+ * of the current device; no host stall). */
+int recon_stream_follow(void *consumer, void *producer);
+
 /* ---- single tracker (PhotoTracker-style handle = batch of one) ---- */
 typedef recon_batch recon_tracker;
 int recon_tracker_create(const recon_config *cfg, const float *calib, void *stream, recon_tracker **out);

@@ -100,6 +100,8 @@ _lib = None
 def lib() -> ctypes.CDLL:
     """Loads librecon_track.so (built by recon_gb300.build / __graft_entry__.build)."""
     global _lib
+    if _lib is not None:  # set once, complete
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(LIB_PATH):
@@ -162,6 +164,7 @@ def lib() -> ctypes.CDLL:
             L.recon_render_gray.argtypes = [vp, vp, vp, vp]
             L.recon_selftest_exact_arith.argtypes = [vp]
             L.recon_selftest_division.argtypes = [vp]
+            L.recon_stream_follow.argtypes = [vp, vp]
             L.recon_kinect_disparity_to_depth.argtypes = [vp, i32, i32, f32, f32, f32, f32, f32, f32, i32, vp, vp]
             L.recon_kinect_rgb_to_gray.argtypes = [vp, i32, i32, vp, vp]
             L.recon_kinect_undistort_gray.argtypes = [vp, i32, i32, vp, vp, vp, vp, vp]
@@ -231,12 +234,22 @@ def _on_device(a) -> int:
     return int(hasattr(a, "is_cuda") and a.is_cuda)
 
 
+def _torch_stream() -> int:
+    """The handle of torch's current stream (what torch.cuda.current_stream()
+    would wrap, without the wrapper: 0.2 against 3 us)."""
+    import torch
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def _order_after_torch(batch) -> None:
     """The batch reads device inputs on its own stream: make that stream wait
     for the work already queued on torch's current stream (which may still be
     writing the tensors being passed).  An event and a wait, no host stall."""
-    import torch
-    torch.cuda.ExternalStream(batch.stream()).wait_stream(torch.cuda.current_stream())
+    own, now = batch.stream() or 0, _torch_stream()
+    if own != now:
+        check(lib().recon_stream_follow(own, now))
 
 
 class DeviceView:
@@ -265,8 +278,9 @@ def _after_producer(consumer, a) -> None:
     """Orders the consumer's stream after the work that produces `a`: the
     owning library stream of a DeviceView, else torch's current stream."""
     if isinstance(a, DeviceView):
-        import torch
-        torch.cuda.ExternalStream(consumer.stream()).wait_stream(torch.cuda.ExternalStream(a.stream))
+        own = consumer.stream() or 0
+        if own != (a.stream or 0):
+            check(lib().recon_stream_follow(own, a.stream))
     elif _on_device(a):
         _order_after_torch(consumer)
 
@@ -935,8 +949,16 @@ def track_params_for(params, frame: int):
 # ---- Kinect pre-processing (include/recon_kinect.h); torch CUDA tensors in and out ----
 
 def _stream_now():
+    return ctypes.c_void_p(_torch_stream())
+
+
+def _new_gray(H: int, W: int, written: int, device):
+    """A uint8 [H, W] image of which a kernel writes the first `written` rows: the others are 0."""
     import torch
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    out = torch.empty((H, W), dtype=torch.uint8, device=device)
+    if written < H:
+        out[written:].zero_()
+    return out
 
 
 def kinect_disparity_to_depth(disp, c0: float, c1: float, min_dist: float, max_dist: float, x_off: float = 0.0,
@@ -955,20 +977,18 @@ def kinect_disparity_to_depth(disp, c0: float, c1: float, min_dist: float, max_d
 
 def kinect_rgb_to_gray(rgb, out=None):
     """OMPFunctions::convert2Gray on the GPU: uint8 [H, W, 3] -> uint8 [H, W]."""
-    import torch
     H, W = rgb.shape[:2]
     if out is None:
-        out = torch.zeros((H, W), dtype=torch.uint8, device=rgb.device)
+        out = _new_gray(H, W, H // 4 * 4, rgb.device)
     check(lib().recon_kinect_rgb_to_gray(_ptr(rgb), W, H, _ptr(out), _stream_now()))
     return out
 
 
 def kinect_undistort_gray(src, K, iK, kc, out=None):
     """OMPFunctions::undistort (lookup form) on the GPU: uint8 [H, W] -> uint8 [H, W]."""
-    import torch
     H, W = src.shape
     if out is None:
-        out = torch.zeros((H, W), dtype=torch.uint8, device=src.device)
+        out = _new_gray(H, W, H // 6 * 6, src.device)
     Kf = np.ascontiguousarray(np.asarray(K, np.float32).reshape(9))
     iKf = np.ascontiguousarray(np.asarray(iK, np.float32).reshape(9))
     kcf = np.ascontiguousarray(np.asarray(kc, np.float32).reshape(-1)[:5])

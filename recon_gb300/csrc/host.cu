@@ -1348,6 +1348,17 @@ int recon_batch_get_work(recon_batch *b, uint64_t *out, int32_t reset) {
 
 void *recon_batch_stream(recon_batch *b) { return b ? (void *)b->stream : nullptr; }
 
+int recon_stream_follow(void *consumer, void *producer) {
+    if (consumer == producer) return RECON_OK;
+    cudaEvent_t e = nullptr;
+    CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    cudaError_t rc = cudaEventRecord(e, (cudaStream_t)producer);
+    if (rc == cudaSuccess) rc = cudaStreamWaitEvent((cudaStream_t)consumer, e, 0);
+    cudaEventDestroy(e);  // its resources go when the wait is done
+    CK(rc);
+    return RECON_OK;
+}
+
 int64_t recon_launch_count(void) { return g_launches.load(); }
 
 int recon_batch_track_sequence(recon_batch *b, int32_t nf, const uint8_t *const *gray, const uint16_t *const *depth,
