@@ -543,13 +543,27 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
-// ICP chunks per k_iter CTA at `level` for a level whose largest instance has
-// `nchunk` chunks: the tuned value, else about five waves of CTAs over the
-// batch's chunks, at most 8 chunks each.  The result does not depend on it.
-int icp_per_cta(const recon_batch *b, int level, int nchunk) {
+// Blocks of 1024 pixels of the instances that run the level with the ICP term:
+// their actual ones, so that a batch of mixed resolutions is spread as evenly as
+// a uniform one.
+long long level_blocks(const recon_batch *b, int level) {
+    long long blocks = 0;
+    for (auto &c : b->cfg) {
+        if (level >= c.levels || c.mode == RECON_PHOTOMETRIC || c.iters[c.levels - 1 - level] <= 0) continue;
+        blocks += ((c.width >> level) * (c.height >> level) + kChunk - 1) / kChunk;
+    }
+    return blocks;
+}
+
+// ICP chunks per k_iter CTA at `level`: the tuned value, else about two waves of
+// CTAs over the batch's chunks, at most 8 chunks each.  The result does not
+// depend on it.  Few waves, because the groups' launches fill one another's last
+// waves (schedule_groups): 30 segments with 1, 2, 3, 5 and 8 waves 15024, 14538,
+// 14963, 15084, 15379 us; 256 mixed pairs 8224, 8187, 8182, 8180, 8194.
+int icp_per_cta(const recon_batch *b, int level) {
     if (b->icp_cpc[level] > 0) return b->icp_cpc[level];
-    int waves = 5 * kIterCtaSlots;
-    return std::min(8, std::max(1, (b->n * nchunk + waves / 2) / waves));
+    const long long waves = 2 * kIterCtaSlots;
+    return (int)std::min(8LL, std::max(1LL, (level_blocks(b, level) + waves / 2) / waves));
 }
 
 // the per-frame Gauss-Newton schedule (gpuEstimateIncrement, phototracker.cpp:666-689)
@@ -584,17 +598,8 @@ int launch_schedule(recon_batch *b, cudaStream_t s, bool in_graph, int first, in
                 CK(launch_pdl(k_icp_mask, dim3((nchunk + per - 1) / per, n), dim3(kLanes), s, D, level, per));
             }
             {
-                // about one wave of CTAs over the blocks of the instances that
-                // run the level (sized by their actual blocks, so that a batch
-                // of mixed resolutions is spread as evenly as a uniform one)
-                long long blocks = 0;
-                for (int i = 0; i < b->n; i++) {
-                    const recon_config &c = b->cfg[i];
-                    if (level >= c.levels || c.mode == RECON_PHOTOMETRIC || c.iters[c.levels - 1 - level] <= 0)
-                        continue;
-                    blocks += ((c.width >> level) * (c.height >> level) + kChunk - 1) / kChunk;
-                }
-                int per = (int)std::max(1LL, (blocks + kPassCtaSlots - 1) / kPassCtaSlots);
+                // about one wave of CTAs
+                int per = (int)std::max(1LL, (level_blocks(b, level) + kPassCtaSlots - 1) / kPassCtaSlots);
                 int gx = (nchunk + per - 1) / per;
                 TimedScope ts(b, s, TK_ICP_STUDENT, in_graph);
                 for (int pass = 1; pass <= 3; pass++)
@@ -602,7 +607,7 @@ int launch_schedule(recon_batch *b, cudaStream_t s, bool in_graph, int first, in
             }
             b->graph_kernels += 4;
         }
-        int per_cta = icp_per_cta(b, level, nchunk);
+        int per_cta = icp_per_cta(b, level);
         int ncta = any_icp ? (nchunk + per_cta - 1) / per_cta : 0;
         // every instance's photometric cluster, then ncta ICP CTAs per
         // instance, the total rounded up to whole clusters
@@ -1248,7 +1253,7 @@ int recon_batch_get_icp_chunks_per_cta(recon_batch *b, int32_t per_level[RECON_M
             const recon_config &c = b->cfg[i];
             if (l < c.levels) maxpix = std::max(maxpix, (c.width >> l) * (c.height >> l));
         }
-        per_level[l] = maxpix ? icp_per_cta(b, l, (maxpix + kChunk - 1) / kChunk) : 0;
+        per_level[l] = maxpix ? icp_per_cta(b, l) : 0;
     }
     return RECON_OK;
 }
