@@ -1503,6 +1503,45 @@ __device__ __forceinline__ void acc27(float *s, const float *j, float r) {
     for (int c = 0; c < 6; c++, q++) s[q] = __fmaf_rn(j[c], r, s[q]);
 }
 
+// The same 27 sums two by two: 12 packed and 3 plain multiply-adds, each half
+// rounded as the plain one is, for 27.  The ICP term's pixels leave their terms as
+// pairs, 8 shared-memory accesses a pixel for 14: 30 segments 14538 -> 14337 us.
+// (The photometric term, whose Jacobian comes by columns, is 1% slower so.)
+struct Terms27 {
+    float2 p[12];
+    float s[3];
+    __device__ __forceinline__ Terms27() {
+#pragma unroll
+        for (int k = 0; k < 12; k++) p[k] = make_float2(0.0f, 0.0f);
+        s[0] = s[1] = s[2] = 0.0f;
+    }
+    __device__ __forceinline__ void add(float2 a, float2 b, float2 c, float r) {
+        p[0] = fma2(dup2(a.x), a, p[0]);
+        p[1] = fma2(dup2(a.x), b, p[1]);
+        p[2] = fma2(dup2(a.x), c, p[2]);
+        s[0] = __fmaf_rn(a.y, a.y, s[0]);
+        p[3] = fma2(dup2(a.y), b, p[3]);
+        p[4] = fma2(dup2(a.y), c, p[4]);
+        p[5] = fma2(dup2(b.x), b, p[5]);
+        p[6] = fma2(dup2(b.x), c, p[6]);
+        s[1] = __fmaf_rn(b.y, b.y, s[1]);
+        p[7] = fma2(dup2(b.y), c, p[7]);
+        p[8] = fma2(dup2(c.x), c, p[8]);
+        s[2] = __fmaf_rn(c.y, c.y, s[2]);
+        p[9] = fma2(dup2(r), a, p[9]);
+        p[10] = fma2(dup2(r), b, p[10]);
+        p[11] = fma2(dup2(r), c, p[11]);
+    }
+    // in acc27's order
+    __device__ __forceinline__ void terms(float *v) const {
+        const float t[27] = {p[0].x, p[0].y, p[1].x, p[1].y, p[2].x, p[2].y, s[0],   p[3].x,  p[3].y,
+                             p[4].x, p[4].y, p[5].x, p[5].y, p[6].x, p[6].y, s[1],   p[7].x,  p[7].y,
+                             p[8].x, p[8].y, s[2],   p[9].x, p[9].y, p[10].x, p[10].y, p[11].x, p[11].y};
+#pragma unroll
+        for (int k = 0; k < 27; k++) v[k] = t[k];
+    }
+};
+
 // Warp totals of the 27 terms by recursive halving: at the step with offset o
 // each lane keeps half of its values and adds the partner's copy of them, so
 // lane q ends with term q.  Every addition pairs the same two partial sums as
@@ -2026,7 +2065,8 @@ __device__ void icp_chunks(const InstDesc &d, IterShared &sh, int level, int c0,
     int t = threadIdx.x;
     const IcpLevel L(d, level);
     const float opt_in = d.opt_in;
-    float *slot = sh.stage + t;
+    // a pixel's terms in the warp's own runs: three pairs, and the residual
+    float *slot = sh.stage + ((t >> 4) & 1) * kChunk + (t & ~31) + 2 * (t & 15), *slot_r = sh.stage + 6 * kChunk + t;
     for (int c = c0; c < c1; c++) {
         if (t == 0 && c + 1 < c1) icp_prefetch_chunk(d, level, c + 1, npix);
         const float *ref = d.ref_pl[level] + (size_t)c * 6 * kChunk + t, *wts = d.icp_w + c * kChunk + t;
@@ -2058,21 +2098,20 @@ __device__ void icp_chunks(const InstDesc &d, IterShared &sh, int level, int c0,
                 icp_point<kDepth>(L, T, opt_in, w[u], p[u], p[u] + 3, q[u], px[u], py[u], in[u], tap[u], j, r);
                 float *v = slot + (g + u) * kLanes;
 #pragma unroll
-                for (int k = 0; k < 6; k++) v[k * kChunk] = j[k];
-                v[6 * kChunk] = r;
+                for (int k = 0; k < 3; k++)
+                    *reinterpret_cast<float2 *>(v + 2 * k * kChunk) = make_float2(j[2 * k], j[2 * k + 1]);
+                slot_r[(g + u) * kLanes] = r;
             }
         }
-        float acc[27];
-#pragma unroll
-        for (int k = 0; k < 27; k++) acc[k] = 0.0f;
+        Terms27 sum;
 #pragma unroll
         for (int m = 0; m < 4; m++) {
             const float *v = slot + m * kLanes;
-            float j[6];
-#pragma unroll
-            for (int k = 0; k < 6; k++) j[k] = v[k * kChunk];
-            acc27(acc, j, v[6 * kChunk]);
+            sum.add(*reinterpret_cast<const float2 *>(v), *reinterpret_cast<const float2 *>(v + 2 * kChunk),
+                    *reinterpret_cast<const float2 *>(v + 4 * kChunk), slot_r[m * kLanes]);
         }
+        float acc[27];
+        sum.terms(acc);
         fx_accumulate(sums, warp_terms(acc, sh.stage + (t & ~31)), bad);
     }
 }
