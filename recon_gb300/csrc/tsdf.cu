@@ -76,7 +76,7 @@ struct Geom {
     float K0, K2, K4, K5, Wf, Hf, Wm2, Hm2;
     float sx, sy, sz;               // centre of voxel 0 (start)
     float vx2, vy2, vz2;            // voxel spacing (2 * voxelSize)
-    float lim, tol, slope;          // update gates
+    float lim, tol, slope, inv_slope, slope_lo;  // update gates; RN(1 / slope), the least numerator for div_rn
     float b0x, b0y, b0z, b1x, b1y, b1z;  // grid bounds
     float ib0x, ib0y, ib0z;         // interpolation origin
     float ivx, ivy, ivz;            // 1 / voxel spacing (voxelize's invVoxelDim)
@@ -101,11 +101,16 @@ __device__ __forceinline__ void mark_negative(uint8_t *flags, const Geom &g, uns
 
 // ---------------------------------------------------------------- update --
 
+// programmatic dependent launches (launch_after)
+__device__ __forceinline__ void wait_before() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 // The largest distance in each 16 x 16 tile of the distance map (infinity where
 // the tile holds a NaN): one warp per tile.
 __global__ void __launch_bounds__(128) k_far_tiles(const float *__restrict__ dist, Geom g, float *__restrict__ far_tiles,
-                                                   int *__restrict__ count) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *count = 0;
+                                                   int *__restrict__ counts) {
+    next_may_start();
+    if (blockIdx.x == 0 && threadIdx.x < 2) counts[threadIdx.x] = 0;
     const int tile = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (tile >= g.tiles_x * g.tiles_y) return;
     const int x = (tile % g.tiles_x) * kFarTile + (lane & 15), y0 = (tile / g.tiles_x) * kFarTile + (lane >> 4);
@@ -126,6 +131,7 @@ struct Block {
     float near;                    // the least depth, less what the roundings may add
     bool outside;                  // no voxel projects into the image
     bool sharp;                    // in front of the camera, projected to better than a pixel
+    bool plain;                    // in front of it, and no coordinate beyond the range of div_rn
     __device__ __forceinline__ Block(const Geom &g, int x0, int y0, int z0) {
         const int lane = threadIdx.x & 31, group = lane & 24;
         const int cx = min(x0 + ((lane & 1) ? kTileX - 1 : 0), g.R - 1);
@@ -138,6 +144,7 @@ struct Block {
         lo_y = hi_y = (ry / rz * g.K4 + g.K5) * g.Hf;
         const float off = 1e-6f * (fabsf(g.T[8] * px) + fabsf(g.T[9] * py) + fabsf(g.T[10] * pz) + fabsf(g.T[11]));
         near = -rz - off;
+        const bool small = fmaxf(fmaxf(fabsf(rx), fabsf(ry)), -rz) <= 0x1p40f;
         const bool pixel = off * fmaxf(fabsf(g.K0) * g.Wf, fabsf(g.K4) * g.Hf) < near;
         for (int o = 1; o < 8; o <<= 1) {
             lo_x = fminf(lo_x, __shfl_xor_sync(0xffffffffu, lo_x, o));
@@ -151,6 +158,7 @@ struct Block {
         const unsigned front = __ballot_sync(0xffffffffu, rz < -16.0f) >> group & 0xffu;
         const unsigned behind = __ballot_sync(0xffffffffu, rz > 16.0f) >> group & 0xffu;
         sharp = front == 0xffu && (__ballot_sync(0xffffffffu, pixel) >> group & 0xffu) == 0xffu;
+        plain = front == 0xffu && fmaxf(fabsf(g.K0), fabsf(g.K4)) <= 16.0f && (__ballot_sync(0xffffffffu, small) >> group & 0xffu) == 0xffu;
         outside = (front == 0xffu || behind == 0xffu) && (!(hi_x >= -3.0f) || !(lo_x < g.Wf + 2.0f) ||
                                                           !(hi_y >= -3.0f) || !(lo_y < g.Hf + 2.0f));
     }
@@ -174,68 +182,85 @@ struct Block {
 };
 
 // The blocks that the update has to visit: 8 lanes per block.  count was set
-// to 0 by k_far_tiles.  Their order in the list is of no matter: every voxel
+// to 0 by k_far_tiles.  A block that is not plain is listed as ~number.  Their order in the list is of no matter: every voxel
 // is in one block.
 __global__ void __launch_bounds__(256)
     k_pick_blocks(const float *__restrict__ far_tiles, Geom g, int bx, int by, int n, int *__restrict__ list,
                   int *__restrict__ count) {
+    next_may_start();
     const int lane = threadIdx.x & 31, i = (blockIdx.x * 256 + threadIdx.x) >> 3, b = min(i, n - 1);
     const Block block(g, b % bx * kTileX, b / bx % by * kTileY, b / bx / by * kRunZ);
+    wait_before();
     const bool hidden = block.hidden(g, far_tiles);  // by all lanes
     const bool visit = (lane & 7) == 0 && i < n && !hidden && !block.outside;
     const unsigned all = __ballot_sync(0xffffffffu, visit);
     int at = 0;
     if (lane == 0 && all) at = atomicAdd(count, __popc(all));
     at = __shfl_sync(0xffffffffu, at, 0);
-    if (visit) list[at + __popc(all & ((1u << lane) - 1))] = b;
+    if (visit) list[at + __popc(all & ((1u << lane) - 1))] = block.plain ? b : ~b;
 }
 
 // updateVoxelsKernel (VoxelGrid_cuda.cu:944-1014) for the 8 voxels along z from
 // (ix, iy, z0)
+//
+// plain (Block::plain, uniform over the warp): the quotients of the projection go
+// through div_rn without a look at the operands.  They are at most 2^40; one below
+// 2^-60, or a zero whose sign is lost, moves the pixel by less than 2^-60 of the
+// image: nothing beside a principal point of 2^-20, and with a smaller one the
+// pixel is before the first.
 __device__ __forceinline__ void fuse_run(float2 *__restrict__ grid, uint8_t *__restrict__ flags,
-                                         const float *__restrict__ dist, const Geom &g, int ix, int iy, int z0,
-                                         unsigned &n_proj, unsigned &n_fused, unsigned &n_changed) {
+                                         const float *__restrict__ dist, const Geom &g, bool plain, int ix, int iy,
+                                         int z0, unsigned &n_proj, unsigned &n_fused, unsigned &n_changed) {
     const float px = g.sx + (float)ix * g.vx2;
     const float py = g.sy + (float)iy * g.vy2;
     // T p summed left to right: the first two products do not depend on z
     const float ax = g.T[0] * px + g.T[1] * py, ay = g.T[4] * px + g.T[5] * py, az = g.T[8] * px + g.T[9] * py;
-    const int W = g.W;
+    const size_t slice = (size_t)g.R * g.R;
+    float2 *gp = grid + (size_t)z0 * slice + (size_t)iy * g.R + ix;
+    float zf = (float)z0;
+    // the run lies in one brick
+    uint8_t *brick = flags + brick_of(g, ix, iy, z0), *super = flags + super_of(g, ix, iy, z0);
 #pragma unroll 2
-    for (int k = 0; k < kRunZ; k++) {
-        const int iz = z0 + k;
-        const float pz = g.sz + (float)iz * g.vz2;
-        float rx = ax + g.T[2] * pz + g.T[3];
-        float ry = ay + g.T[6] * pz + g.T[7];
+    for (int k = 0; k < kRunZ; k++, gp += slice, zf += 1.0f) {
+        const float pz = g.sz + zf * g.vz2;
+        const float rx = ax + g.T[2] * pz + g.T[3];
+        const float ry = ay + g.T[6] * pz + g.T[7];
         const float rz = az + g.T[10] * pz + g.T[11];
         const float voxel_dist = -rz;
-        rx /= rz;
-        ry /= rz;
-        const float ux = (rx * g.K0 + g.K2) * g.Wf;
-        const float uy = (ry * g.K4 + g.K5) * g.Hf;
+        const float irz = rt::rcp_rn(rz);
+        float qx = rt::div_rn(rx, voxel_dist, irz), qy = rt::div_rn(ry, voxel_dist, irz);
+        if (!plain) {
+            qx = rt::ieee_div(rx, rz);
+            qy = rt::ieee_div(ry, rz);
+        }
+        const float ux = (qx * g.K0 + g.K2) * g.Wf;
+        const float uy = (qy * g.K4 + g.K5) * g.Hf;
         // int(u) in [1, size - 2): the reference's safeBorder of 1
         if (!(ux >= 1.0f && ux < g.Wm2 && uy >= 1.0f && uy < g.Hm2)) continue;
         n_proj++;
-        const int ui = (int)ux, vi = (int)uy;
-        const float *dp = dist + (size_t)vi * W + ui;
-        const float a = __ldg(dp), b = __ldg(dp + 1), c = __ldg(dp + W), d = __ldg(dp + W + 1);
-        if (a < g.lim || b < g.lim || c < g.lim || d < g.lim) continue;
-        const float fu = ux - (float)ui;
-        const float fv = uy - (float)vi;
+        // trunc by a sum rounded toward zero: no conversions
+        const float su = rt::index_sum(ux), sv = rt::index_sum(uy);
+        const float *dp = dist + (rt::index_of(sv) * g.W + rt::index_of(su));
+        const float a = __ldg(dp), b = __ldg(dp + 1), c = __ldg(dp + g.W), d = __ldg(dp + g.W + 1);
+        if (fminf(fminf(a, b), fminf(c, d)) < g.lim) continue;
+        const float fu = ux - (su - 8388608.0f);
+        const float fv = uy - (sv - 8388608.0f);
         const float z = (1 - fu) * (1 - fv) * a + fu * (1 - fv) * b + (1 - fu) * fv * c + fu * fv * d;
         if (fabsf(z - a) > g.tol || fabsf(z - b) > g.tol || fabsf(z - c) > g.tol || fabsf(z - d) > g.tol) continue;
-        const float sdf = -(voxel_dist - z) / g.slope;
+        const float dz = -(voxel_dist - z);
+        float sdf = rt::div_rn(dz, -g.slope, g.inv_slope);
+        if (!(fabsf(dz) >= g.slope_lo && fabsf(dz) <= 0x1p60f)) sdf = rt::ieee_div(dz, g.slope);
         if (sdf < -1.25f) continue;
         n_fused++;
         const float nt = fmaxf(fminf(1.0f, sdf), -1.0f);
-        float2 *gp = grid + ((size_t)iz * g.R + iy) * g.R + ix;
         const float2 old = *gp;
-        const float nx = (old.y * old.x + 1.0f * nt) / (old.y + 1.0f);
+        const float nx = (old.y * old.x + nt) / (old.y + 1.0f);
         const float ny = fminf(1.0f + old.y, 16.0f);
         if (__float_as_uint(nx) != __float_as_uint(old.x) || __float_as_uint(ny) != __float_as_uint(old.y)) {
             *gp = make_float2(nx, ny);
             n_changed++;
         }
-        if (nx < 0.0f) mark_negative(flags, g, ix, iy, iz);
+        if (nx < 0.0f) *brick = *super = 1;
     }
 }
 
@@ -250,14 +275,14 @@ __global__ void __launch_bounds__(kTileX * kTileY)
     const int x0 = blockIdx.x * kTileX, y0 = blockIdx.y * kTileY, z0 = blockIdx.z * kRunZ;
     if (threadIdx.x < 32) {
         const Block block(g, x0, y0, z0);
-        if (lane == 0) s_skip = block.outside;
+        if (lane == 0) s_skip = block.outside ? 1 : (block.plain ? 0 : 2);
     }
     __syncthreads();
-    if (s_skip) return;
+    if (s_skip == 1) return;
     const int ix = x0 + lane, iy = y0 + (threadIdx.x >> 5);
     if (ix >= g.R) return;
     unsigned n_proj = 0, n_fused = 0, n_changed = 0;
-    fuse_run(grid, flags, dist, g, ix, iy, z0, n_proj, n_fused, n_changed);
+    fuse_run(grid, flags, dist, g, s_skip == 0, ix, iy, z0, n_proj, n_fused, n_changed);
     if (kCount) {
         n_proj = __reduce_add_sync(0xffffffffu, n_proj);
         n_fused = __reduce_add_sync(0xffffffffu, n_fused);
@@ -270,24 +295,35 @@ __global__ void __launch_bounds__(kTileX * kTileY)
     }
 }
 
-// The blocks of k_pick_blocks' list, so many at a time as fit on the device.
-// What bounds it is the latency of each voxel's chain from the projection over
-// the four distances to the voxel itself, and the bytes of the voxels in front
-// of the surface.  A CTA for each block of a 512^3 grid spent 339 us on a frame,
-// of which 57% of the voxels are outside the image and 18 to 32% hidden behind
-// the surface; more voxels in flight per thread (2, 4 or 8 along z loaded
-// together) were slower (357 to 397 us), exact quotients by one reciprocal no
-// faster.
+// The blocks of k_pick_blocks' list, each taken by the next CTA that is free
+// (counts: the blocks listed, and those taken).  What bounds it is instruction
+// issue, about 110 a voxel and 63% of the slots.  A CTA for each block of a 512^3
+// grid spent 339 us on a frame, of which 57% of the voxels are outside the image
+// and 18 to 32% hidden behind the surface; all three launches of the listed
+// update take 280 us, 346 with the blocks dealt out evenly beforehand (256^3: 55
+// us, 63 without the launches' overlap, and 50 for all blocks, but six frames with
+// their ray casts on three streams 744 against 785).  More voxels in flight per
+// thread (2, 4 or 8 along z loaded together) were slower.
 __global__ void __launch_bounds__(kTileX * kTileY, kListCtas)
     k_update_list(float2 *__restrict__ grid, uint8_t *__restrict__ flags, const float *__restrict__ dist, Geom g, int bx,
-                  int by, const int *__restrict__ list, const int *__restrict__ count) {
-    const int n = *count, lane = threadIdx.x & 31, row = threadIdx.x >> 5;
-    for (int i = blockIdx.x; i < n; i += gridDim.x) {
-        const int b = list[i];
+                  int by, const int *__restrict__ list, int *__restrict__ counts) {
+    wait_before();
+    __shared__ int s_next[2];
+    const int n = counts[0], lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_next[0] = atomicAdd(counts + 1, 1);
+    __syncthreads();
+    for (int turn = 0; s_next[turn] < n; turn ^= 1) {
+        const int entry = list[s_next[turn]], b = entry < 0 ? ~entry : entry;
+        // the next one is asked for while this one is worked on
+        int next = 0;
+        if (threadIdx.x == 0) next = atomicAdd(counts + 1, 1);
         const int ix = b % bx * kTileX + lane;
         unsigned n_proj = 0, n_fused = 0, n_changed = 0;
         if (ix < g.R)
-            fuse_run(grid, flags, dist, g, ix, b / bx % by * kTileY + row, b / bx / by * kRunZ, n_proj, n_fused, n_changed);
+            fuse_run(grid, flags, dist, g, entry >= 0, ix, b / bx % by * kTileY + row, b / bx / by * kRunZ, n_proj, n_fused,
+                     n_changed);
+        if (threadIdx.x == 0) s_next[turn ^ 1] = next;
+        __syncthreads();
     }
 }
 
@@ -862,7 +898,7 @@ struct recon_tsdf {
     uint8_t *flags = nullptr;
     float *dist = nullptr;
     float *far_tiles = nullptr;  // of an update: the largest distance per tile of the map,
-    int *list = nullptr;         // and the blocks to visit, after their number
+    int *list = nullptr;         // and the blocks to visit, after their number and that of those taken
     float4 *xyz = nullptr, *shaded = nullptr, *normal = nullptr;
     void *staging = nullptr;  // device copy of a host measurement (uint16 or float4 frame)
     size_t staging_bytes = 0;
@@ -978,6 +1014,8 @@ Geom make_geom(const recon_tsdf_params &p, const float *T3x4, const float *K) {
     g.lim = vsx * 2;
     g.tol = p.cube_dim[0] / 200.0f;
     g.slope = p.cube_dim[0] * 0.030f;
+    g.inv_slope = 1.0f / g.slope;
+    g.slope_lo = g.slope >= 0x1p-60f && g.slope <= 0x1p60f ? 0x1p-60f : INFINITY;
     g.b0x = p.cube_origin[0] - p.cube_dim[0];
     g.b0y = p.cube_origin[1] - p.cube_dim[1];
     g.b0z = p.cube_origin[2] - p.cube_dim[2];
@@ -1025,6 +1063,25 @@ struct Timed {
 // Launches through cudaLaunchKernelEx, whose return value is the launch's own
 // status: an error another part of the process left pending is neither
 // reported as this library's nor cleared.
+// A programmatic dependent of the launch before it in the stream: it may start
+// while that one ends, and waits for it by itself (wait_before).
+template <typename... KArgs, typename... Args>
+int launch_after(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+    if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
+    rt::add_launches(1);
+    return RECON_OK;
+}
+
 template <typename... KArgs, typename... Args>
 int launch(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
@@ -1124,7 +1181,7 @@ int recon_tsdf_create(const recon_tsdf_params *p, void *stream, recon_tsdf **out
     alloc((void **)&v->flags, n_flag_bytes(*p));
     alloc((void **)&v->dist, n_pixels(*p) * sizeof(float));
     alloc((void **)&v->far_tiles, n_far_tiles(*p) * sizeof(float));
-    alloc((void **)&v->list, (1 + n_blocks(*p)) * sizeof(int));
+    alloc((void **)&v->list, (2 + n_blocks(*p)) * sizeof(int));
     alloc((void **)&v->xyz, n_pixels(*p) * sizeof(float4));
     alloc((void **)&v->shaded, n_pixels(*p) * sizeof(float4));
     alloc((void **)&v->normal, n_pixels(*p) * sizeof(float4));
@@ -1230,11 +1287,11 @@ int recon_tsdf_update(recon_tsdf *v, const float T[16], const float K[9]) {
                       (unsigned long long *)nullptr);
     rc = launch(k_far_tiles, dim3((g.tiles_x * g.tiles_y + 3) / 4), dim3(128), v->stream, v->dist, g, v->far_tiles, v->list);
     if (!rc)
-        rc = launch(k_pick_blocks, dim3((n + 31) / 32), dim3(256), v->stream, v->far_tiles, g, (int)grd.x, (int)grd.y, n,
-                    v->list + 1, v->list);
+        rc = launch_after(k_pick_blocks, dim3((n + 31) / 32), dim3(256), v->stream, v->far_tiles, g, (int)grd.x, (int)grd.y, n,
+                    v->list + 2, v->list);
     if (!rc)
-        rc = launch(k_update_list, dim3(152 * kListCtas), dim3(kTileX * kTileY), v->stream, v->grid, v->flags, v->dist, g,
-                    (int)grd.x, (int)grd.y, v->list + 1, v->list);
+        rc = launch_after(k_update_list, dim3(152 * kListCtas), dim3(kTileX * kTileY), v->stream, v->grid, v->flags, v->dist, g,
+                    (int)grd.x, (int)grd.y, v->list + 2, v->list);
     return rc;
 }
 
