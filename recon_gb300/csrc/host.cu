@@ -699,7 +699,10 @@ int run_schedule(recon_batch *b) {
         }
         e = cudaStreamEndCapture(cs[0], &g);
         release();
-        if (rc) return rc;
+        if (rc) {
+            if (g) cudaGraphDestroy(g);
+            return rc;
+        }
         if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
         e = cudaGraphInstantiate(&b->graph, g, 0);
         cudaGraphDestroy(g);

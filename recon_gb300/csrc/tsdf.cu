@@ -155,10 +155,13 @@ struct Block {
         }
         // |rz| >= 16 mm at every corner keeps the rounding of the projected
         // coordinates far below the 4-pixel margin
+        // (votes of all lanes: none may depend on another's outcome)
         const unsigned front = __ballot_sync(0xffffffffu, rz < -16.0f) >> group & 0xffu;
         const unsigned behind = __ballot_sync(0xffffffffu, rz > 16.0f) >> group & 0xffu;
-        sharp = front == 0xffu && (__ballot_sync(0xffffffffu, pixel) >> group & 0xffu) == 0xffu;
-        plain = front == 0xffu && fmaxf(fabsf(g.K0), fabsf(g.K4)) <= 16.0f && (__ballot_sync(0xffffffffu, small) >> group & 0xffu) == 0xffu;
+        const unsigned to_pixel = __ballot_sync(0xffffffffu, pixel) >> group & 0xffu;
+        const unsigned all_small = __ballot_sync(0xffffffffu, small) >> group & 0xffu;
+        sharp = front == 0xffu && to_pixel == 0xffu;
+        plain = front == 0xffu && all_small == 0xffu && fmaxf(fabsf(g.K0), fabsf(g.K4)) <= 16.0f;
         outside = (front == 0xffu || behind == 0xffu) && (!(hi_x >= -3.0f) || !(lo_x < g.Wf + 2.0f) ||
                                                           !(hi_y >= -3.0f) || !(lo_y < g.Hf + 2.0f));
     }
@@ -182,8 +185,8 @@ struct Block {
 };
 
 // The blocks that the update has to visit: 8 lanes per block.  count was set
-// to 0 by k_far_tiles.  A block that is not plain is listed as ~number.  Their order in the list is of no matter: every voxel
-// is in one block.
+// to 0 by k_far_tiles.  A block that is not plain is listed as ~number.  Their
+// order in the list is of no matter: every voxel is in one block.
 __global__ void __launch_bounds__(256)
     k_pick_blocks(const float *__restrict__ far_tiles, Geom g, int bx, int by, int n, int *__restrict__ list,
                   int *__restrict__ count) {
