@@ -253,7 +253,7 @@ size_t layout(InstDesc &d, char *base) {
         d.cur_gray[l] = nl ? a.take<float>(nl) : nullptr;
         d.ref_pts[l] = nl ? a.take<float4>(nl) : nullptr;
         d.ref_nrm[l] = nl ? a.take<float4>(nl) : nullptr;
-        d.ref_pl[l] = nl ? a.take<float>(6 * (size_t)((nl + kChunk - 1) / kChunk) * kChunk) : nullptr;
+        d.ref_pl[l] = nl ? a.take<float>(ref_plane_floats(nl)) : nullptr;
         d.cur_pts[l] = nl && l > 0 ? a.take<float4>(nl) : nullptr;
         d.sel_I[l] = (l < d.L) ? a.take<float>(P) : nullptr;
         d.sel_J[l] = (l < d.L) ? a.take<float>(6 * (size_t)P) : nullptr;
@@ -987,6 +987,9 @@ int recon_batch_create(int32_t n, const recon_config *cfgs, const float *calibs,
         b->arenas.push_back(mem);
         cudaMemsetAsync(mem, 0, bytes, b->stream);
         layout(d, (char *)mem);
+        // no pixel has a point (z is NaN) until a keyframe is set, nor past a level's last one
+        for (int l = 0; l < d.L; l++)
+            cudaMemsetAsync(d.ref_pl[l], 0xff, ref_plane_floats((d.W >> l) * (d.H >> l)) * sizeof(float), b->stream);
         b->max_pix = std::max(b->max_pix, c.width * c.height);
         b->max_L = std::max(b->max_L, c.levels);
         b->max_P = std::max(b->max_P, c.n_select);

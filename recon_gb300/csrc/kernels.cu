@@ -1131,7 +1131,7 @@ __device__ __forceinline__ void icp_mask_blocks(const InstDesc &d, int level, co
         float r4[4];
 #pragma unroll
         for (int g = 0; g < 4; g += kBatch) {
-            // (past the last pixel the planes hold a point of depth 0: it is not stored)
+            // (past the last pixel the planes hold no point: nothing is stored)
             float p[kBatch][6], q[kBatch][3], px[kBatch], py[kBatch];
             bool in[kBatch];
             IcpTaps<kDepth> tap[kBatch];

@@ -45,7 +45,7 @@ struct InstDesc {
     float4 *ref_nrm[kMaxLevels];  // nx ny nz 0
     // the same for the ICP kernels, in blocks of 1024 pixels (ref_plane):
     // [pixels / 1024][6][1024], x y z nx ny nz, z NaN where the pixel has no
-    // point; zero past the level's last pixel
+    // point, before the first keyframe and past the level's last pixel
     float *ref_pl[kMaxLevels];
     float *gmag;                  // W*H: the keyframe pixels' gradient magnitudes
     int *grad_hist;               // select_bins
@@ -88,7 +88,8 @@ struct InstDesc {
     int *trace_count;
 };
 
-// Plane k of pixel i in a level's ref_pl
+// Floats in a level's ref_pl of n pixels, and plane k of pixel i there
+__host__ __device__ constexpr size_t ref_plane_floats(int n) { return 6 * (size_t)((n + kChunk - 1) / kChunk) * kChunk; }
 __host__ __device__ constexpr size_t ref_plane(int i, int k) { return (size_t)(i / kChunk * 6 + k) * kChunk + i % kChunk; }
 
 // Programmatic dependent launch.  The kernels of the per-frame schedule are
