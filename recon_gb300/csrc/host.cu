@@ -571,26 +571,27 @@ int icp_per_cta(const recon_batch *b, int level) {
 // other groups run beside it
 int launch_schedule(recon_batch *b, cudaStream_t s, bool in_graph, int first, int n) {
     auto D = b->d_desc + first;
-    bool any_icp = false;
-    for (int i = first; i < first + n; i++) any_icp |= (b->cfg[i].mode != RECON_PHOTOMETRIC);
     for (int level = b->max_L - 1; level >= 0; level--) {
-        int maxit = 0, maxpix = 0;
+        // the iterations of the level, and the pixels of its ICP term.  A kernel is
+        // launched only where one of the instances runs it: a launch all of whose
+        // CTAs left before pdl_wait would complete before the launches ahead of it,
+        // and the next one's wait covers only the launch before it.
+        int maxit = 0, icp_pix = 0;
         for (int i = first; i < first + n; i++) {
             const recon_config &c = b->cfg[i];
             if (level >= c.levels) continue;
             int it = c.iters[c.levels - 1 - level];
             if (it > maxit) maxit = it;
-            int px = (c.width >> level) * (c.height >> level);
-            if (px > maxpix) maxpix = px;
+            if (it > 0 && c.mode != RECON_PHOTOMETRIC) icp_pix = std::max(icp_pix, (c.width >> level) * (c.height >> level));
         }
         if (maxit == 0) continue;
-        int nchunk = (maxpix + kChunk - 1) / kChunk;
-        if (any_icp && maxpix <= kPrepareFusedMaxPix) {
+        int nchunk = (icp_pix + kChunk - 1) / kChunk;
+        if (icp_pix > 0 && icp_pix <= kPrepareFusedMaxPix) {
             // small grid: mask and Student-t passes in one cluster launch
             TimedScope ts(b, s, TK_ICP_PREP, in_graph);
             CK(launch_pdl(k_icp_prepare, dim3(kIterCluster, n), dim3(1024), s, D, level));
             b->graph_kernels += 1;
-        } else if (any_icp) {
+        } else if (icp_pix > 0) {
             {
                 TimedScope ts(b, s, TK_ICP_MASK, in_graph);
                 // up to 4 blocks per CTA, as far as the device stays filled
@@ -608,7 +609,7 @@ int launch_schedule(recon_batch *b, cudaStream_t s, bool in_graph, int first, in
             b->graph_kernels += 4;
         }
         int per_cta = icp_per_cta(b, level);
-        int ncta = any_icp ? (nchunk + per_cta - 1) / per_cta : 0;
+        int ncta = (nchunk + per_cta - 1) / per_cta;
         // every instance's photometric cluster, then ncta ICP CTAs per
         // instance, the total rounded up to whole clusters
         int gx = kIterCluster * n + (n * ncta + kIterCluster - 1) / kIterCluster * kIterCluster;

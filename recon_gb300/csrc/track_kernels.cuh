@@ -96,8 +96,10 @@ __host__ __device__ constexpr size_t ref_plane(int i, int k) { return (size_t)(i
 // launched so that the next kernel may start while this one finishes:
 // pdl_trigger lets it be scheduled, and pdl_wait (griddepcontrol.wait) returns
 // once every earlier kernel of the stream has completed and its writes are
-// visible.  Before pdl_wait a kernel reads only the instance descriptors (not
-// written by any kernel of the schedule) and writes nothing.
+// visible.  That holds through the launch before: a launch must have a CTA that
+// waits (launch_schedule), else it completes ahead of its predecessors and the
+// next wait is for it alone.  Before pdl_wait a kernel reads only the instance
+// descriptors (not written by any kernel of the schedule) and writes nothing.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
