@@ -594,8 +594,10 @@ int launch_schedule(recon_batch *b, cudaStream_t s, bool in_graph, int first, in
         } else if (icp_pix > 0) {
             {
                 TimedScope ts(b, s, TK_ICP_MASK, in_graph);
-                // up to 4 blocks per CTA, as far as the device stays filled
-                int per = std::min(4, std::max(1, b->n * nchunk / kMaskCtaSlots));
+                // up to 4 blocks per CTA, as far as the batch's blocks fill the device (one
+                // 640x480 instance among forty of 80x60, geometric: 239 us, 256 with as many
+                // blocks per CTA as forty-one of 640x480 would have)
+                int per = (int)std::min(4LL, std::max(1LL, level_blocks(b, level) / kMaskCtaSlots));
                 CK(launch_pdl(k_icp_mask, dim3((nchunk + per - 1) / per, n), dim3(kLanes), s, D, level, per));
             }
             {
@@ -629,10 +631,13 @@ int launch_schedule(recon_batch *b, cudaStream_t s, bool in_graph, int first, in
     return RECON_OK;
 }
 
-// The batch as up to four groups of instances [group[k], group[k + 1]) of about
-// as many pixels each, whose launches do not wait for one another: while one
-// group solves, prepares its weights or drains its last CTAs, the others keep the
-// SMs busy.  An instance's result does not depend on the launch it is part of.
+// The batch as up to four groups of consecutive instances [group[k], group[k +
+// 1]), whose launches do not wait for one another: a group ends at the instance
+// that takes the batch's pixels to its share (instances of like sizes are shared
+// out evenly; one that is large beside the others stays with those before it, and
+// there are fewer groups then).  While one group solves, prepares its weights or
+// drains its last CTAs, the others keep the SMs busy.  An instance's result does
+// not depend on the launch it is part of.
 // 640x480 bi-objective segments with 1, 2, 4 and 8 groups: 2 instances 4512,
 // 4376, -, - us; 8 instances 7403, 6397, 6307, 6487; 30 instances 17514, 15083,
 // 15054, 15245; 256 mixed pairs 9290, 8406, 8177, 8133.
