@@ -2474,16 +2474,16 @@ __device__ __forceinline__ void student_body(const InstDesc *D, int level) {
         float r_next = 0.0f;
         uint8_t m_next = 0;
         if (i < n) {
-            r_next = __ldg(d.icp_r2 + i);
-            m_next = __ldg(d.icp_mask + i);
+            r_next = d.icp_r2[i];
+            m_next = d.icp_mask[i];
         }
         for (; i < n; i += stride) {
             // the next pixel's loads are in flight while this one is weighed
             float r = r_next;
             uint8_t mk = m_next;
             if (i + stride < n) {
-                r_next = __ldg(d.icp_r2 + i + stride);
-                m_next = __ldg(d.icp_mask + i + stride);
+                r_next = d.icp_r2[i + stride];
+                m_next = d.icp_mask[i + stride];
             }
             if (pass == 3) {
                 d.icp_w[i] = mk ? fminf(weight(r), 1.0f) : 0.0f;

@@ -1,0 +1,31 @@
+"""Which arrays the kernels read with __ldg (ld.global.nc): memory must be
+read-only as long as a kernel that reads it so runs.  A violation need not show
+in results, so the sources are looked at."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "recon_gb300", "csrc")
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def body(text, head):
+    """The function that begins with `head`, up to the brace that closes it."""
+    start = text.index(head)
+    depth, k = 0, text.index("{", start)
+    while True:
+        depth += {"{": 1, "}": -1}.get(text[k], 0)
+        k += 1
+        if depth == 0:
+            return text[start:k]
+
+
+def test_preparation_kernel_reads_what_it_wrote_with_plain_loads():
+    code = body(source("kernels.cu"), "void student_body(")
+    written = set(re.findall(r"\bd\.(icp_\w+)\[[^\]]*\]\s*=[^=]", code))
+    assert {"icp_r2", "icp_mask", "icp_w"} <= written
+    for name in written:
+        assert not re.search(r"__ldg\([^;]*\bd\." + name, code), name
