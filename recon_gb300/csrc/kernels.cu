@@ -1322,19 +1322,19 @@ __global__ void __launch_bounds__(kLanes, 5) k_icp_student_pass(const InstDesc *
             if (b0 + u >= b_last || i >= n) continue;
             if (i + 3 < n) {
                 // 16- and 4-byte aligned: the arrays start on 256-byte boundaries
-                r[u] = __ldg(reinterpret_cast<const float4 *>(d.icp_r2 + i));
-                if (pass == 3) m[u] = __ldg(reinterpret_cast<const uchar4 *>(d.icp_mask + i));
+                r[u] = __ldcg(reinterpret_cast<const float4 *>(d.icp_r2 + i));
+                if (pass == 3) m[u] = __ldcg(reinterpret_cast<const uchar4 *>(d.icp_mask + i));
             } else {
                 // the instance's last pixels (n not a multiple of 4)
-                r[u].x = __ldg(d.icp_r2 + i);
-                m[u].x = __ldg(d.icp_mask + i);
+                r[u].x = __ldcg(d.icp_r2 + i);
+                m[u].x = __ldcg(d.icp_mask + i);
                 if (i + 1 < n) {
-                    r[u].y = __ldg(d.icp_r2 + i + 1);
-                    m[u].y = __ldg(d.icp_mask + i + 1);
+                    r[u].y = __ldcg(d.icp_r2 + i + 1);
+                    m[u].y = __ldcg(d.icp_mask + i + 1);
                 }
                 if (i + 2 < n) {
-                    r[u].z = __ldg(d.icp_r2 + i + 2);
-                    m[u].z = __ldg(d.icp_mask + i + 2);
+                    r[u].z = __ldcg(d.icp_r2 + i + 2);
+                    m[u].z = __ldcg(d.icp_mask + i + 2);
                 }
             }
         }
@@ -2082,7 +2082,7 @@ __device__ void icp_chunks(const InstDesc &d, IterShared &sh, int level, int c0,
             bool in[kBatch];
 #pragma unroll
             for (int u = 0; u < kBatch; u++) {
-                w[u] = __ldg(wts + (g + u) * kLanes);
+                w[u] = __ldcg(wts + (g + u) * kLanes);
 #pragma unroll
                 for (int k = 0; k < 6; k++) p[u][k] = __ldg(ref + k * kChunk + (g + u) * kLanes);
             }

@@ -99,7 +99,10 @@ __host__ __device__ constexpr size_t ref_plane(int i, int k) { return (size_t)(i
 // visible.  That holds through the launch before: a launch must have a CTA that
 // waits (launch_schedule), else it completes ahead of its predecessors and the
 // next wait is for it alone.  Before pdl_wait a kernel reads only the instance
-// descriptors (not written by any kernel of the schedule) and writes nothing.
+// descriptors and the keyframe (not written by any kernel of the schedule) and
+// writes nothing.  What the schedule's kernels write is never read with __ldg,
+// which is for memory that nothing writes while the kernel runs: a kernel that is
+// waiting already runs.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 

@@ -29,3 +29,16 @@ def test_preparation_kernel_reads_what_it_wrote_with_plain_loads():
     assert {"icp_r2", "icp_mask", "icp_w"} <= written
     for name in written:
         assert not re.search(r"__ldg\([^;]*\bd\." + name, code), name
+
+
+def test_schedule_reads_what_its_launches_write_past_the_read_only_path():
+    """The launches of a frame overlap: a kernel is running while the one before
+    it still writes."""
+    text = source("kernels.cu")
+    for head in ("k_icp_mask(const InstDesc *D", "k_icp_student_pass(const InstDesc *D", "void icp_chunks(",
+                 "bool photo_cluster(", "void finalize_iter(", "void student_body("):
+        code = body(text, head)
+        pointers = "|".join(re.findall(r"\*(\w+)\s*=\s*d\.(?:icp_\w+|ph_\w+|fx)\b", code) + re.findall(
+            r",\s*\*(\w+)\s*=\s*d\.icp_\w+", code)) or "none"
+        for load in re.findall(r"__ldg\(([^;]*);", code):
+            assert not re.search(r"\bd\.(icp_|ph_|fx\b|T\b|stats\b)|\b(" + pointers + r")\b", load), (head, load)
