@@ -169,7 +169,9 @@ struct Block {
     // that its voxels can see is too short for them to be fused.  A slack of 4
     // pixels and of 1e-4 covers the roundings of the projection, of the
     // interpolated distance and of the quotient.
-    __device__ __forceinline__ bool hidden(const Geom &g, const float *__restrict__ far_tiles) const {
+    // (far_tiles is written while the kernel that reads it already waits: a plain
+    // load, not one for read-only memory.)
+    __device__ __forceinline__ bool hidden(const Geom &g, const float *far_tiles) const {
         const int lane = threadIdx.x & 31;
         const int tx0 = (int)fmaxf(lo_x - 4.0f, 0.0f) / kFarTile, ty0 = (int)fmaxf(lo_y - 4.0f, 0.0f) / kFarTile;
         const int tx1 = (int)fminf(hi_x + 6.0f, g.Wf - 1.0f) / kFarTile;
@@ -178,7 +180,7 @@ struct Block {
         const bool look = sharp && !outside && n <= kFarMost;
         float far = 0.0f;
         if (look)
-            for (int i = lane & 7; i < n; i += 8) far = fmaxf(far, __ldg(far_tiles + (ty0 + i / nx) * g.tiles_x + tx0 + i % nx));
+            for (int i = lane & 7; i < n; i += 8) far = fmaxf(far, far_tiles[(ty0 + i / nx) * g.tiles_x + tx0 + i % nx]);
         for (int o = 1; o < 8; o <<= 1) far = fmaxf(far, __shfl_xor_sync(0xffffffffu, far, o));
         return look && (far < g.lim || near - far > 1.25f * g.slope + 1e-4f * (near + g.slope));
     }
@@ -188,8 +190,7 @@ struct Block {
 // to 0 by k_far_tiles.  A block that is not plain is listed as ~number.  Their
 // order in the list is of no matter: every voxel is in one block.
 __global__ void __launch_bounds__(256)
-    k_pick_blocks(const float *__restrict__ far_tiles, Geom g, int bx, int by, int n, int *__restrict__ list,
-                  int *__restrict__ count) {
+    k_pick_blocks(const float *far_tiles, Geom g, int bx, int by, int n, int *list, int *count) {
     next_may_start();
     const int lane = threadIdx.x & 31, i = (blockIdx.x * 256 + threadIdx.x) >> 3, b = min(i, n - 1);
     const Block block(g, b % bx * kTileX, b / bx % by * kTileY, b / bx / by * kRunZ);
@@ -309,7 +310,7 @@ __global__ void __launch_bounds__(kTileX * kTileY)
 // thread (2, 4 or 8 along z loaded together) were slower.
 __global__ void __launch_bounds__(kTileX * kTileY, kListCtas)
     k_update_list(float2 *__restrict__ grid, uint8_t *__restrict__ flags, const float *__restrict__ dist, Geom g, int bx,
-                  int by, const int *__restrict__ list, int *__restrict__ counts) {
+                  int by, const int *list, int *counts) {
     wait_before();
     __shared__ int s_next[2];
     const int n = counts[0], lane = threadIdx.x & 31, row = threadIdx.x >> 5;

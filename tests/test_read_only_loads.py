@@ -42,3 +42,13 @@ def test_schedule_reads_what_its_launches_write_past_the_read_only_path():
             r",\s*\*(\w+)\s*=\s*d\.icp_\w+", code)) or "none"
         for load in re.findall(r"__ldg\(([^;]*);", code):
             assert not re.search(r"\bd\.(icp_|ph_|fx\b|T\b|stats\b)|\b(" + pointers + r")\b", load), (head, load)
+
+
+def test_listed_update_reads_its_list_with_plain_loads():
+    """k_pick_blocks and k_update_list wait for the launch that writes what they
+    read: no pointer to it promises (const and __restrict__) that it stays as it is."""
+    text = source("tsdf.cu")
+    assert not re.search(r"__ldg\([^;]*\b(far_tiles|list|counts?)\b", text)
+    for head in ("k_pick_blocks(", "k_update_list(", "bool hidden("):
+        params = re.search(re.escape(head) + r"([^)]*)\)", text).group(1)
+        assert not re.search(r"__restrict__\s+(far_tiles|list|counts?)\b", params), head
