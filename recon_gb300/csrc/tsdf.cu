@@ -55,13 +55,16 @@ constexpr int kTileY = 8;
 constexpr int kRunZ = 8;
 constexpr int kFarTile = 16;    // distance map tiles of the update's test for blocks behind the surface
 constexpr int kFarMost = 256;   // tiles that a block may look at
-constexpr int kListCtas = 8;    // CTAs per SM of the update by list
+constexpr int kUpdateCtas = 8;  // CTAs per SM of an update: 32 registers
 // From this many blocks on the update picks the blocks to visit first: two small
-// launches, which cost more than they save on a coarse grid.  640x480 frames, all
-// blocks / picked ones, four frames with their ray casts: 64^3 203 / 222 us,
-// 160^3 (2000 blocks) 340 / 361; six frames on 256^3 (8192) 785 / 758; two on
-// 512^3 (65536) 1014 / 812.
-constexpr int kListBlocks = 6144;
+// launches more, which have to save more than they cost on a single grid.  The
+// update of one grid by itself, 640x480 frames of a room, all blocks / picked ones:
+// 192^3 (3456 blocks) 29 / 38 us, 256^3 (8192) 51 / 59, 320^3 (16000) 90 / 99, 352^3
+// (21296) 117 / 116, 512^3 (65536) 344 / 339.  (What picking saves depends on how
+// much of the grid lies behind surfaces.  With the frames of three grids on their
+// streams, where other work fills the launches' gaps, four scenes on 256^3 took
+// 762, 805, 753 and 766 us with all blocks, 745, 818, 746 and 751 with picked ones.)
+constexpr int kListBlocks = 18000;
 constexpr int kRayTileX = 8;  // ray cast CTA: one warp on 8 x 4 pixels (rays differ widely in length;
 constexpr int kRayTileY = 4;  // one-warp CTAs let the block scheduler balance the SMs)
 constexpr int kRayCtas = 28;  // ray cast CTAs per SM: 72 registers.  32 (64 registers) spill more and 24 leave fewer
@@ -269,9 +272,10 @@ __device__ __forceinline__ void fuse_run(float2 *__restrict__ grid, uint8_t *__r
 }
 
 // All blocks of the grid.  counts (kCount): voxels [projected into the image,
-// fused, changed].
+// fused, changed].  As many CTAs per SM as the listed update has, for the latency
+// of its gathers: 256^3 51 us, 512^3 344; 53 and 373 at the registers it would take.
 template <bool kCount>
-__global__ void __launch_bounds__(kTileX * kTileY)
+__global__ void __launch_bounds__(kTileX * kTileY, kUpdateCtas)
     k_update(float2 *__restrict__ grid, uint8_t *__restrict__ flags, const float *__restrict__ dist, Geom g,
              unsigned long long *__restrict__ counts) {
     __shared__ int s_skip;
@@ -301,14 +305,12 @@ __global__ void __launch_bounds__(kTileX * kTileY)
 
 // The blocks of k_pick_blocks' list, each taken by the next CTA that is free
 // (counts: the blocks listed, and those taken).  What bounds it is instruction
-// issue, about 110 a voxel and 63% of the slots.  A CTA for each block of a 512^3
-// grid spent 339 us on a frame, of which 57% of the voxels are outside the image
-// and 18 to 32% hidden behind the surface; all three launches of the listed
-// update take 280 us, 346 with the blocks dealt out evenly beforehand (256^3: 55
-// us, 63 without the launches' overlap, and 50 for all blocks, but six frames with
-// their ray casts on three streams 744 against 785).  More voxels in flight per
-// thread (2, 4 or 8 along z loaded together) were slower.
-__global__ void __launch_bounds__(kTileX * kTileY, kListCtas)
+// issue, about 110 a voxel and 63% of the slots.  On a 512^3 grid, of whose voxels
+// a frame has 57% outside the image and 18 to 32% hidden behind the surface, all
+// three launches of the listed update take 280 us; 346 with the blocks dealt out
+// evenly beforehand (kListBlocks has a CTA for each block of the grid beside it).
+// More voxels in flight per thread (2, 4 or 8 along z loaded together) were slower.
+__global__ void __launch_bounds__(kTileX * kTileY, kUpdateCtas)
     k_update_list(float2 *__restrict__ grid, uint8_t *__restrict__ flags, const float *__restrict__ dist, Geom g, int bx,
                   int by, const int *list, int *counts) {
     wait_before();
@@ -1294,7 +1296,7 @@ int recon_tsdf_update(recon_tsdf *v, const float T[16], const float K[9]) {
         rc = launch_after(k_pick_blocks, dim3((n + 31) / 32), dim3(256), v->stream, v->far_tiles, g, (int)grd.x, (int)grd.y, n,
                     v->list + 2, v->list);
     if (!rc)
-        rc = launch_after(k_update_list, dim3(152 * kListCtas), dim3(kTileX * kTileY), v->stream, v->grid, v->flags, v->dist, g,
+        rc = launch_after(k_update_list, dim3(152 * kUpdateCtas), dim3(kTileX * kTileY), v->stream, v->grid, v->flags, v->dist, g,
                     (int)grd.x, (int)grd.y, v->list + 2, v->list);
     return rc;
 }
