@@ -235,12 +235,15 @@ def _on_device(a) -> int:
 
 
 def _torch_stream() -> int:
-    """The handle of torch's current stream (what torch.cuda.current_stream()
-    would wrap, without the wrapper: 0.2 against 3 us)."""
+    """The handle of torch's current stream, without the wrapper object of
+    torch.cuda.current_stream() (0.2 against 3 us) where torch has the calls for it."""
     import torch
     if not torch.cuda.is_initialized():
         torch.cuda.init()
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    try:
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    except AttributeError:  # private names: another torch may not have them
+        return torch.cuda.current_stream().cuda_stream
 
 
 def _order_after_torch(batch) -> None:
