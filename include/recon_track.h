@@ -298,8 +298,9 @@ int recon_photometric_iteration_noalloc(const recon_photo_view *view, float *T_d
  * two for every float in [0, 2^23) on the current GPU and stores the number of
  * mismatches (0 on a correct device). */
 int recon_selftest_exact_arith(int64_t *mismatches);
-/* Mismatches of the library's reciprocal (every mantissa) and division
- * (pseudo-random operands) against the compiler's IEEE division. */
+/* Mismatches of the library's reciprocal (every mantissa, in seven binades) and
+ * division (pseudo-random operands, and numerators below its range in the
+ * expressions that take them) against the compiler's IEEE division. */
 int recon_selftest_division(int64_t *mismatches);
 
 /* Makes `consumer` wait for the work queued so far on `producer` (two streams

@@ -997,7 +997,11 @@ __device__ __forceinline__ bool icp_project(const IcpLevel &L, float qx, float q
 // The four taps of a projected pixel.  At level 0 they are depths, and the
 // points are formed from them as genPointsCloud6Kernel does (d2z.cu:436-469; zero
 // where there is no depth): a quarter of the bytes and of the cache lines that
-// gathering points costs, for 36 operations, half of them packed.  At the other
+// gathering points costs, for 36 operations, half of them packed.  (The division's
+// operands are looked at from above only.  A numerator below its range, a depth or
+// a distance from the principal point of less than 2^-60, still gives the rounded
+// quotient down to 2^-102, then one within a unit in the last place, and a zero may
+// lose its sign: nothing in a sum of millimetres.)  At the other
 // levels (averages of points) they are float4 points.
 template <bool kDepth> struct IcpTaps;
 template <> struct IcpTaps<true> {

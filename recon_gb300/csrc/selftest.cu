@@ -30,34 +30,47 @@ __global__ void k_check_trunc(unsigned long long *bad) {
     add_count(bad, c);
 }
 
-// every mantissa at the ends and the middle of the range, both signs: the
-// reciprocal against the correctly rounded one
+// every mantissa in seven binades of [2^-60, 2^60], the first and the last among
+// them, and 2^60, both signs: the reciprocal against the correctly rounded one
 __global__ void k_check_rcp(unsigned long long *bad) {
     unsigned long long c = 0;
     uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < 0x800000u; m += stride)
-        for (uint32_t E = 127 - 60; E < 127 + 60; E += 20)
+        for (uint32_t k = 0; k < 8; k++) {
+            uint32_t E = k < 6 ? 127 - 60 + 20 * k : 127 + 53 + k;  // 67, 87, .. 167, 186, 187
+            if (k == 7 && m) continue;
             for (uint32_t sign = 0; sign < 2; sign++) {
                 float b = __uint_as_float(sign << 31 | E << 23 | m), y = __frcp_rn(b);
                 float2 y2 = rcp_rn2(dup2(b));
                 c += rcp_rn(b) != y || y2.x != y || y2.y != y;
             }
+        }
     add_count(bad, c);
 }
 
-// pseudo-random operands of the range (a linear congruential sequence a
-// thread): quotients against the compiler's division, and packed sums and
-// differences of products against separately rounded ones
+// a linear congruential sequence a thread
+struct Draws {
+    unsigned long long s;
+    __device__ __forceinline__ explicit Draws(unsigned long long seed)
+        : s((blockIdx.x * blockDim.x + threadIdx.x) * 0x9E3779B97F4A7C15ull + seed) {}
+    __device__ __forceinline__ uint32_t bits() {
+        s = s * 6364136223846793005ull + 1442695040888963407ull;
+        return (uint32_t)(s >> 32);
+    }
+    // a value of either sign in [2^lo, 2^hi]
+    __device__ __forceinline__ float value(int lo, int hi) {
+        uint32_t m = bits(), E = 127 + lo + (bits() >> 8) % (hi - lo + 1);
+        return __uint_as_float((m & 0x80000000u) | E << 23 | (E == 127u + hi ? 0u : m & 0x7fffffu));
+    }
+};
+
+// pseudo-random operands of the range: quotients against the compiler's division,
+// and packed sums and differences of products against separately rounded ones
 __global__ void k_check_div(unsigned long long *bad, int per_thread) {
-    unsigned long long c = 0, s = (blockIdx.x * blockDim.x + threadIdx.x) * 0x9E3779B97F4A7C15ull + 12345;
-    auto next = [&]() {
-        s = s * 6364136223846793005ull + 1442695040888963407ull;
-        uint32_t r = (uint32_t)(s >> 32);
-        s = s * 6364136223846793005ull + 1442695040888963407ull;
-        return __uint_as_float((r & 0x807fffffu) | ((127u - 60u + (uint32_t)(s >> 40) % 120u) << 23));
-    };
+    unsigned long long c = 0;
+    Draws draw(12345);
     for (int i = 0; i < per_thread; i++) {
-        float a0 = next(), a1 = next(), b = next();
+        float a0 = draw.value(-60, 60), a1 = draw.value(-60, 60), b = draw.value(-60, 60);
         float2 q = div_rn2(make_float2(a0, a1), dup2(-b), rcp_rn2(dup2(b)));
         // a product and a sum stay two roundings
         float2 s2 = add2(mul2(make_float2(a0, a1), dup2(b)), make_float2(a1, a0), unseen_one());
@@ -65,6 +78,38 @@ __global__ void k_check_div(unsigned long long *bad, int per_thread) {
         c += s2.x != __fadd_rn(__fmul_rn(a0, b), a1) || s2.y != __fadd_rn(__fmul_rn(a1, b), a0);
         c += d2.x != __fsub_rn(a1, __fmul_rn(a0, b)) || d2.y != __fsub_rn(a0, __fmul_rn(a1, b));
         c += !div_in_range(a0, a1, b) || div_rn(a0, -b, rcp_rn(b)) != a0 / b || q.x != a0 / b || q.y != a1 / b;
+    }
+    add_count(bad, c);
+}
+
+// Numerators below the range, which some callers pass without a look: zeros,
+// denormal and small values, in the callers' own expressions, and as a quotient
+// (IcpTaps), which is exact down to numerators of 2^-102 and below that within a
+// unit in the last place.
+__global__ void k_check_small(unsigned long long *bad, int per_thread) {
+    unsigned long long c = 0;
+    Draws draw(54321);
+    auto over = [](float a, float b) { return div_rn2(dup2(a), dup2(-b), rcp_rn2(dup2(b))); };
+    for (int i = 0; i < per_thread; i++) {
+        uint32_t r = draw.bits();
+        // exponent field 0 .. 66, a zero now and then
+        float tiny = (r & 63u) == 0 ? 0.0f : __uint_as_float((r >> 8 & 0x7fffffu) | (draw.bits() >> 8) % 67 << 23);
+        float sigma2 = fabsf(draw.value(-20, 60)), scale = fabsf(draw.value(-7, 1)), f = fabsf(draw.value(-20, 20));
+        // Student-t: 5 + r^2 / sigma^2, by either form
+        float t = 5.0f + tiny / sigma2;
+        float2 q = over(tiny, sigma2);
+        c += 5.0f + div_rn(tiny, -sigma2, rcp_rn(sigma2)) != t || 5.0f + q.x != t || 5.0f + q.y != t;
+        // Tukey: 1 - (|r| / scale / 4.6851)^2
+        float2 u = over(tiny, scale), ub = div_rn2(u, dup2(-4.6851f), dup2(1.0f / 4.6851f));
+        float v = tiny / scale / 4.6851f;
+        c += 1.0f - ub.x * ub.x != 1.0f - v * v || !(u.x <= 4.6851f);
+        // depth: 1 - e / 1e4
+        float2 e = div_rn2(dup2(tiny), dup2(-10000.0f), dup2(1.0f / 10000.0f));
+        c += 1.0f - e.x != 1.0f - tiny / 10000.0f;
+        // a coordinate over a focal length
+        float a = r & 64u ? -tiny : tiny, exact = a / f;
+        float2 p = over(a, f);
+        c += fabsf(a) >= 0x1p-102f ? p.x != exact : !(fabsf(p.x - exact) <= 0x1p-23f * fabsf(exact) + 0x1p-126f);
     }
     add_count(bad, c);
 }
@@ -109,5 +154,6 @@ extern "C" int recon_selftest_division(int64_t *mismatches) {
     return count_mismatches(mismatches, "recon_selftest_division: null argument", [](unsigned long long *d) {
         rt::k_check_rcp<<<152 * 8, 256>>>(d);
         rt::k_check_div<<<152 * 8, 256>>>(d, 4000);
+        rt::k_check_small<<<152 * 8, 256>>>(d, 1000);
     });
 }
