@@ -302,6 +302,10 @@ int recon_selftest_exact_arith(int64_t *mismatches);
  * division (pseudo-random operands, and numerators below its range in the
  * expressions that take them) against the compiler's IEEE division. */
 int recon_selftest_division(int64_t *mismatches);
+/* Mismatches of the normal equations' fixed-point sums (single values of every
+ * exponent, sums, their rounding to FP64 at ties and carries) against 128-bit
+ * integer arithmetic. */
+int recon_selftest_fixed_point(int64_t *mismatches);
 
 /* Makes `consumer` wait for the work queued so far on `producer` (two streams
  * of the current device; no host stall). */

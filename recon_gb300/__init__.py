@@ -164,6 +164,7 @@ def lib() -> ctypes.CDLL:
             L.recon_render_gray.argtypes = [vp, vp, vp, vp]
             L.recon_selftest_exact_arith.argtypes = [vp]
             L.recon_selftest_division.argtypes = [vp]
+            L.recon_selftest_fixed_point.argtypes = [vp]
             L.recon_stream_follow.argtypes = [vp, vp]
             L.recon_kinect_disparity_to_depth.argtypes = [vp, i32, i32, f32, f32, f32, f32, f32, f32, i32, vp, vp]
             L.recon_kinect_rgb_to_gray.argtypes = [vp, i32, i32, vp, vp]
@@ -625,6 +626,13 @@ def selftest_division() -> int:
     """Mismatches of the kernels' reciprocal and division against IEEE division, run on the current GPU."""
     out = np.zeros(1, np.int64)
     check(lib().recon_selftest_division(out.ctypes.data))
+    return int(out[0])
+
+
+def selftest_fixed_point() -> int:
+    """Mismatches of the normal equations' fixed-point sums against 128-bit integers, run on the current GPU."""
+    out = np.zeros(1, np.int64)
+    check(lib().recon_selftest_fixed_point(out.ctypes.data))
     return int(out[0])
 
 

@@ -1,11 +1,13 @@
-// selftest.cu -- compares the truncation of the Student-t variance sums
-// (exact_arith.cuh) with the conversion it replaces, and the reciprocal and
-// division of pair_math.cuh with the compiler's, on the GPU the library runs on.
+// selftest.cu -- compares, on the GPU the library runs on, the truncation of the
+// Student-t variance sums (exact_arith.cuh) with the conversion it replaces, the
+// reciprocal and division of pair_math.cuh with the compiler's, and the fixed-point
+// sums of fx.cuh with 128-bit integers.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "../../include/recon_track.h"
 #include "exact_arith.cuh"
+#include "fx.cuh"
 #include "pair_math.cuh"
 
 namespace rt {
@@ -114,6 +116,97 @@ __global__ void k_check_small(unsigned long long *bad, int per_thread) {
     add_count(bad, c);
 }
 
+// a sum in units of 2^-64, rounded to FP64: to 64 bits of which the last is set
+// when any bit after it was, then by the hardware's conversion
+__device__ double round_q64(unsigned __int128 q) {
+    bool neg = (q >> 127) != 0;
+    unsigned __int128 u = neg ? (unsigned __int128)0 - q : q;
+    int s = 0;
+    for (; (u >> s >> 64) != 0; s++) {}
+    unsigned long long top = (unsigned long long)(u >> s);
+    if ((u & (((unsigned __int128)1 << s) - 1)) != 0) top |= 1ull;
+    double v = ldexp(__ull2double_rn(top), s - 64);
+    return neg ? -v : v;
+}
+__device__ __forceinline__ bool same(double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); }
+
+// One value of every exponent and sign (mantissas of all zeros, all ones and
+// random bits), and sums of 40: fx_accumulate against fx_split and against the
+// value in 128 bits, and what is out of range.
+__global__ void k_check_fx_sum(unsigned long long *bad, int per_thread) {
+    unsigned long long c = 0;
+    Draws draw(777);
+    for (int i = 0; i < per_thread; i++) {
+        uint32_t acc[4] = {0u, 0u, 0u, 0u};
+        unsigned __int128 want = 0;
+        long long limbs[kFxLimbs] = {0, 0, 0, 0};
+        int n = i & 1 ? 40 : 1, flag = 0, split_flag = 0;
+        bool out = false;
+        for (int k = 0; k < n; k++) {
+            uint32_t r = draw.bits(), E = n > 1 ? (draw.bits() >> 8) % 175u : (draw.bits() >> 8) % 256u;
+            uint32_t M = draw.bits() & 0x7fffffu;
+            if ((r & 3u) < 2u) M = r & 1u ? 0x7fffffu : 0u;
+            float v = __uint_as_float((r & 0x80000000u) | E << 23 | M);
+            fx_accumulate(acc, v, flag);
+            int k0;
+            long long lo, hi;
+            fx_split(v, k0, lo, hi, split_flag);
+            limbs[k0] += lo;
+            if (hi) limbs[k0 + 1] += hi;
+            if (E >= 175u) {
+                out = true;
+                continue;
+            }
+            // (a denormal value is below the unit)
+            unsigned __int128 m = E ? (unsigned __int128)(M | 0x800000u) : 0;
+            int s = (int)E - 86;
+            m = s >= 0 ? m << s : (s <= -24 ? 0 : m >> -s);
+            want += r >> 31 ? (unsigned __int128)0 - m : m;
+        }
+        unsigned __int128 got = (unsigned __int128)acc[3] << 96 | (unsigned __int128)acc[2] << 64 |
+                                (unsigned __int128)acc[1] << 32 | acc[0];
+        c += got != want || (flag != 0) != out || (split_flag != 0) != out;
+        c += !same(fx_to_double(limbs), round_q64(want));
+    }
+    add_count(bad, c);
+}
+
+// fx_to_double of limbs that overlap, of sums of every length, and of halves: a
+// 53-bit mantissa (random, even, odd, all ones) with one half of its last place
+// after it, and a little more or less than that
+__global__ void k_check_fx_round(unsigned long long *bad, int per_thread) {
+    unsigned long long c = 0;
+    Draws draw(4242);
+    for (int i = 0; i < per_thread; i++) {
+        unsigned long long a = (unsigned long long)draw.bits() << 32 | draw.bits();
+        unsigned long long b = (unsigned long long)draw.bits() << 32 | draw.bits();
+        uint32_t r = draw.bits();
+        unsigned __int128 q;
+        if (r & 1u) {
+            unsigned long long m = (r & 6u) == 6u ? (1ull << 53) - 1 : a >> 11 | 1ull << 52;
+            int s = (r >> 8) % 73u;  // the half's place
+            q = ((unsigned __int128)m << 1 | 1) << s;
+            if (s && (r & 24u) == 8u) q += 1;
+            if ((r & 24u) == 16u) q -= 1;
+        } else {
+            q = ((unsigned __int128)a << 64 | b) >> (1 + (r >> 8) % 127u);
+        }
+        if (r & 32u) q = (unsigned __int128)0 - q;
+        long long limbs[kFxLimbs];
+        for (int k = 0; k < kFxLimbs; k++) limbs[k] = (long long)(uint32_t)(q >> (32 * k));
+        limbs[3] = (int)(uint32_t)limbs[3];
+        c += !same(fx_to_double(limbs), round_q64(q));
+        // the same total with pieces moved from limb to limb
+        for (int k = 0; k < kFxLimbs - 1; k++) {
+            long long t = (int)draw.bits() >> 4;
+            limbs[k] += t * (1ll << 32);
+            limbs[k + 1] -= t;
+        }
+        c += !same(fx_to_double(limbs), round_q64(q));
+    }
+    add_count(bad, c);
+}
+
 }  // namespace
 }  // namespace rt
 
@@ -155,5 +248,12 @@ extern "C" int recon_selftest_division(int64_t *mismatches) {
         rt::k_check_rcp<<<152 * 8, 256>>>(d);
         rt::k_check_div<<<152 * 8, 256>>>(d, 4000);
         rt::k_check_small<<<152 * 8, 256>>>(d, 1000);
+    });
+}
+
+extern "C" int recon_selftest_fixed_point(int64_t *mismatches) {
+    return count_mismatches(mismatches, "recon_selftest_fixed_point: null argument", [](unsigned long long *d) {
+        rt::k_check_fx_sum<<<152 * 4, 256>>>(d, 200);
+        rt::k_check_fx_round<<<152 * 4, 256>>>(d, 400);
     });
 }
