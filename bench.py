@@ -49,13 +49,14 @@ KEYFRAME_EVERY = 10
 ITERS = (1, 3, 10, 5)
 LAMBDA = 0.5
 N_SELECT = 8192
-# algorithmic bytes per point and GN iteration (photometric: xyz 12 + I_ref 4 +
-# J 24 + 4 bilinear taps 16 + depth tap 4; the fused kernel keeps the residual
-# and depth weight in registers, so the 16 bytes of the reference's separate
-# passes are not counted; ICP: point+normal 24 + 4 taps x 12 + mask 4 + weight 4
-# + index 4)
+# algorithmic bytes per point and GN iteration.  Photometric: xyz 12 + I_ref 4 +
+# J 24 + 4 bilinear taps 16 + depth tap 4 (the fused kernel keeps the residual and
+# depth weight in registers, so the 16 bytes of the reference's separate passes are
+# not counted).  ICP: the reference's point and normal 24 + weight 4 + the pixel's
+# share of the current frame's depths 4 (level 0, where neighbours share their taps;
+# the coarser levels read points, 16, which are not counted).
 B_PHOTO = 60
-B_ICP = 84
+B_ICP = 32
 # learned initialisation: trained parameters and the shortened schedule it runs
 LEARNED_WEIGHTS = "initnet_200k.npz"
 # (in a sweep of shortened schedules on this trajectory: the most frames per
@@ -1191,7 +1192,10 @@ def main():
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "kernel": "k_iter",
                          "peak_source": peak_kind,
+                         "traffic_frac": traffic / per_launch_s / 1e9 / peak if traffic and per_launch_s > 0 else None,
                          "algorithmic_bytes_per_launch": per_launch_bytes,
+                         "bytes_rule": f"{B_PHOTO} B per photometric point-iteration + {B_ICP} B per ICP "
+                                       "point-iteration; traffic: DRAM bytes of the average launch, profiled",
                          "avg_launch_ms": per_launch_s * 1000.0,
                          "timing": "per-launch CUDA events on the batch stream, separate K-step pass of the plain arm"},
             "cpu_baseline": cpu,

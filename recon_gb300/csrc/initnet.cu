@@ -81,9 +81,9 @@ __device__ __forceinline__ void copy16_or_zero(void *dst, const void *src, bool 
 //
 // The CTA copies its pixels' patches into shared memory once (16 bytes a copy,
 // rows padded so that ldmatrix meets no bank twice); reading them as fragments
-// from global memory took every warp of the NG through the same 4-byte loads
-// and their index arithmetic (a batch of 256: 32 to 64 channels at 8x10 72 -> 14 us,
-// 64 to 64 at 4x5 50 -> 14).  MT is as large as 38 KB of patches allow where that
+// from global memory takes every warp of the NG through the same 4-byte loads
+// and their index arithmetic (a batch of 256, the third and the fourth layer: 14 us each
+// so, 72 and 50 that way).  MT is as large as 38 KB of patches allow where that
 // still leaves a CTA per SM: the weights' fragments then serve MT tiles.
 constexpr int kConvWarps = 16;
 constexpr int conv_tiles(int cin) { return cin >= 128 ? 1 : cin >= 64 ? 2 : 4; }
@@ -312,8 +312,8 @@ __global__ void k_head_fwd(const __nv_bfloat16 *a6, int P, const float *wfc, con
 // gradients of kHeadChunk samples at a time and the features of kHeadTile of them
 // are staged in shared memory by all threads, thread c adds its products over
 // the samples in order.  CTA 0 adds the loss: every thread's squared errors (its
-// entries in order), then a fixed tree.  One CTA that read its features one
-// sample after another took 27 us for 256 samples.
+// entries in order), then a fixed tree.  (One CTA that reads its features one sample
+// after another takes 27 us for 256 samples.)
 constexpr int kHeadChunk = 128, kHeadTile = 64;
 __global__ void k_head_grad(const float *y, const float *t, const float *feat, int N, float *gwfc, float *gbfc,
                             float *loss) {
@@ -392,6 +392,20 @@ __device__ __forceinline__ void mma_bf16(float *c, const uint32_t *a, uint32_t b
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// four channels: the network's own activations are aligned to 8 bytes, the
+// caller's input (the layer of 4 channels) to 4
+template <int CIN> __device__ __forceinline__ uint2 load4(const __nv_bfloat16 *p) {
+    if constexpr (CIN > 4) return __ldg(reinterpret_cast<const uint2 *>(p));
+    const unsigned *q = reinterpret_cast<const unsigned *>(p);
+    return make_uint2(__ldg(q), __ldg(q + 1));
+}
+
+constexpr int kWgKT = 64, kWgMS = 64, kWgThreads = 128;
+// where row k's words of the staged patches lie: their index with these bits
+// turned, alike for the 8 rows of a fragment (the stores of 16 rows' words then
+// share a bank 4 times instead of 8)
+__device__ __forceinline__ constexpr int wg_swizzle(int k) { return 8 * ((k >> 3) & 3); }
+
 // Weight and bias gradients of a convolution on the tensor cores:
 // gW[co][k] = sum_m dz[m][co] X[m][k], X the 3x3 / stride 2 / pad 1 patches
 // of the layer input (k = tap * Cin + c), a GEMM whose reduction runs over
@@ -406,21 +420,8 @@ __device__ __forceinline__ void mma_bf16(float *c, const uint32_t *a, uint32_t b
 // gradient at k = Kp: the split's FP32 sum of dz (each thread adds its pixel
 // pairs in order, the threads of a co are then added in thread order).  It is
 // bound by staging the patches: with a tap's bit and an offset per pixel and
-// column instead of the whole index arithmetic per element, and four channels a
-// load, the six layers of a batch of 256 take 166 us against 274.
-// four channels: the network's own activations are aligned to 8 bytes, the
-// caller's input (the layer of 4 channels) to 4
-template <int CIN> __device__ __forceinline__ uint2 load4(const __nv_bfloat16 *p) {
-    if constexpr (CIN > 4) return __ldg(reinterpret_cast<const uint2 *>(p));
-    const unsigned *q = reinterpret_cast<const unsigned *>(p);
-    return make_uint2(__ldg(q), __ldg(q + 1));
-}
-
-constexpr int kWgKT = 64, kWgMS = 64, kWgThreads = 128;
-// where row k's words of the staged patches lie: their index with these bits
-// turned, alike for the 8 rows of a fragment (the stores of 16 rows' words then
-// share a bank 4 times instead of 8)
-__device__ __forceinline__ constexpr int wg_swizzle(int k) { return 8 * ((k >> 3) & 3); }
+// column, and four channels a load, the six layers of a batch of 256 take 166 us;
+// 274 with the index arithmetic for each element.
 template <int L>
 __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad_tc(const float *dz, const __nv_bfloat16 *in, int N, int nsplit,
                                                               int per, float *partial) {

@@ -115,10 +115,10 @@ __global__ void k_convert_level0(const InstDesc *D, const uint8_t *const *in_gra
 // and the 2x2 reductions of fastDownSampleHdrKernel and downSampleCloud6Kernel
 // for the coarser levels (the expressions of k_downsample, in its order), so
 // every value is identical to the separate kernels'.  A CTA of 256 threads
-// takes a 32x32 tile of level 0 (54 us for 30 640x480 frames, of which the bytes
-// take 24; 68 us with IEEE divisions and one pixel per access): each thread converts one 2x2 block and
-// reduces it to its level-1 pixel in registers; levels 2 and 3 come from the
-// level-1 tile in shared memory.  Level 0 is never read back.
+// takes a 32x32 tile of level 0: each thread converts one 2x2 block and reduces it
+// to its level-1 pixel in registers; levels 2 and 3 come from the level-1 tile in
+// shared memory.  Level 0 is never read back.  54 us for 30 640x480 frames, of which
+// the bytes take 24; 68 with IEEE divisions and one pixel per access.
 constexpr int kPyrTile = 32;
 
 __device__ __forceinline__ void cloud_point(const PixelRays &rays, int xi, int yi, float z, float4 &o) {
@@ -490,8 +490,8 @@ __device__ __forceinline__ float4 ref_point(const InstDesc &d, const PixelRays &
 // and masks (computeNormalsCudaKernel, d2z.cu:503-537).  It is bound by the 56
 // bytes that it writes per pixel; a pixel's four neighbours are formed from their
 // depths again, which costs less than reading points that another kernel wrote
-// (30 640x480 frames: 108 us here and 39 for the conversion, against 105 and 80,
-// and no launch of its own, 52 us, to form the points of a fused depth).
+// (30 640x480 frames: 108 us here and 39 for the conversion; 105 and 80 where the
+// conversion writes the points, and a launch of 52 us to form those of a fused depth).
 __global__ void k_normals(const InstDesc *D, const int *active, int per_cta) {
     INST_DESC;
     if (!active[blockIdx.y]) return;
@@ -1254,9 +1254,9 @@ __global__ void __launch_bounds__(kLanes, kMaskCtas)
 // variance sum, which CTA 0 stores.  The sums are exact int64 sums, so the
 // result does not depend on how the pixels are split; one launch per pass
 // keeps every SM busy without any CTA waiting on another.  48 registers: five
-// CTAs per SM (kPassCtaSlots).  It was bound by the two IEEE divisions of the
-// weight: with the exact division by a reciprocal (StudentW), the three passes of
-// level 0 of 30 640x480 instances take 45 us against 63, level 1 23 against 27.
+// CTAs per SM (kPassCtaSlots).  The three passes of
+// level 0 of 30 640x480 instances take 45 us, level 1 23; 63 and 27 with IEEE
+// divisions in place of those by a reciprocal (StudentW).
 // Passes 1 and 2 need no mask: a pixel that is no correspondence has r^2 = 0.
 __global__ void __launch_bounds__(kLanes, 5) k_icp_student_pass(const InstDesc *D, int level, int pass,
                                                              int blocks_per_cta) {
@@ -2132,11 +2132,10 @@ __device__ __forceinline__ int packed_index(int r, int c) {
 // handed over through shared memory; every global value is loaded in one round
 // trip at the start, since the FP64 solve that follows is one serial chain on
 // warp 0.  Warp 1 meanwhile resets the sums, keeps the work counters and writes
-// the optional trace.  With the small-twist path, the column-at-once Cholesky and
-// the lane-parallel conjugate gradients of solve.cuh (measured on one instance, graph replay):
-// an iteration of 320x240 photometric tracking 21.7 us against 25.1 us, a
-// bi-objective 640x480 frame of 19 iterations 559 against 630 us, a 482x362
-// geometric keyframe and frame with the CG solver 458 against 668 us.
+// the optional trace.  What bounds it is that chain, 64 cycles an FP64 instruction:
+// about 7.5 of the 16.7 us of an iteration of 320x240 photometric tracking (one
+// instance, graph replay), 3.4 us less than with the general exponential and a
+// column-by-column Cholesky in place of solve.cuh's short forms.
 __device__ __forceinline__ void finalize_iter(const InstDesc &d, SolveShared &sh, int level, int it, bool use_ph,
                                               bool use_icp) {
     int lane = threadIdx.x & 31, set = threadIdx.x >> 5;
@@ -2258,13 +2257,13 @@ __device__ __forceinline__ void finalize_iter(const InstDesc &d, SolveShared &sh
 // atomics, so the result does not depend on K or on the order in which CTAs
 // finish; k_solve then fuses, solves and updates the pose.
 //
-// What bounds it: at the fine levels the FP32 issue of about 300 operations a
-// pixel with the latency of its taps (a level-0 launch of 30 640x480 instances
-// reads 32 bytes a pixel, 44 us at the measured HBM rate, and takes 125 us,
-// 148 us before; level 1 52 us, before 57), at the coarse levels and for a single
-// instance the photometric chain (level 3 of 30 instances 15 us, before 18; a 320x240
-// photometric iteration with its solve 17.0 us, before 21.7).  Measured and not kept: two
-// pixels in packed arithmetic with the pose in shared memory (135 us: a third fewer
+// What bounds it: at the fine levels instruction issue, about 390 a pixel, and the
+// latency of its taps (a level-0 launch of 30 640x480 instances moves 335 MB of
+// DRAM, 49 us at the measured HBM rate, and takes 117 us; level 1 48 us), at the
+// coarse levels and for a single instance the photometric chain (level 3 of 30
+// instances 20 us; a 320x240 photometric iteration with its solve 16.7 us).
+// Measured and not kept, on a scene whose level-0 launch takes 125 us: two pixels in
+// packed arithmetic with the pose in shared memory (135 us: a third fewer
 // instructions, but the constants' loads and 80 registers), inputs copied two
 // blocks ahead into shared memory (3 CTAs an SM, of which clusters of 8 leave 11% of
 // the slots empty: 134 us), one share of the blocks for each resident CTA (151 us:

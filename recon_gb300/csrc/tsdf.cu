@@ -557,9 +557,8 @@ struct Corner {
 // What bounds it is instruction issue (58% of the slots; DRAM 2%), so the rays
 // of a warp are kept on the same part of the walk: all cross empty blocks, then
 // all walk, and the fine search waits until none can walk on.  640x480 rays on
-// a 256^3 grid of a room: 95.6 million warp instructions with every block
-// crossed axis by axis in loops of additions, 57.4 million so; 193 -> 148 us
-// alone, and six frames of three streams 950 -> 779 us.
+// a 256^3 grid of a room take 57.4 million warp instructions and 148 us; 95.6
+// million and 193 us with every block crossed axis by axis in loops of additions.
 __device__ bool traverse(bool in_grid, const float2 *__restrict__ grid, const uint8_t *__restrict__ flags, const Geom &g,
                          const Ray &r, float idx, float idy, float idz, int s0, int s1, int s2, float enterT,
                          float exitT, int iter, float *t_hit) {
@@ -969,9 +968,6 @@ void invert_rt4(const float *M, float *Mi) {
     Mi[12] = 0; Mi[13] = 0; Mi[14] = 0; Mi[15] = 1;
 }
 
-// the launch constants of SimParams (VoxelGrid.cpp:48-106; kernel prologues
-// VoxelGrid_cuda.cu:745-756, 957-965): T3x4 is the first three rows of the
-// pose the kernel uses
 // whether start + n * step is exact in float for every start on the axis' grid
 // (b0 + v * step) and every n that a walk of max_steps can take: b0 and step
 // are multiples of a power of two u, and the sums stay below 2^24 u
@@ -987,6 +983,9 @@ bool walk_is_exact(float b0, float step, int R) {
     return std::ldexp(std::fabs((double)b0) + (double)step * (4 * R + 32), -u) < 16777216.0;
 }
 
+// the launch constants of SimParams (VoxelGrid.cpp:48-106; kernel prologues
+// VoxelGrid_cuda.cu:745-756, 957-965): T3x4 is the first three rows of the
+// pose the kernel uses
 Geom make_geom(const recon_tsdf_params &p, const float *T3x4, const float *K) {
     Geom g;
     memset(&g, 0, sizeof(g));
@@ -1066,9 +1065,6 @@ struct Timed {
     }
 };
 
-// Launches through cudaLaunchKernelEx, whose return value is the launch's own
-// status: an error another part of the process left pending is neither
-// reported as this library's nor cleared.
 // A programmatic dependent of the launch before it in the stream: it may start
 // while that one ends, and waits for it by itself (wait_before).
 template <typename... KArgs, typename... Args>
@@ -1088,6 +1084,9 @@ int launch_after(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, 
     return RECON_OK;
 }
 
+// Launches through cudaLaunchKernelEx, whose return value is the launch's own
+// status: an error another part of the process left pending is neither
+// reported as this library's nor cleared.
 template <typename... KArgs, typename... Args>
 int launch(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
