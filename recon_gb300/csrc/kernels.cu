@@ -2257,7 +2257,7 @@ __device__ __forceinline__ void finalize_iter(const InstDesc &d, SolveShared &sh
 // atomics, so the result does not depend on K or on the order in which CTAs
 // finish; k_solve then fuses, solves and updates the pose.
 //
-// What bounds it: at the fine levels instruction issue, about 390 a pixel, and the
+// What bounds it: at the fine levels instruction issue, about 320 a pixel, and the
 // latency of its taps (a level-0 launch of 30 640x480 instances moves 335 MB of
 // DRAM, 49 us at the measured HBM rate, and takes 117 us; level 1 48 us), at the
 // coarse levels and for a single instance the photometric chain (level 3 of 30
