@@ -1354,10 +1354,12 @@ int64_t recon_batch_get_array(recon_batch *b, int32_t inst, const char *name, in
     if (sz > nbytes) return fail(RECON_ERR_INVALID_ARG, "destination too small");
     CK(cudaStreamSynchronize(b->stream));
     if (nm == "cur_pts" && level == 0) {
-        // not stored: the points of the depth image, as the kernels form them
+        // not stored: the points of the depth image, as the kernels form them (a NaN,
+        // from an infinite depth on the principal point's column or row, is the GPU's)
         std::vector<float> z(n0);
         CK(cudaMemcpy(z.data(), d.cur_z, (size_t)n0 * 4, cudaMemcpyDeviceToHost));
         const float *K = d.calib + 43;  // the IR camera matrix (calib.h:22-37)
+        const uint32_t nan_bits = 0x7fffffffu;
         float *o = (float *)host_dst;
         for (int i = 0; i < n0; i++, o += 4) {
             bool ok = z[i] < 0;
@@ -1365,6 +1367,8 @@ int64_t recon_batch_get_array(recon_batch *b, int32_t inst, const char *name, in
             o[1] = ok ? ((float)(i / d.W) - K[5]) * z[i] / K[4] : 0.0f;
             o[2] = ok ? z[i] : 0.0f;
             o[3] = ok ? 1.0f : 0.0f;
+            for (int k = 0; k < 2; k++)
+                if (o[k] != o[k]) memcpy(o + k, &nan_bits, sizeof(nan_bits));
         }
         return sz;
     }
